@@ -21,13 +21,43 @@ namespace vfs {
 constexpr int KB = 256;
 constexpr int MAXCOL = 64;  // largest restart length
 
+// Blocks of the reductions and update sweeps: two cells per thread (one turn of
+// the dots' loop, every load of a thread in flight at once) until the grid
+// fills four blocks per SM.  A 104x40x72 grid (327 k cells) at 20 columns:
+// four cells per thread left half the SMs' blocks unused.
 int krylov_nblocks(size_t n) {
-  size_t b = (n + KB * 4 - 1) / (KB * 4);
+  size_t b = (n + KB * 2 - 1) / (KB * 2);
   if (b > 152 * 4) b = 152 * 4;
   return (int)(b ? b : 1);
 }
 
 __device__ __forceinline__ bool is_done(const KrylovState* st) { return *(volatile const int*)&st->done; }
+// done and epoch to pinned host memory (the host reads them after the event
+// that follows the iteration).
+__device__ __forceinline__ void post_status(const KrylovState* st, int* hst) {
+  if (!hst) return;
+  volatile int* h = hst;
+  h[0] = st->done;
+  h[1] = st->epoch;
+  __threadfence_system();
+}
+// True in every thread of the block that arrives last (each block calls it
+// once, after its partials): that block sums the partials of all blocks in a
+// fixed order, so the result does not depend on which block it is, and a
+// separate one-block launch (3 us of a captured iteration) is saved.  The
+// ticket is back at zero when the block continues.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
 __device__ __forceinline__ bool met(const KrylovState* st, double r) {
   return r <= st->rtol * st->bnorm && (st->atol <= 0. || r <= st->atol);
 }
@@ -99,10 +129,56 @@ int launch_vnext(KrylovState* st, const double* w, double* vn, size_t n, cudaStr
   return (int)cudaGetLastError();
 }
 
-// Multi-dot partials: parts[b * ld + q] = sum over the block's cells of V_q . w
-// for q < nv, chunks of 4 columns per sweep (w is re-read from L2).
+// Multi-dot partials: parts[q * nblocks + b] = sum over block b's cells of
+// V_q . w for q < nv, up to DCH columns per sweep (w is re-read from L2).
 // nv < 0: use the device's current column count st->j + 1 (graph-replayable).
 __device__ __forceinline__ int nv_of(const KrylovState* st, int nv) { return nv < 0 ? st->j + 1 : nv; }
+constexpr int DCH = 8;
+
+// Sums of DCH values over a warp by halving exchanges: 4 + 2 + 1 adds leave
+// one value per lane, two more finish it, 9 FP64 adds instead of 8 x 5 (the
+// adds go through the FP64 pipe at 16 cycles a warp, which is what the plain
+// tree cost: 640 cycles a column and block).  Lane l ends with the sum of
+// value warp_sum8_index(l).
+__device__ __forceinline__ double warp_sum8(const double* a, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  double t[4];
+  const bool h4 = lane & 16, h2 = lane & 8, h1 = lane & 4;
+#pragma unroll
+  for (int q = 0; q < 4; q++) t[q] = (h4 ? a[q + 4] : a[q]) + __shfl_xor_sync(FULL, h4 ? a[q] : a[q + 4], 16);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const double keep = h2 ? t[q + 2] : t[q], send = h2 ? t[q] : t[q + 2];
+    t[q] = keep + __shfl_xor_sync(FULL, send, 8);
+  }
+  const double keep = h1 ? t[1] : t[0], send = h1 ? t[0] : t[1];
+  double r = keep + __shfl_xor_sync(FULL, send, 4);
+  r += __shfl_xor_sync(FULL, r, 2);
+  r += __shfl_xor_sync(FULL, r, 1);
+  return r;
+}
+__device__ __forceinline__ int warp_sum8_index(int lane) { return (lane & 16 ? 4 : 0) | (lane & 8 ? 2 : 0) | (lane & 4 ? 1 : 0); }
+
+// Sum the multi-dot partials into st->h (and accumulate the column in hacc):
+// one warp per dot (q = warp, warp + 8, ...), each lane summing a fixed
+// stride of the block partials in four chains, then the warp tree.
+__device__ __forceinline__ void dots_finish(KrylovState* st, const double* parts, int nparts, int nv, int pass) {
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int q = threadIdx.x >> 5; q < nv; q += nw) {
+    const double* pq = parts + (size_t)q * nparts;
+    double s[4] = {0., 0., 0., 0.};
+    for (int p = lane; p < nparts; p += 128) {
+#pragma unroll
+      for (int u = 0; u < 4; u++)
+        if (p + 32 * u < nparts) s[u] += __ldcg(pq + p + 32 * u);
+    }
+    const double t = warp_sum((s[0] + s[1]) + (s[2] + s[3])) * st->vs[q];
+    if (lane == 0) {
+      st->h[q] = t;
+      st->hacc[q] = (pass == 1) ? t : st->hacc[q] + t;
+    }
+  }
+}
 
 // NQ consecutive basis columns V0 .. V0 + (NQ-1) n against w: two cells per
 // turn (their loads in flight together), each thread's cells accumulated in
@@ -131,60 +207,111 @@ __device__ __forceinline__ void dot_chunk(const double* __restrict__ V0, const d
   }
 }
 
-__global__ void __launch_bounds__(KB) k_multidot(const KrylovState* st, const double* __restrict__ V, int nv,
-                                                 const double* __restrict__ w, size_t n, double* parts, int ld) {
+__global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* __restrict__ V, int nv,
+                                                 const double* __restrict__ w, size_t n, double* parts, int pass) {
   if (is_done(st)) return;
   nv = nv_of(st, nv);
-  __shared__ double sh[32];
-  for (int q0 = 0; q0 < nv; q0 += 4) {
-    double a[4] = {0., 0., 0., 0.};
-    const int nq = min(4, nv - q0);
+  __shared__ double red[KB / 32][MAXCOL + DCH];
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  for (int q0 = 0; q0 < nv; q0 += DCH) {
+    double a[DCH] = {0., 0., 0., 0., 0., 0., 0., 0.};
     const double* V0 = V + (size_t)q0 * n;
-    switch (nq) {
+    switch (min(DCH, nv - q0)) {
+      case 8: dot_chunk<8>(V0, w, n, a); break;
+      case 7: dot_chunk<7>(V0, w, n, a); break;
+      case 6: dot_chunk<6>(V0, w, n, a); break;
+      case 5: dot_chunk<5>(V0, w, n, a); break;
       case 4: dot_chunk<4>(V0, w, n, a); break;
       case 3: dot_chunk<3>(V0, w, n, a); break;
       case 2: dot_chunk<2>(V0, w, n, a); break;
       default: dot_chunk<1>(V0, w, n, a); break;
     }
-    for (int q = 0; q < nq; q++) {
-      const double r = block_sum(a[q], sh);
-      if (threadIdx.x == 0) parts[(size_t)blockIdx.x * ld + q0 + q] = r;
-    }
+    const double r = warp_sum8(a, lane);
+    if ((lane & 3) == 0) red[wp][q0 + warp_sum8_index(lane)] = r;
   }
-}
-
-// Sum the multi-dot partials into st->h (and accumulate the column in hacc).
-// One warp per dot (q = warp, warp + 8, ...): each lane sums a fixed stride
-// of the block partials, then the warp tree; no block barriers, and the
-// order is fixed, so the result is deterministic.
-__global__ void k_multidot_finish(KrylovState* st, const double* __restrict__ parts, int nparts, int nv, int ld, int pass) {
-  if (is_done(st)) return;
-  nv = nv_of(st, nv);
-  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int q = threadIdx.x >> 5; q < nv; q += nw) {
-    double s = 0.;
-    for (int p = lane; p < nparts; p += 32) s += parts[(size_t)p * ld + q];
-    s = warp_sum(s) * st->vs[q];
-    if (lane == 0) {
-      st->h[q] = s;
-      st->hacc[q] = (pass == 1) ? s : st->hacc[q] + s;
-    }
+  __syncthreads();
+  for (int q = threadIdx.x; q < nv; q += blockDim.x) {
+    double r = 0.;
+    for (int u = 0; u < KB / 32; u++) r += red[u][q];
+    parts[(size_t)q * gridDim.x + blockIdx.x] = r;
   }
+  if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, pass);
 }
 
 int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
                     cudaStream_t s) {
-  const int nb = krylov_nblocks(n);
-  const int ld = 72;
-  k_multidot<<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches;
-  k_multidot_finish<<<1, KB, 0, s>>>(st, parts, nb, nv, ld, pass); ++g_launches;
+  k_multidot<<<krylov_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, pass); ++g_launches;
   return (int)cudaGetLastError();
 }
 
-// w -= sum_q h[q] V_q, with the partials of ||w||^2 after the update.
-__global__ void __launch_bounds__(KB) k_gs_update(const KrylovState* st, const double* __restrict__ V, int nv,
-                                                  double* __restrict__ w, size_t n, double* parts) {
-  if (is_done(st)) return;
+// Close Arnoldi column j from the nparts partials of ||w||^2 (one block):
+// ||w||, Hessenberg column, Givens rotations, residual estimate |g[j+1]|,
+// convergence test, 1 / h[j+1][j] for the next basis vector, and the status
+// to the host.  The column, the previous rotations and g[j] are staged in
+// shared memory by the whole block first, so that the serial rotation loop
+// of thread 0 reads no global memory.
+__device__ __forceinline__ void arnoldi_close(KrylovState* st, const double* parts, int nparts, int* hst) {
+  __shared__ double sh[32];
+  __shared__ double hc[MAXCOL + 2], cq[MAXCOL + 1], sq[MAXCOL + 1];
+  double s = 0.;
+  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += __ldcg(parts + p);
+  const int m = st->m, j = st->j;
+  for (int q = threadIdx.x; q <= j; q += blockDim.x) hc[q] = st->hacc[q];
+  for (int q = threadIdx.x; q < j; q += blockDim.x) {
+    cq[q] = st->cs[q];
+    sq[q] = st->sn[q];
+  }
+  s = block_sum(s, sh);  // (its barriers also order the staging)
+  if (threadIdx.x != 0) return;
+  const double hn = sqrt(s);
+  double* Hc = st->H + (size_t)j * (m + 1);
+  hc[j + 1] = hn;
+  for (int q = 0; q < j; q++) {
+    const double a = hc[q], b = hc[q + 1];
+    hc[q] = cq[q] * a + sq[q] * b;
+    hc[q + 1] = -sq[q] * a + cq[q] * b;
+  }
+  for (int q = 0; q < j; q++) Hc[q] = hc[q];
+  const double a = hc[j], b = hc[j + 1];
+  const double den = sqrt(a * a + b * b);
+  const double c = den > 0. ? a / den : 1., sn = den > 0. ? b / den : 0.;
+  st->cs[j] = c;
+  st->sn[j] = sn;
+  Hc[j] = den;
+  Hc[j + 1] = 0.;
+  st->g[j + 1] = -sn * st->g[j];
+  st->g[j] = c * st->g[j];
+  st->resid = fabs(st->g[j + 1]);
+  st->hn = hn;
+  st->inv_hn = hn > 0. ? 1. / hn : 0.;
+  st->vs[j + 1] = st->orth2 ? 1. : st->inv_hn;  // CGS2 normalises the column in k_vnext_in
+  st->j = j + 1;
+  st->it += 1;
+  if (met(st, st->resid) || hn == 0. || !(st->resid == st->resid)) st->done = 1;
+  post_status(st, hst);
+}
+// The close as its own launch, for a probed iteration (which times it alone).
+__global__ void __launch_bounds__(KB) k_arnoldi_finish(KrylovState* st, const double* __restrict__ parts, int nparts,
+                                                       int* hst) {
+  if (is_done(st)) {
+    if (threadIdx.x == 0) post_status(st, hst);
+    return;
+  }
+  arnoldi_close(st, parts, nparts, hst);
+}
+int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, int* hst, cudaStream_t s) {
+  k_arnoldi_finish<<<1, KB, 0, s>>>(st, parts, nparts, hst); ++g_launches;
+  return (int)cudaGetLastError();
+}
+
+// w -= sum_q h[q] V_q, with the partials of ||w||^2 after the update; close:
+// the last block closes the Arnoldi column.
+__global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double* __restrict__ V, int nv,
+                                                  double* __restrict__ w, size_t n, double* parts, int close, int* hst) {
+  if (is_done(st)) {
+    if (close && blockIdx.x == 0 && threadIdx.x == 0) post_status(st, hst);
+    return;
+  }
   nv = nv_of(st, nv);
   __shared__ double sh[32];
   __shared__ double hs[72];
@@ -199,25 +326,29 @@ __global__ void __launch_bounds__(KB) k_gs_update(const KrylovState* st, const d
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = s;
+  if (close && last_block(st->ticket)) arnoldi_close(st, parts, gridDim.x, hst);
 }
-int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int pass,
+int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int close, int* hst,
                      cudaStream_t s) {
-  (void)pass;
-  k_gs_update<<<krylov_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches;
+  k_gs_update<<<krylov_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, close, hst); ++g_launches;
   return (int)cudaGetLastError();
 }
 
 // One-pass classical Gram-Schmidt update of column j = st->j: the
 // orthogonalised vector u = w - sum_q h_q vs_q V_q is stored unnormalised as
 // V_{j+1}, its multigrid-precision copy as the next preconditioner input, and
-// the partials of ||u||^2 go to parts (k_arnoldi_finish sets vs_{j+1}).
+// the partials of ||u||^2 go to parts; the close of the column sets vs_{j+1}
+// (close: by the last block, else k_arnoldi_finish).
 // dinv (nullable): 1 / D of the FP16 normalised multigrid operator, applied
 // to the multigrid copy after its rounding to T.
 template <typename T>
-__global__ void __launch_bounds__(KB) k_cgs_update(const KrylovState* st, double* V, const double* __restrict__ w,
+__global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, const double* __restrict__ w,
                                                    T* __restrict__ out, size_t n, double* parts,
-                                                   const float* __restrict__ dinv) {
-  if (is_done(st)) return;
+                                                   const float* __restrict__ dinv, int close, int* hst) {
+  if (is_done(st)) {
+    if (close && blockIdx.x == 0 && threadIdx.x == 0) post_status(st, hst);
+    return;
+  }
   const int nv = st->j + 1;
   __shared__ double sh[32];
   __shared__ double hs[72];
@@ -254,17 +385,18 @@ __global__ void __launch_bounds__(KB) k_cgs_update(const KrylovState* st, double
   }
   s = block_sum(s, sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = s;
+  if (close && last_block(st->ticket)) arnoldi_close(st, parts, gridDim.x, hst);
 }
 template <typename T>
-int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, cudaStream_t s,
-                      const float* dinv) {
-  k_cgs_update<T><<<krylov_nblocks(n), KB, 0, s>>>(st, V, w, out, n, parts, dinv); ++g_launches;
+int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, int close, int* hst,
+                      cudaStream_t s, const float* dinv) {
+  k_cgs_update<T><<<krylov_nblocks(n), KB, 0, s>>>(st, V, w, out, n, parts, dinv, close, hst); ++g_launches;
   return (int)cudaGetLastError();
 }
-template int launch_cgs_update<float>(KrylovState*, double*, const double*, float*, size_t, double*, cudaStream_t,
-                                      const float*);
-template int launch_cgs_update<double>(KrylovState*, double*, const double*, double*, size_t, double*, cudaStream_t,
-                                       const float*);
+template int launch_cgs_update<float>(KrylovState*, double*, const double*, float*, size_t, double*, int, int*,
+                                      cudaStream_t, const float*);
+template int launch_cgs_update<double>(KrylovState*, double*, const double*, double*, size_t, double*, int, int*,
+                                       cudaStream_t, const float*);
 
 // Fused CGS2 middle pass: w <- w - V h (h from the first pass), and the
 // second pass's dots V_q . w computed on the updated element while the basis
@@ -273,8 +405,8 @@ template int launch_cgs_update<double>(KrylovState*, double*, const double*, dou
 // increasing capacities serves every column count (graph-replayable) while
 // the FP64 FMAs issued stay within 4 of 2 nv per element.
 template <int NV0, int NV>
-__global__ void __launch_bounds__(KB) k_gs_update_dots(const KrylovState* st, const double* __restrict__ V, int nv,
-                                                       double* __restrict__ w, size_t n, double* parts, int ld) {
+__global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const double* __restrict__ V, int nv,
+                                                       double* __restrict__ w, size_t n, double* parts) {
   if (is_done(st)) return;
   nv = nv_of(st, nv);
   if (nv <= NV0 || nv > NV) return;
@@ -307,74 +439,23 @@ __global__ void __launch_bounds__(KB) k_gs_update_dots(const KrylovState* st, co
   for (int q = threadIdx.x; q < nv; q += blockDim.x) {
     double x = 0.;
     for (int u = 0; u < KB / 32; u++) x += red[u][q];
-    parts[(size_t)blockIdx.x * ld + q] = x;
+    parts[(size_t)q * gridDim.x + blockIdx.x] = x;
   }
+  if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, 2);
 }
 
 // nv < 0: device column count, capacity chosen from cap (>= the largest nv).
 int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s,
                           int cap) {
   const int nb = krylov_nblocks(n);
-  const int ld = 72;
   if (nv > 32 || (nv < 0 && cap > 32)) return -1;
   // nv >= 0: the one bucket holding nv; nv < 0: every bucket up to cap
   const int lo = nv < 0 ? 0 : nv, hi = nv < 0 ? cap : nv;
-  if (lo <= 4) { k_gs_update_dots<0, 4><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches; }
-  if (lo <= 8 && hi > 4) { k_gs_update_dots<4, 8><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches; }
-  if (lo <= 16 && hi > 8) { k_gs_update_dots<8, 16><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches; }
-  if (lo <= 24 && hi > 16) { k_gs_update_dots<16, 24><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches; }
-  if (hi > 24) { k_gs_update_dots<24, 32><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts, ld); ++g_launches; }
-  k_multidot_finish<<<1, KB, 0, s>>>(st, parts, nb, nv, ld, 2); ++g_launches;
-  return (int)cudaGetLastError();
-}
-
-// Close Arnoldi column j: ||w||, Hessenberg column, Givens rotation, residual
-// estimate |g[j+1]|, convergence test, 1 / h[j+1][j] for the next basis vector.
-// The column, the previous rotations and g[j] are staged in shared memory by
-// the whole block first, so that the serial rotation loop of thread 0 reads
-// no global memory.
-__global__ void k_arnoldi_finish(KrylovState* st, const double* __restrict__ parts, int nparts) {
-  if (is_done(st)) return;
-  __shared__ double sh[32];
-  __shared__ double hc[MAXCOL + 2], cq[MAXCOL + 1], sq[MAXCOL + 1];
-  double s = 0.;
-  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += parts[p];
-  const int m = st->m, j = st->j;
-  for (int q = threadIdx.x; q <= j; q += blockDim.x) hc[q] = st->hacc[q];
-  for (int q = threadIdx.x; q < j; q += blockDim.x) {
-    cq[q] = st->cs[q];
-    sq[q] = st->sn[q];
-  }
-  s = block_sum(s, sh);  // (its barriers also order the staging)
-  if (threadIdx.x != 0) return;
-  const double hn = sqrt(s);
-  double* Hc = st->H + (size_t)j * (m + 1);
-  hc[j + 1] = hn;
-  for (int q = 0; q < j; q++) {
-    const double a = hc[q], b = hc[q + 1];
-    hc[q] = cq[q] * a + sq[q] * b;
-    hc[q + 1] = -sq[q] * a + cq[q] * b;
-  }
-  for (int q = 0; q < j; q++) Hc[q] = hc[q];
-  const double a = hc[j], b = hc[j + 1];
-  const double den = sqrt(a * a + b * b);
-  const double c = den > 0. ? a / den : 1., sn = den > 0. ? b / den : 0.;
-  st->cs[j] = c;
-  st->sn[j] = sn;
-  Hc[j] = den;
-  Hc[j + 1] = 0.;
-  st->g[j + 1] = -sn * st->g[j];
-  st->g[j] = c * st->g[j];
-  st->resid = fabs(st->g[j + 1]);
-  st->hn = hn;
-  st->inv_hn = hn > 0. ? 1. / hn : 0.;
-  st->vs[j + 1] = st->orth2 ? 1. : st->inv_hn;  // CGS2 normalises the column in k_vnext_in
-  st->j = j + 1;
-  st->it += 1;
-  if (met(st, st->resid) || hn == 0. || !(st->resid == st->resid)) st->done = 1;
-}
-int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, cudaStream_t s) {
-  k_arnoldi_finish<<<1, KB, 0, s>>>(st, parts, nparts); ++g_launches;
+  if (lo <= 4) { k_gs_update_dots<0, 4><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
+  if (lo <= 8 && hi > 4) { k_gs_update_dots<4, 8><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
+  if (lo <= 16 && hi > 8) { k_gs_update_dots<8, 16><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
+  if (lo <= 24 && hi > 16) { k_gs_update_dots<16, 24><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
+  if (hi > 24) { k_gs_update_dots<24, 32><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
   return (int)cudaGetLastError();
 }
 
@@ -464,10 +545,5 @@ template int launch_vnext_in<float>(KrylovState*, const double*, double*, float*
                                     const float*);
 template int launch_vnext_in<double>(KrylovState*, const double*, double*, double*, size_t, cudaStream_t, double*,
                                      const float*);
-
-// done and epoch (adjacent) to pinned host memory
-int launch_status_copy(const KrylovState* st, int* hst, cudaStream_t s) {
-  return (int)cudaMemcpyAsync(hst, &st->done, 2 * sizeof(int), cudaMemcpyDeviceToHost, s);
-}
 
 }  // namespace vfs

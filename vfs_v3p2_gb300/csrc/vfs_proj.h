@@ -84,6 +84,7 @@ struct KrylovState {
   double* hacc;   // m+1 accumulated dots of the column
   double* vs;     // m+1 column scales: basis vector q is vs[q] * V_q
   int orth2;      // 1: CGS2 (columns stored normalised, vs = 1)
+  unsigned ticket[1];  // blocks of the running reduction that have arrived (0 between launches)
 };
 
 // parts must hold nblocks * (m + 2) doubles.
@@ -92,28 +93,31 @@ int launch_norm_init(KrylovState* st, const double* r, size_t n, double* parts, 
 int launch_vec_scale_first(KrylovState* st, const double* r, double* v0, size_t n, cudaStream_t s);
 int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
                     cudaStream_t s);
-int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int pass, cudaStream_t s);
+// close: the launch's last block closes the Arnoldi column (what
+// launch_arnoldi_finish does as its own launch) and writes done and epoch to
+// the pinned host ints hst.
+int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int close, int* hst,
+                     cudaStream_t s);
 // In the Krylov kernels nv < 0 (and vn == nullptr) mean "take the column
 // count from the device state", so one iteration is a fixed launch sequence.
 // second CGS pass fused with the first update (capacity <= 32); returns -1 beyond
 int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s,
                           int cap = 32);
 template <typename T>
-int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, cudaStream_t s,
-                      const float* dinv = nullptr);
+int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, int close, int* hst,
+                      cudaStream_t s, const float* dinv = nullptr);
 template <typename T>
 int launch_vnext_in(KrylovState* st, const double* w, double* vn, T* out, size_t n, cudaStream_t s, double* V = nullptr,
                     const float* dinv = nullptr);
 // w = A z (aj-scaled FP64 operator, z in T) and Z[st->j] = z on the interior
 template <typename T>
 int launch_apply64_krylov(const OpView<double>& A, const T* z, T* Z, const KrylovState* st, double* w, cudaStream_t s);
-int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, cudaStream_t s);
+int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, int* hst, cudaStream_t s);
 int launch_vnext(KrylovState* st, const double* w, double* vn, size_t n, cudaStream_t s);
 int launch_lsq_update(KrylovState* st, cudaStream_t s);
 template <typename T>
 int launch_x_update(KrylovState* st, const T* Z, size_t n, double* x, cudaStream_t s);
 int launch_restart_reset(KrylovState* st, cudaStream_t s);
-int launch_status_copy(const KrylovState* st, int* hst, cudaStream_t s);
 int launch_norm2(const double* v, size_t n, double* parts, double* out, cudaStream_t s);
 
 }  // namespace vfs
