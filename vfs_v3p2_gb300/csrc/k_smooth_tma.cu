@@ -281,7 +281,7 @@ __global__ void __launch_bounds__(TMA_NT, 1)
       for (int idx = tid; idx < TMA_TW * nj; idx += TMA_NCONS) {
         const int jl = idx / TMA_TW, ic = min(i0 + idx % TMA_TW, d.mx - 2);
         const int c = cidx(d, ic, 1 + jl, k);
-        const float v = __ldg(xi + c) + omega * su[idx];
+        const float v = fmaf(omega, su[idx], __ldg(xi + c));
         if (i0 + idx % TMA_TW <= d.mx - 2) xo[c] = v;
       }
       consumers_sync();  // the next tile restages su, sp, sl

@@ -185,23 +185,26 @@ struct FaceData {
 // aj of the face form with its code bits cleared, and the code bits.
 __device__ __forceinline__ float face_aj(float v) { return __int_as_float(__float_as_int(v) & ~0xF); }
 __device__ __forceinline__ unsigned face_code(float v) { return (unsigned)__float_as_int(v) & 0xFu; }
+// Every contraction is written out, and the product with aj is one the
+// compiler may not contract into the caller's b - (A x): the kernels that
+// share this row must round alike whatever surrounds it.
 __device__ __forceinline__ float face_row(const FaceData& f, const float* x) {
   const float xc = x[CP], xe = x[EP], xw = x[WP], xn = x[NP], xs = x[SP], xt = x[TP], xb = x[BP];
   const float xte = x[TE], xbe = x[BE], xtw = x[TW], xbw = x[BW];
   // +i face of c: the pair (C, E) at k+1 / k / k-1
   const float ce = xc + xe, te = xt + xte, be = xb + xbe;
-  const float Fic = f.fic.x * (xe - xc) + f.fic.y * (((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be));
+  const float Fic = fmaf(f.fic.x, xe - xc, f.fic.y * (((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be)));
   // +i face of c-i: the pair (W, C)
   const float wc = xw + xc, tw = xtw + xt, bw = xbw + xb;
-  const float Fiw = f.fiw.x * (xc - xw) + f.fiw.y * (((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw));
+  const float Fiw = fmaf(f.fiw.x, xc - xw, f.fiw.y * (((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw)));
   // +k face of c: the pair (C, T) at i+1 / i / i-1
   const float ct = xc + xt, ete = xe + xte, wtw = xw + xtw;
-  const float Fkc = f.fkc.x * (xt - xc) + f.fkc.y * (((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw));
+  const float Fkc = fmaf(f.fkc.x, xt - xc, f.fkc.y * (((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw)));
   // +k face of c-k: the pair (B, C)
   const float bc = xb + xc, eb = xbe + xe, wb = xbw + xw;
-  const float Fkb = f.fkb.x * (xc - xb) + f.fkb.y * (((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb));
-  const float Fj = f.gjc * (xn - xc) - f.gjs * (xc - xs);
-  return f.aj * ((Fic - Fiw) + Fj + (Fkc - Fkb));
+  const float Fkb = fmaf(f.fkb.x, xc - xb, f.fkb.y * (((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb)));
+  const float Fj = fmaf(f.gjc, xn - xc, -(f.gjs * (xc - xs)));
+  return __fmul_rn(f.aj, (Fic - Fiw) + Fj + (Fkc - Fkb));
 }
 // The face data and the 11 stencil values of interior cell (i, j, k), every
 // load issued before any arithmetic (periodic wraps as in stencil_gather).
@@ -249,11 +252,11 @@ struct FaceX {
   float jis, jks;  // the same of the +j face of c-j
   float kjc, kjb;  // j cross weight of the +k faces of c and c-k
 };
-// w (U - L) of a cross term: U is the pair at +1 or, one-sided, the face's
-// centre pair ctr; L the pair at -1 or the centre pair.
-__device__ __forceinline__ float face_cross(float w, float ctr, float up, float dn) {
+// a + w (U - L) of a cross term: U is the pair at +1 or, one-sided, the
+// face's centre pair ctr; L the pair at -1 or the centre pair.
+__device__ __forceinline__ float face_cross(float w, float ctr, float up, float dn, float a) {
   const unsigned q = face_xc(w);
-  return face_xw(w) * (((q & 1u) ? ctr : up) - ((q & 2u) ? ctr : dn));
+  return fmaf(face_xw(w), ((q & 1u) ? ctr : up) - ((q & 2u) ? ctr : dn), a);
 }
 // Row of the general face form from the 19 stencil values: aj times the
 // divergence of the six face fluxes, each with its normal term and both
@@ -265,27 +268,27 @@ __device__ __forceinline__ float face_row_all(const FaceData& f, const FaceX& e,
   const float xne = x[NE], xse = x[SE], xnw = x[NW], xsw = x[SW], xtn = x[TN], xbn = x[BN], xts = x[TS], xbs = x[BS];
   // +i face of c: the pair (C, E) at k+1 / k-1 and at j+1 / j-1
   const float ce = xc + xe, te = xt + xte, be = xb + xbe;
-  const float Fic = f.fic.x * (xe - xc) + f.fic.y * (((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be)) +
-                    face_cross(e.ijc, ce, xn + xne, xs + xse);
+  const float Fic = face_cross(e.ijc, ce, xn + xne, xs + xse,
+                               fmaf(f.fic.x, xe - xc, f.fic.y * (((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be))));
   // +i face of c-i: the pair (W, C)
   const float wc = xw + xc, tw = xtw + xt, bw = xbw + xb;
-  const float Fiw = f.fiw.x * (xc - xw) + f.fiw.y * (((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw)) +
-                    face_cross(e.ijw, wc, xnw + xn, xsw + xs);
+  const float Fiw = face_cross(e.ijw, wc, xnw + xn, xsw + xs,
+                               fmaf(f.fiw.x, xc - xw, f.fiw.y * (((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw))));
   // +j face of c: the pair (C, N) at i+1 / i-1 and at k+1 / k-1
   const float cn = xc + xn;
-  const float Fjc = f.gjc * (xn - xc) + face_cross(e.jic, cn, xe + xne, xw + xnw) + face_cross(e.jkc, cn, xt + xtn, xb + xbn);
+  const float Fjc = face_cross(e.jkc, cn, xt + xtn, xb + xbn, face_cross(e.jic, cn, xe + xne, xw + xnw, f.gjc * (xn - xc)));
   // +j face of c-j: the pair (S, C)
   const float sc = xs + xc;
-  const float Fjs = f.gjs * (xc - xs) + face_cross(e.jis, sc, xse + xe, xsw + xw) + face_cross(e.jks, sc, xts + xt, xbs + xb);
+  const float Fjs = face_cross(e.jks, sc, xts + xt, xbs + xb, face_cross(e.jis, sc, xse + xe, xsw + xw, f.gjs * (xc - xs)));
   // +k face of c: the pair (C, T) at i+1 / i-1 and at j+1 / j-1
   const float ct = xc + xt, ete = xe + xte, wtw = xw + xtw;
-  const float Fkc = f.fkc.x * (xt - xc) + f.fkc.y * (((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw)) +
-                    face_cross(e.kjc, ct, xn + xtn, xs + xts);
+  const float Fkc = face_cross(e.kjc, ct, xn + xtn, xs + xts,
+                               fmaf(f.fkc.x, xt - xc, f.fkc.y * (((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw))));
   // +k face of c-k: the pair (B, C)
   const float bc = xb + xc, eb = xbe + xe, wb = xbw + xw;
-  const float Fkb = f.fkb.x * (xc - xb) + f.fkb.y * (((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb)) +
-                    face_cross(e.kjb, bc, xbn + xn, xbs + xs);
-  return f.aj * ((Fic - Fiw) + (Fjc - Fjs) + (Fkc - Fkb));
+  const float Fkb = face_cross(e.kjb, bc, xbn + xn, xbs + xs,
+                               fmaf(f.fkb.x, xc - xb, f.fkb.y * (((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb))));
+  return __fmul_rn(f.aj, (Fic - Fiw) + (Fjc - Fjs) + (Fkc - Fkb));
 }
 // The row's S and N coefficients (its j-line couplings) over aj: the
 // coefficients of x_S and x_N in face_row_all's divergence -- the j faces'
@@ -884,7 +887,7 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
     const int i = min(i0 + il, d.mx - 2), j = 1 + jl;
     const int c = k * d.mx * d.my + j * d.mx + i;
     const T x0 = xi ? __ldg(xi + c) : T(0);
-    const T v = x0 + omega * su[idx];
+    const T v = fma(omega, su[idx], x0);
     if (i0 + il <= d.mx - 2) xo[c] = v;
   }
 }
@@ -1004,7 +1007,7 @@ __device__ __forceinline__ void smooth_tile_w(const OpView<float>& A, const floa
     const int l = idx & 31, jl = idx >> 5;
     const int i = min(i0 - 1 + l, d.mx - 2);
     const int c = k * sz + (1 + jl) * sy + i;
-    const float v = __ldg(xi + c) + omega * su[idx];
+    const float v = fmaf(omega, su[idx], __ldg(xi + c));
     if (l >= 1 && l <= SMOOTH_W_TW && i0 - 1 + l <= d.mx - 2) xo[c] = v;
   }
 }
@@ -1096,6 +1099,16 @@ __device__ __forceinline__ void resrestrict_tile(const OpView<T>& A, const T* __
 }
 
 
+// Trilinear value of MyInterpolation from the coarse cell (c), its neighbours
+// at +-1 in j, in i and in both, and the same four at +-1 in k: weights
+// (9 3 3 1) x (3 1) / 64, every contraction written out (see face_row).
+template <typename T>
+__device__ __forceinline__ T prolong_value(T c0, T j0, T i0, T ij0, T c1, T j1, T i1, T ij1) {
+  const T a = fma(i0, T(3), fma(j0, T(3), c0 * T(9))) + ij0;
+  const T b = fma(i1, T(3), fma(j1, T(3), c1 * T(9))) + ij1;
+  return fma(a, T(3) / T(64), b * (T(1) / T(64)));
+}
+
 // One tile of the prolongation (see k_prolong): fine columns
 // (1 + TX bx + tx, 1 + TY by + ty), planes 1 + KCHUNK bz ...
 template <typename T>
@@ -1128,10 +1141,9 @@ __device__ __forceinline__ void prolong_tile(const Dims& f, const uint8_t* __res
     const int kc = sk ? k : (k + 1) / 2;
     const int ia = (cd[u] & 3) - 1, ja = ((cd[u] >> 2) & 3) - 1, ka = ((cd[u] >> 4) & 3) - 1;
 #define X(a, b, cc) xc[cidx(c, a, b, cc)]
-    const T v = (X(ic, jc, kc) * T(9) + X(ic, jc + ja, kc) * T(3) + X(ic + ia, jc, kc) * T(3) + X(ic + ia, jc + ja, kc)) *
-                    (T(3) / T(64)) +
-                (X(ic, jc, kc + ka) * T(9) + X(ic, jc + ja, kc + ka) * T(3) + X(ic + ia, jc, kc + ka) * T(3) +
-                 X(ic + ia, jc + ja, kc + ka)) / T(64);
+    const T v = prolong_value<T>(X(ic, jc, kc), X(ic, jc + ja, kc), X(ic + ia, jc, kc), X(ic + ia, jc + ja, kc),
+                                 X(ic, jc, kc + ka), X(ic, jc + ja, kc + ka), X(ic + ia, jc, kc + ka),
+                                 X(ic + ia, jc + ja, kc + ka));
 #undef X
     const T vv = (cd[u] & 0x80) ? T(0) : v;
     if (in && k0 + u <= f.mz - 2) xf[cidx(f, i1, j1, k)] = add ? xo[u] + vv : vv;

@@ -22,6 +22,7 @@
 #include <string>
 #include <vector>
 
+#include "mg_coarse.h"
 #include "mg_group.h"
 #include "mg_tiles.cuh"
 #include "mg_stage.h"
@@ -460,6 +461,7 @@ struct MGCfg {
   bool face;       // FP32 face form on 11-slot levels (FP32 multigrid only)
   bool solo;       // the grid's solve runs alone
   int stage;       // how the finest face-form sweeps stage their operands (SweepStage)
+  int cluster = 0;  // levels 1 .. cluster (and the coarsest) run as one cluster launch (0: none)
   int pre(int l) const { return l == top ? nu1 : nu1c; }
   int post(int l) const { return l == top ? nu2 : nu2c; }
 };
@@ -529,8 +531,78 @@ int level_writes(const Grid& g, int l, const MGCfg& c) {
   return c.pre(l) + (c.pre(l) == 0 ? 1 : 0) + c.post(l);
 }
 
+// The cluster launch's arguments for the levels up to `top` (its right-hand
+// side, solution and cluster size left to the caller).
+void coarse_args(Grid& g, int top, const MGCfg& c, CvArgs& a) {
+  a = CvArgs{};
+  a.top = top;
+  for (int l = 0; l <= top; l++) {
+    Level& L = g.lev[l];
+    CvLevel& v = a.lev[l];
+    v.d = L.d;
+    v.ffi = L.ffi;
+    v.ffk = L.ffk;
+    v.ffj = L.ffj;
+    v.faj = L.faj;
+    v.lf = L.lf32;
+    v.rw = L.rw32;
+    v.nvert = L.nvert;
+    v.pcode = L.pcode;
+    v.npre = c.pre(l);
+    v.npost = c.post(l);
+  }
+  a.Binv = g.lev[0].Binv32;
+  a.n0 = g.lev[0].nco;
+  a.b0 = g.lev[0].b32;
+  for (int q = 0; q < CV_MAXSWEEP; q++) {
+    a.wpre[0][q] = q < c.nu1c ? (float)c.wc[0][q] : 0.f;
+    a.wpost[0][q] = q < c.nu2c ? (float)c.wc[1][q] : 0.f;
+    a.wpre[1][q] = q < c.nu1 ? (float)c.wf[0][q] : 0.f;
+    a.wpost[1][q] = q < c.nu2 ? (float)c.wf[1][q] : 0.f;
+  }
+  a.topset = top == c.top ? 1 : 0;
+}
+
+// Highest level the cluster launch takes: the FP32 face form's 11-slot
+// levels under full coarsening, with a dense coarsest solve that fits every
+// block, at least one sweep on each side, and room in shared memory.  A
+// probed or debugged solve runs the levels' own launches, which it times or
+// checks one by one (the same bits).
+#ifndef VFS_CV_MAXCELLS
+#define VFS_CV_MAXCELLS 70000
+#endif
+int coarse_top(Grid& g, const MGCfg& c) {
+  if (!c.solo || g_probe.kind != 0 || g_debug || !c.face || c.half || g.si || g.sj || g.sk) return 0;
+  if (!g.lev[0].Binv32 || g.lev[0].nco < 1 || g.lev[0].nco > CV_DENSE_MAX) return 0;
+  if (c.nu1c < 1 || c.nu2c < 1 || c.nu1c > CV_MAXSWEEP || c.nu2c > CV_MAXSWEEP) return 0;
+  int top = 0;
+  for (int l = 1; l < g.L && l < CV_MAXLEV; l++) {
+    const bool sweeps = l != c.top || (c.nu1 >= 1 && c.nu2 >= 1 && c.nu1 <= CV_MAXSWEEP && c.nu2 <= CV_MAXSWEEP);
+    if (!face_level(g.lev[l]) || !sweeps || n_interior(g.lev[l].d) > VFS_CV_MAXCELLS) break;
+    top = l;
+  }
+  for (; top > 0; top--) {
+    CvArgs a;
+    coarse_args(g, top, c, a);
+    if (cv_cluster(a)) return top;
+  }
+  return 0;
+}
+
 template <typename T>
 T* vcycle(Grid& g, int l, T* b, T* xa, T* xb, const MGCfg& c, const int* skip, cudaStream_t s) {
+  if constexpr (sizeof(T) == 4) {
+    if (l > 0 && l == c.cluster) {
+      CvArgs a;
+      coarse_args(g, l, c, a);
+      cv_cluster(a);
+      a.b = b;
+      a.x = xa;
+      a.skip = skip;
+      dbg("coarse_vcycle", l, launch_coarse_vcycle(a, s), s);
+      return xa;
+    }
+  }
   Level& L = g.lev[l];
   const bool half = sizeof(T) == 4 && c.half;
   const bool face = sizeof(T) == 4 && !half && c.face;
@@ -655,6 +727,7 @@ int precond(vfs_ctx* ctx, Grid& g, const vfs_solve_params& p, const double* v, T
   T* bf = bbuf<T>(F);
   MGCfg mc = mgcfg(p, g.L - 1, g.half_ok);
   mc.solo = solo;
+  mc.cluster = coarse_top(g, mc);
   const float* dinv = dinv_sel<T>(F, mc.half);
   if (with_input) dbg("scale_in", g.L - 1, launch_scale_in<T>(F.d, nullptr, v, bf, skip, s, dinv), s);
   T* res = vcycle<T>(g, g.L - 1, bf, z, tmp, mc, skip, s);
@@ -759,6 +832,7 @@ void issue_iteration(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv 
   Level& F = g.lev[g.L - 1];
   MGCfg mc = mgcfg(p, g.L - 1, g.half_ok);
   mc.solo = g.solo;
+  mc.cluster = coarse_top(g, mc);
   vcycle<T>(g, g.L - 1, bbuf<T>(F), xbuf<T>(F)[0], xbuf<T>(F)[1], mc, &g.st->done, s);
   issue_krylov<T>(g, p, s, nv);
 }
