@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_apply64_krylov(OpV
   if (skipped(A.skip)) return;
   T* zj = Z + (size_t)st->j * ncell(A.d);
   const double vs = st->vs[st->j];
-  TILE_LOOP(A.d) {
+  TILE_LOOP_Z(A.d, plane_block(A.flip, blockIdx.z, gridDim.z)) {
     const double s = stencil_clamped<MASK, double>(A.d, A.coef, z, i, j, k);
     if (!_in) continue;
     const size_t c = cidx(A.d, i, j, k);
@@ -106,8 +106,9 @@ __global__ void __launch_bounds__(TX* TY) k_apply_face(OpView<float> A, const fl
     float xv[19];
     if (all) {
       FaceX e;
+      float sc, nc;
       face_gather_all(A, x, i, j, k, f, e, xv);
-      y[cidx(A.d, i, j, k)] = face_row_all(f, e, xv);
+      y[cidx(A.d, i, j, k)] = face_row_all(f, e, xv, sc, nc);
     } else {
       face_gather(A, x, i, j, k, f, xv);
       y[cidx(A.d, i, j, k)] = face_row(f, xv);
@@ -127,17 +128,44 @@ __global__ void __launch_bounds__(VFS_SMOOTH_NT, PAIR ? VFS_SMOOTH_MINB_HALF : (
              T* __restrict__ xo, T omega, int TW) {
   if (skipped(A.skip)) return;
   extern __shared__ unsigned char smraw[];
-  smooth_tile<MASK, T, TC, PAIR, UU, ZG>(A, lf, xi, b, xo, omega, TW, blockIdx.x, blockIdx.y, smraw);
+  smooth_tile<MASK, T, TC, PAIR, UU, ZG>(A, lf, xi, b, xo, omega, TW, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y),
+                                         smraw);
 }
 
-// The face-form sweep with warp-row neighbours (smooth_tile_w): 30-column tiles.
-template <int U>
+// The face-form sweeps with warp-row neighbours: 30-column tiles; two rows a
+// warp and four blocks per SM on the 11-slot form (smooth_tile_w), four rows
+// and two blocks on the general one (smooth_tile_wg; 512x256x256: 674 us one
+// cell per thread, 1 row 638, 2 rows 619, 4 rows 554, 16 warps a block 599).
+// What limits both is L1: the line arrays leave 56 KB of it per SM, and a load
+// in flight holds its lines (4 KB more shared memory a block, padded lines,
+// cost 48 -> 69 us and 554 -> 838 us).
 __global__ void __launch_bounds__(VFS_SMOOTH_NT, VFS_SMOOTH_W_MINB)
     k_smooth_w(OpView<float> A, const float* __restrict__ lf, const float* __restrict__ xi,
                const float* __restrict__ b, float* __restrict__ xo, float omega) {
   if (skipped(A.skip)) return;
   extern __shared__ unsigned char smraw[];
-  smooth_tile_w<U>(A, lf, xi, b, xo, omega, blockIdx.x, blockIdx.y, smraw);
+  smooth_tile_w<VFS_SMOOTH_W_U>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), smraw);
+}
+__global__ void __launch_bounds__(VFS_SMOOTH_NT, 2)
+    k_smooth_wg(OpView<float> A, const float* __restrict__ lf, const float* __restrict__ xi,
+                const float* __restrict__ b, float* __restrict__ xo, float omega) {
+  if (skipped(A.skip)) return;
+  extern __shared__ float sm[];
+  smooth_tile_wg<4>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), sm);
+}
+static int smooth_w_launch(const OpView<float>& A, const float* lf, const float* xi, const float* b, float* xo,
+                           float omega, cudaStream_t s) {
+  static const cudaError_t attr = [] {
+    const cudaError_t e = cudaFuncSetAttribute(k_smooth_w, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_smooth_wg, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+  }();
+  if (attr != cudaSuccess) return (int)attr;
+  const dim3 g((A.d.mx - 2 + SMOOTH_W_TW - 1) / SMOOTH_W_TW, A.d.mz - 2);
+  const size_t sm = smooth_smem<float>(32, A.d.my - 2);
+  if (A.ffc) k_smooth_wg<<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
+  else k_smooth_w<<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
+  ++g_launches;
+  return (int)cudaGetLastError();
 }
 template <unsigned MASK, typename T, typename TC, bool PAIR, int UU, bool ZG>
 static void smooth_attrs1() {
@@ -163,6 +191,12 @@ static void smooth_launch(bool small, dim3 g, size_t sm, cudaStream_t s, const O
   else if (small && !PAIR)
     k_smooth<MASK, T, TC, PAIR, VFS_SMOOTH_U_SMALL, false><<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega, tw);
   else k_smooth<MASK, T, TC, PAIR, VFS_SMOOTH_U, false><<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega, tw);
+}
+
+// The rows' lines must fit: 48 KB a block at four blocks per SM, 96 KB at two
+// (longer lines take narrower tiles of the one-cell-per-thread sweep).
+static bool smooth_w_fits(const Dims& d, bool ch) {
+  return smooth_smem<float>(32, d.my - 2) <= (size_t)(ch ? 48 : 96) * 1024;
 }
 
 template <typename T>
@@ -201,16 +235,12 @@ int launch_smooth(const OpView<T>& A, const T* lf, const T* xi, const T* b, T* x
   const bool small = sizeof(T) == 4 && solo && (size_t)g.x * g.y < 2 * 152;  // (FP64: spills at two cells)
   bool done = false;
   if constexpr (sizeof(T) == 4) {
-    if (A.ffi && ch && xi && cols == 0 && tw == 32 && !small && VFS_SMOOTH_W_U > 0) {
-      // automatic full-width tiles on the face form: the warp-row sweep
-      static bool wattr = false;
-      if (!wattr) {
-        cudaFuncSetAttribute(k_smooth_w<VFS_SMOOTH_W_U>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        wattr = true;
-      }
-      const dim3 gw((ni + SMOOTH_W_TW - 1) / SMOOTH_W_TW, nk);
-      k_smooth_w<VFS_SMOOTH_W_U><<<gw, VFS_SMOOTH_NT, smooth_smem<float>(32, nj), s>>>(A, lf, xi, b, xo, omega);
-      done = true;
+    // automatic tiles on the face form: the warp-row sweep, on full-width
+    // tiles (11-slot form) or two blocks per SM (general form, whose lines of
+    // more than 128 rows have narrower tiles otherwise)
+    const bool wide = ch ? tw == 32 && !small : ni >= SMOOTH_W_TW && (size_t)((ni + 29) / 30) * nk >= 2 * 152;
+    if (A.ffi && (ch || A.ffc) && xi && cols == 0 && wide && smooth_w_fits(A.d, ch)) {
+      return smooth_w_launch(A, lf, xi, b, xo, omega, s);
     } else if (A.ffi && ch) {
       smooth_launch<MASK_CH, T, FaceOp, false>(small, g, sm, s, A, lf, xi, b, xo, omega, tw);
       done = true;
@@ -423,7 +453,8 @@ __global__ void __launch_bounds__(256, VFS_STENCIL_MINB) k_resrestrict_tiled(OpV
                                                            T* __restrict__ xc) {
   if (skipped(A.skip)) return;
   __shared__ T sr[2][8][64];
-  resrestrict_tile<MASK, T, TC>(A, x, b, rw, c, nvc, bc, xc, blockIdx.x, blockIdx.y, blockIdx.z, sr);
+  resrestrict_tile<MASK, T, TC>(A, x, b, rw, c, nvc, bc, xc, blockIdx.x, blockIdx.y,
+                                plane_block(A.flip, blockIdx.z, gridDim.z), sr);
 }
 
 template <typename T, typename TC>
@@ -509,17 +540,19 @@ int launch_restrict(const Dims& f, const T* x, const double* nvf, const Dims& c,
 template <typename T>
 __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_prolong(Dims f, const uint8_t* __restrict__ code, Dims c,
                                                                       const T* __restrict__ xc, T* __restrict__ xf,
-                                                                      int add, int si, int sj, int sk, const int* skip) {
+                                                                      int add, int si, int sj, int sk, const int* skip,
+                                                                      int flip) {
   if (skipped(skip)) return;
-  prolong_tile<T>(f, code, c, xc, xf, add, si, sj, sk, blockIdx.x, blockIdx.y, blockIdx.z, threadIdx.x, threadIdx.y);
+  prolong_tile<T>(f, code, c, xc, xf, add, si, sj, sk, blockIdx.x, blockIdx.y, plane_block(flip, blockIdx.z, gridDim.z),
+                  threadIdx.x, threadIdx.y);
 }
 
 template <typename T>
 int launch_prolong(const Dims& f, const uint8_t* code, const Dims& c, const T* xc, T* xf, int add, const int* skip,
-                   cudaStream_t s) {
+                   cudaStream_t s, int flip) {
   // semi-coarsening flags are implied by equal extents
   const int si = (c.mx == f.mx), sj = (c.my == f.my), sk = (c.mz == f.mz);
-  k_prolong<T><<<tile_grid(f), dim3(TX, TY), 0, s>>>(f, code, c, xc, xf, add, si, sj, sk, skip); ++g_launches;
+  k_prolong<T><<<tile_grid(f), dim3(TX, TY), 0, s>>>(f, code, c, xc, xf, add, si, sj, sk, skip, flip); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -576,7 +609,7 @@ int launch_scale_in(const Dims& d, const double* aj, const double* v, T* out, co
                                            const double*, int, int, int, T*, T*, cudaStream_t);                       \
   template int launch_restrict<T>(const Dims&, const T*, const double*, const Dims&, const double*, int, int, int, T*, \
                                   cudaStream_t);                                                                      \
-  template int launch_prolong<T>(const Dims&, const uint8_t*, const Dims&, const T*, T*, int, const int*, cudaStream_t); \
+  template int launch_prolong<T>(const Dims&, const uint8_t*, const Dims&, const T*, T*, int, const int*, cudaStream_t, int); \
   template int launch_coarse_gemv<T>(const Dims&, const T*, int, const T*, T*, const T*, const int*, cudaStream_t);  \
   template int launch_scale_in<T>(const Dims&, const double*, const double*, T*, const int*, cudaStream_t,             \
                                   const float*);

@@ -26,11 +26,17 @@ __host__ __forceinline__ dim3 tile_grid(const Dims& d) {
   return dim3((ni + TX - 1) / TX, (nj + TY - 1) / TY, (nk + KCHUNK - 1) / KCHUNK);
 }
 
-#define TILE_LOOP(d)                                                       \
+// The k-plane block a block works on: the last first when flipped.  Kernels
+// that follow one another over a large level walk it in turn forwards and
+// backwards, so that each starts on the planes the one before left in L2.
+__device__ __forceinline__ int plane_block(int flip, int b, int n) { return flip ? n - 1 - b : b; }
+
+#define TILE_LOOP(d) TILE_LOOP_Z(d, blockIdx.z)
+#define TILE_LOOP_Z(d, bz)                                                 \
   const int i = 1 + blockIdx.x * TX + threadIdx.x;                         \
   const int j = 1 + blockIdx.y * TY + threadIdx.y;                         \
   const bool _in = (i <= (d).mx - 2) && (j <= (d).my - 2);                 \
-  const int _k0 = 1 + blockIdx.z * KCHUNK;                                 \
+  const int _k0 = 1 + (bz) * KCHUNK;                                       \
   const int _k1 = min(_k0 + KCHUNK, (d).mz - 1);                           \
   for (int k = _k0; k < _k1; k++)
 
@@ -206,6 +212,31 @@ __device__ __forceinline__ float face_row(const FaceData& f, const float* x) {
   const float Fj = fmaf(f.gjc, xn - xc, -(f.gjs * (xc - xs)));
   return __fmul_rn(f.aj, (Fic - Fiw) + Fj + (Fkc - Fkb));
 }
+// The same with the one-sided cases (beside bodies and walls: a pair replaced
+// by the face's own) branched around elsewhere, 28 instructions a row.  Pays
+// on the sweeps that one cell's instructions bound (small levels: 128x64x64
+// 14.7 -> 13.8 us); where loads bound a kernel, the branch keeps them from
+// moving up (the finest restriction 46.7 -> 48.8 us).
+__device__ __forceinline__ float face_row_b(const FaceData& f, const float* x) {
+  const float xc = x[CP], xe = x[EP], xw = x[WP], xn = x[NP], xs = x[SP], xt = x[TP], xb = x[BP];
+  const float xte = x[TE], xbe = x[BE], xtw = x[TW], xbw = x[BW];
+  const float te = xt + xte, be = xb + xbe, tw = xtw + xt, bw = xbw + xb;
+  const float ete = xe + xte, wtw = xw + xtw, eb = xbe + xe, wb = xbw + xw;
+  float pi = te - be, pw = tw - bw, pk = ete - wtw, pb = eb - wb;
+  if (((f.cc & 0xFu) | (f.cw & 3u) | (f.cb & 0xCu)) != 0u) {
+    const float ce = xc + xe, wc = xw + xc, ct = xc + xt, bc = xb + xc;
+    pi = ((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be);
+    pw = ((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw);
+    pk = ((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw);
+    pb = ((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb);
+  }
+  const float Fic = fmaf(f.fic.x, xe - xc, f.fic.y * pi);
+  const float Fiw = fmaf(f.fiw.x, xc - xw, f.fiw.y * pw);
+  const float Fkc = fmaf(f.fkc.x, xt - xc, f.fkc.y * pk);
+  const float Fkb = fmaf(f.fkb.x, xc - xb, f.fkb.y * pb);
+  const float Fj = fmaf(f.gjc, xn - xc, -(f.gjs * (xc - xs)));
+  return __fmul_rn(f.aj, (Fic - Fiw) + Fj + (Fkc - Fkb));
+}
 // The face data and the 11 stencil values of interior cell (i, j, k), every
 // load issued before any arithmetic (periodic wraps as in stencil_gather).
 __device__ __forceinline__ void face_gather(const OpView<float>& A, const float* __restrict__ x, int i, int j, int k,
@@ -254,56 +285,69 @@ struct FaceX {
 };
 // a + w (U - L) of a cross term: U is the pair at +1 or, one-sided, the
 // face's centre pair ctr; L the pair at -1 or the centre pair.
+template <bool SIDED>
 __device__ __forceinline__ float face_cross(float w, float ctr, float up, float dn, float a) {
+  if (!SIDED) return fmaf(w, up - dn, a);
   const unsigned q = face_xc(w);
   return fmaf(face_xw(w), ((q & 1u) ? ctr : up) - ((q & 2u) ? ctr : dn), a);
 }
 // Row of the general face form from the 19 stencil values: aj times the
 // divergence of the six face fluxes, each with its normal term and both
 // cross terms (poisson.c:1173-1558: the i+1 face's g12 and g13 pairs, the
-// j+1 face's g21 and g23 pairs, the k+1 face's g31 and g32 pairs).
-__device__ __forceinline__ float face_row_all(const FaceData& f, const FaceX& e, const float* x) {
+// j+1 face's g21 and g23 pairs, the k+1 face's g31 and g32 pairs); and the
+// row's S and N coefficients (its j-line couplings) over aj, the
+// coefficients of x_S and x_N in that divergence: the j faces' normal
+// weights, the j cross terms of the i and k faces (the pair at j-1 or j+1
+// unless the regime takes the centre pair) and the j faces' cross terms
+// whose centre pair is the pair they take.  SIDED: some cross term takes a
+// centre pair (its codes are read); else every code is 0.
+template <bool SIDED>
+__device__ __forceinline__ float face_row_gen(const FaceData& f, const FaceX& e, const float* x, float& s, float& n) {
   const float xc = x[CP], xe = x[EP], xw = x[WP], xn = x[NP], xs = x[SP], xt = x[TP], xb = x[BP];
   const float xte = x[TE], xbe = x[BE], xtw = x[TW], xbw = x[BW];
   const float xne = x[NE], xse = x[SE], xnw = x[NW], xsw = x[SW], xtn = x[TN], xbn = x[BN], xts = x[TS], xbs = x[BS];
-  // +i face of c: the pair (C, E) at k+1 / k-1 and at j+1 / j-1
-  const float ce = xc + xe, te = xt + xte, be = xb + xbe;
-  const float Fic = face_cross(e.ijc, ce, xn + xne, xs + xse,
-                               fmaf(f.fic.x, xe - xc, f.fic.y * (((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be))));
-  // +i face of c-i: the pair (W, C)
-  const float wc = xw + xc, tw = xtw + xt, bw = xbw + xb;
-  const float Fiw = face_cross(e.ijw, wc, xnw + xn, xsw + xs,
-                               fmaf(f.fiw.x, xc - xw, f.fiw.y * (((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw))));
-  // +j face of c: the pair (C, N) at i+1 / i-1 and at k+1 / k-1
-  const float cn = xc + xn;
-  const float Fjc = face_cross(e.jkc, cn, xt + xtn, xb + xbn, face_cross(e.jic, cn, xe + xne, xw + xnw, f.gjc * (xn - xc)));
-  // +j face of c-j: the pair (S, C)
-  const float sc = xs + xc;
-  const float Fjs = face_cross(e.jks, sc, xts + xt, xbs + xb, face_cross(e.jis, sc, xse + xe, xsw + xw, f.gjs * (xc - xs)));
-  // +k face of c: the pair (C, T) at i+1 / i-1 and at j+1 / j-1
-  const float ct = xc + xt, ete = xe + xte, wtw = xw + xtw;
-  const float Fkc = face_cross(e.kjc, ct, xn + xtn, xs + xts,
-                               fmaf(f.fkc.x, xt - xc, f.fkc.y * (((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw))));
-  // +k face of c-k: the pair (B, C)
-  const float bc = xb + xc, eb = xbe + xe, wb = xbw + xw;
-  const float Fkb = face_cross(e.kjb, bc, xbn + xn, xbs + xs,
-                               fmaf(f.fkb.x, xc - xb, f.fkb.y * (((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb))));
+  const float ce = xc + xe, te = xt + xte, be = xb + xbe;  // pairs along the +i face of c
+  const float wc = xw + xc, tw = xtw + xt, bw = xbw + xb;  // of c-i
+  const float ct = xc + xt, ete = xe + xte, wtw = xw + xtw;  // along the +k face of c
+  const float bc = xb + xc, eb = xbe + xe, wb = xbw + xw;    // of c-k
+  float pi = te - be, pw = tw - bw, pk = ete - wtw, pb = eb - wb;
+  if (SIDED) {
+    pi = ((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be);
+    pw = ((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw);
+    pk = ((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw);
+    pb = ((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb);
+  }
+  const float Fic = face_cross<SIDED>(e.ijc, ce, xn + xne, xs + xse, fmaf(f.fic.x, xe - xc, f.fic.y * pi));
+  const float Fiw = face_cross<SIDED>(e.ijw, wc, xnw + xn, xsw + xs, fmaf(f.fiw.x, xc - xw, f.fiw.y * pw));
+  const float cn = xc + xn, sc = xs + xc;  // along the +j faces of c and c-j
+  const float Fjc = face_cross<SIDED>(e.jkc, cn, xt + xtn, xb + xbn,
+                                      face_cross<SIDED>(e.jic, cn, xe + xne, xw + xnw, f.gjc * (xn - xc)));
+  const float Fjs = face_cross<SIDED>(e.jks, sc, xts + xt, xbs + xb,
+                                      face_cross<SIDED>(e.jis, sc, xse + xe, xsw + xw, f.gjs * (xc - xs)));
+  const float Fkc = face_cross<SIDED>(e.kjc, ct, xn + xtn, xs + xts, fmaf(f.fkc.x, xt - xc, f.fkc.y * pk));
+  const float Fkb = face_cross<SIDED>(e.kjb, bc, xbn + xn, xbs + xs, fmaf(f.fkb.x, xc - xb, f.fkb.y * pb));
+  if (SIDED) {
+    auto nq1 = [](float w) { return (face_xc(w) & 1u) ? 0.f : face_xw(w); };  // upper pair at +1
+    auto nq2 = [](float w) { return (face_xc(w) & 2u) ? 0.f : face_xw(w); };  // lower pair at -1
+    auto ctr = [](float w) {  // the centre pair: +w as the upper pair, -w as the lower one
+      const unsigned q = face_xc(w);
+      return ((q & 1u) ? face_xw(w) : 0.f) - ((q & 2u) ? face_xw(w) : 0.f);
+    };
+    s = f.gjs - nq2(e.ijc) + nq2(e.ijw) - nq2(e.kjc) + nq2(e.kjb) - ctr(e.jis) - ctr(e.jks);
+    n = f.gjc + nq1(e.ijc) - nq1(e.ijw) + nq1(e.kjc) - nq1(e.kjb) + ctr(e.jic) + ctr(e.jkc);
+  } else {
+    s = f.gjs - e.ijc + e.ijw - e.kjc + e.kjb;
+    n = f.gjc + e.ijc - e.ijw + e.kjc - e.kjb;
+  }
   return __fmul_rn(f.aj, (Fic - Fiw) + (Fjc - Fjs) + (Fkc - Fkb));
 }
-// The row's S and N coefficients (its j-line couplings) over aj: the
-// coefficients of x_S and x_N in face_row_all's divergence -- the j faces'
-// normal weights, the j cross terms of the i and k faces (the pair at j-1 or
-// j+1 unless the regime takes the centre pair) and the j faces' cross terms
-// whose centre pair is the pair they take.
-__device__ __forceinline__ void face_row_sn(const FaceData& f, const FaceX& e, float& s, float& n) {
-  auto nq1 = [](float w) { return (face_xc(w) & 1u) ? 0.f : face_xw(w); };  // upper pair at +1
-  auto nq2 = [](float w) { return (face_xc(w) & 2u) ? 0.f : face_xw(w); };  // lower pair at -1
-  auto ctr = [](float w) {  // the centre pair: +w as the upper pair, -w as the lower one
-    const unsigned q = face_xc(w);
-    return ((q & 1u) ? face_xw(w) : 0.f) - ((q & 2u) ? face_xw(w) : 0.f);
-  };
-  s = f.gjs - nq2(e.ijc) + nq2(e.ijw) - nq2(e.kjc) + nq2(e.kjb) - ctr(e.jis) - ctr(e.jks);
-  n = f.gjc + nq1(e.ijc) - nq1(e.ijw) + nq1(e.kjc) - nq1(e.kjb) + ctr(e.jic) + ctr(e.jkc);
+// As in face_row, the one-sided cases (beside bodies and walls) are branched
+// around elsewhere.
+__device__ __forceinline__ float face_row_all(const FaceData& f, const FaceX& e, const float* x, float& s, float& n) {
+  const unsigned q = face_xc(e.ijc) | face_xc(e.ijw) | face_xc(e.jic) | face_xc(e.jkc) | face_xc(e.jis) |
+                     face_xc(e.jks) | face_xc(e.kjc) | face_xc(e.kjb);
+  if (q | (f.cc & 0xFu) | (f.cw & 3u) | (f.cb & 0xCu)) return face_row_gen<true>(f, e, x, s, n);
+  return face_row_gen<false>(f, e, x, s, n);
 }
 // face_gather plus the cross weights of c, c-i, c-j, c-k and the eight x
 // values face_row leaves out (NE SE NW SW TN BN TS BS), periodic wraps as in
@@ -589,7 +633,7 @@ __device__ __forceinline__ void face_phase1(const OpView<float>& A, const float*
         x11[TP] = xv[u][5]; x11[BP] = xv[u][6]; x11[TE] = xv[u][7]; x11[BE] = xv[u][8]; x11[TW] = xv[u][9];
         x11[BW] = xv[u][10];
       }
-      const float ax = ZG ? 0.f : face_row(f[u], x11);
+      const float ax = ZG ? 0.f : face_row_b(f[u], x11);
       const float a = jl > 0 ? f[u].aj * f[u].gjs : 0.f, cn = jl < nj - 1 ? f[u].aj * f[u].gjc : 0.f;
       su[idx] = live ? (bb[u] - ax) * inv[u] : 0.f;
       sp[idx] = live ? a * inv[u] : 0.f;
@@ -600,7 +644,7 @@ __device__ __forceinline__ void face_phase1(const OpView<float>& A, const float*
 
 // Phase 1 on the general face form (levels with i-j or j-k cross terms):
 // the residual from face_row_all and the line couplings aj times
-// face_row_sn's coefficients (the cross terms add to them; the pivots 1/m are
+// the row's S and N coefficients (the cross terms add to them; the pivots 1/m are
 // factored from the assembled rows).  From a zero guess only aj, the
 // assembled FP32 SP and NP, b and 1/m are read.
 template <int U, bool ZG>
@@ -641,8 +685,7 @@ __device__ __forceinline__ void face_phase1_all(const OpView<float>& A, const fl
       const bool live = (i0 + idx % tw <= d.mx - 2) && aj != 0.f;
       float ax = 0.f;
       if (!ZG) {
-        ax = face_row_all(f[u], e[u], xv[u]);
-        face_row_sn(f[u], e[u], av[u], cv[u]);
+        ax = face_row_all(f[u], e[u], xv[u], av[u], cv[u]);
         av[u] *= aj;
         cv[u] *= aj;
       }
@@ -1012,6 +1055,164 @@ __device__ __forceinline__ void smooth_tile_w(const OpView<float>& A, const floa
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same on the general face form (levels with i-j or j-k cross terms).  A
+// warp takes U consecutive rows, which share their x values and j faces: 15
+// loads a cell at four rows where the one-cell-per-thread gather has 44.
+//
+// Offsets are unsigned bytes from the arrays' uniform bases (one 32-bit add a
+// row and plane instead of a 64-bit product a load): an array of 16-byte
+// entries stays below 2^32 bytes up to 2^28 cells, whose grid (1.2 KB a cell)
+// no card holds.
+// ---------------------------------------------------------------------------
+template <typename V>
+__device__ __forceinline__ V ldb(const V* __restrict__ p, unsigned o) {
+  return __ldg(reinterpret_cast<const V*>(reinterpret_cast<const char*>(p) + o));
+}
+// A warp's place in the tile.
+struct WarpTile {
+  unsigned o, sy, okB, okT;  // byte offsets (4-byte arrays): row 0 of the lane's column, a row, planes k-1 and k+1
+  bool comp;                 // the lane is a cell
+};
+__device__ __forceinline__ WarpTile warp_tile(const Dims& d, int bx, int by) {
+  WarpTile p;
+  const int sz = d.mx * d.my, lane = threadIdx.x & 31, k = 1 + by;
+  int il = SMOOTH_W_TW * bx + lane;
+  p.comp = lane >= 1 && lane <= SMOOTH_W_TW && il <= d.mx - 2;
+  if (d.ip && il == 0) il = d.mx - 2;
+  else if (d.ip && il == d.mx - 1) il = 1;
+  p.o = 4u * (unsigned)(k * sz + min(il, d.mx - 1));
+  p.sy = 4u * (unsigned)d.mx;
+  p.okB = 4u * (unsigned)(((k == 1 && d.kp) ? d.mz - 3 : -1) * sz);
+  p.okT = 4u * (unsigned)(((k == d.mz - 2 && d.kp) ? 3 - d.mz : 1) * sz);
+  return p;
+}
+// Row j = jb + u (u = 0: the row before jl = jb) with the periodic seam, none
+// past the ghost row.
+__device__ __forceinline__ unsigned warp_row(const Dims& d, const WarpTile& p, int j) {
+  const int nj = d.my - 2;
+  return p.o + (unsigned)(j == 0 ? (d.jp ? nj : 0) : (j > nj ? (d.jp && j == nj + 1 ? 1 : nj + 1) : j)) * p.sy;
+}
+__device__ __forceinline__ float from_e(float v) { return __shfl_down_sync(0xFFFFFFFFu, v, 1); }
+__device__ __forceinline__ float from_w(float v) { return __shfl_up_sync(0xFFFFFFFFu, v, 1); }
+
+// Scaled residual and line couplings of row jl into the line arrays.
+__device__ __forceinline__ void put_line(float* su, float* sp, float* sl, int jl, int nj, bool live, float r, float inv,
+                                         float lo, float hi) {
+  const int idx = jl * 32 + (threadIdx.x & 31);
+  su[idx] = live ? r * inv : 0.f;
+  sp[idx] = live && jl > 0 ? lo * inv : 0.f;
+  sl[idx] = live && jl < nj - 1 ? hi * inv : 0.f;
+}
+
+// Rows jb .. jb + U - 1 of a tile, every load issued before any arithmetic.
+template <int U>
+__device__ __forceinline__ void warp_rows(const OpView<float>& A, const WarpTile& p, const float* __restrict__ lf,
+                                          const float* __restrict__ x, const float* __restrict__ b, float* su, float* sp,
+                                          float* sl, int jb) {
+  const Dims d = A.d;
+  const int nj = d.my - 2;
+  float xc[U + 2], xt[U + 2], xb[U + 2], gj[U + 1], ajr[U], ajb[U], bb[U], inv[U], kjb[U];
+  float2 fic[U], fkc[U], fkb[U];
+  float4 cr[U + 1];
+#pragma unroll
+  for (int u = 0; u < U + 2; u++) {
+    const unsigned c = warp_row(d, p, jb + u);
+    xc[u] = ldb(x, c);
+    xt[u] = ldb(x, c + p.okT);
+    xb[u] = ldb(x, c + p.okB);
+  }
+  {
+    const unsigned c = warp_row(d, p, jb);
+    gj[0] = p.comp ? ldb(A.ffj, c) : 0.f;
+    cr[0] = p.comp ? ldb(A.ffc, 4u * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const unsigned c = p.o + (unsigned)min(jb + 1 + u, nj) * p.sy;
+    fic[u] = ldb(A.ffi, 2u * c);
+    ajr[u] = ldb(A.faj, c);
+    gj[u + 1] = p.comp ? ldb(A.ffj, c) : 0.f;
+    fkc[u] = p.comp ? ldb(A.ffk, 2u * c) : make_float2(0.f, 0.f);
+    fkb[u] = p.comp ? ldb(A.ffk, 2u * (c + p.okB)) : make_float2(0.f, 0.f);
+    ajb[u] = p.comp ? ldb(A.faj, c + p.okB) : 0.f;
+    cr[u + 1] = ldb(A.ffc, 4u * c);
+    kjb[u] = p.comp ? ldb(reinterpret_cast<const float*>(A.ffc), 4u * (c + p.okB) + 12u) : 0.f;
+    bb[u] = p.comp ? ldb(b, c) : 0.f;
+    inv[u] = p.comp ? ldb(lf, c) : 0.f;
+  }
+  float ce[U + 2], cw[U + 2];
+#pragma unroll
+  for (int u = 0; u < U + 2; u++) {
+    ce[u] = from_e(xc[u]);
+    cw[u] = from_w(xc[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < U; u++) {
+    const int jl = jb + u;
+    if (jl >= nj) break;  // the same for the warp
+    FaceData f;
+    float v[19];
+    v[CP] = xc[u + 1];
+    v[SP] = xc[u];
+    v[NP] = xc[u + 2];
+    v[EP] = ce[u + 1];
+    v[WP] = cw[u + 1];
+    v[TP] = xt[u + 1];
+    v[BP] = xb[u + 1];
+    v[TE] = from_e(v[TP]);
+    v[TW] = from_w(v[TP]);
+    v[BE] = from_e(v[BP]);
+    v[BW] = from_w(v[BP]);
+    f.fic = fic[u];
+    f.fiw = make_float2(from_w(fic[u].x), from_w(fic[u].y));
+    f.fkc = fkc[u];
+    f.fkb = fkb[u];
+    f.gjc = gj[u + 1];
+    f.gjs = gj[u];
+    f.aj = face_aj(ajr[u]);
+    f.cc = face_code(ajr[u]);
+    f.cw = face_code(from_w(ajr[u]));
+    f.cb = face_code(ajb[u]);
+    const bool live = p.comp && f.aj != 0.f;
+    v[SE] = ce[u];
+    v[SW] = cw[u];
+    v[NE] = ce[u + 2];
+    v[NW] = cw[u + 2];
+    v[TS] = xt[u];
+    v[TN] = xt[u + 2];
+    v[BS] = xb[u];
+    v[BN] = xb[u + 2];
+    const FaceX e{cr[u + 1].x, from_w(cr[u + 1].x), cr[u + 1].y, cr[u + 1].z, cr[u].y, cr[u].z, cr[u + 1].w, kjb[u]};
+    float s, n;
+    const float ax = face_row_all(f, e, v, s, n);
+    put_line(su, sp, sl, jl, nj, live, bb[u] - ax, inv[u], s * f.aj, n * f.aj);
+  }
+}
+
+// A tile of the sweep: residuals by all warps, column solves by the first, the
+// write by all.
+template <int U>
+__device__ __forceinline__ void smooth_tile_wg(const OpView<float>& A, const float* __restrict__ lf,
+                                              const float* __restrict__ xi, const float* __restrict__ b,
+                                              float* __restrict__ xo, float omega, int bx, int by, float* su) {
+  constexpr int NW = VFS_SMOOTH_NT / 32;
+  const int nj = A.d.my - 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float *sp = su + 32 * nj, *sl = sp + 32 * nj;
+  const WarpTile p = warp_tile(A.d, bx, by);
+  for (int jb = warp * U; jb < nj; jb += NW * U) warp_rows<U>(A, p, lf, xi, b, su, sp, sl, jb);
+  __syncthreads();
+  if (warp == 0) line_solve<float>(su, sp, sl, nj, 32, lane);
+  __syncthreads();
+  if (!p.comp) return;
+  char* out = reinterpret_cast<char*>(xo);
+#pragma unroll 8
+  for (int jl = warp; jl < nj; jl += NW) {
+    const unsigned c = p.o + (unsigned)(1 + jl) * p.sy;
+    *reinterpret_cast<float*>(out + c) = fmaf(omega, su[jl * 32 + lane], ldb(xi, c));
+  }
+}
+
 // Columns per block: the requested tile (0 = automatic), narrowed while
 // three staged line arrays exceed 48 KB or the tile is twice the width of
 // the level; automatically also narrowed (down to 8) while the sweep has
@@ -1067,7 +1268,8 @@ __device__ __forceinline__ void resrestrict_tile(const OpView<T>& A, const T* __
         } else {
           FaceX fe;
           face_gather_all(A, x, fic, fjc, fk, fd, fe, xv);
-          ax = face_row_all(fd, fe, xv);
+          T s, n;
+          ax = face_row_all(fd, fe, xv, s, n);
         }
       } else {
         TC cv[19];

@@ -110,6 +110,7 @@ struct OpView {
   // code in its two low mantissa bits (bit 0: the upper pair is the face's
   // centre pair, bit 1: the lower pair)
   const float4* ffc = nullptr;
+  int flip = 0;  // walk the k planes from the last one
 };
 
 __device__ __forceinline__ bool skipped(const int* f) { return f && *(volatile const int*)f; }

@@ -83,7 +83,7 @@ int launch_restrict(const Dims& f, const T* x, const double* nvf, const Dims& c,
 // xf += P xc (MyInterpolation) using the prolongation codes of the fine level; add == 0 overwrites
 template <typename T>
 int launch_prolong(const Dims& f, const uint8_t* code, const Dims& c, const T* xc, T* xf, int add, const int* skip,
-                   cudaStream_t s);
+                   cudaStream_t s, int flip = 0);
 // x = Binv b over the packed interior of the coarsest level (b scaled by dsc first when dsc != nullptr)
 template <typename T>
 int launch_coarse_gemv(const Dims& d, const T* Binv, int n, const T* b, T* x, const T* dsc, const int* skip,
