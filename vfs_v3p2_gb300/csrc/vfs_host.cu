@@ -1854,15 +1854,17 @@ int grid_set_nvert(vfs_ctx* ctx, Grid& g, const double* nvert) {
 }
 
 // Everything derived from the finest coordinates and nvert: coarse nodes and
-// masks (every other node; MyNvertRestriction), the metrics of every level,
-// the restriction weights and the inverse metric.  The operator is rebuilt
+// masks (every other node; MyNvertRestriction), the metrics of every level
+// (coords: the coordinates changed), the restriction weights and the inverse
+// metric.  The operator is rebuilt
 // by vfs_poisson_lhs.
-int grid_derive(vfs_ctx* ctx, Grid& g) {
+int grid_derive(vfs_ctx* ctx, Grid& g, bool coords) {
   const int L = g.L;
   for (int l = L - 2; l >= 0; l--)
     launch_coarsen(g.lev[l + 1].d, g.lev[l].d, g.si, g.sj, g.sk, g.lev[l + 1].coor, g.lev[l + 1].nvert, g.lev[l].coor,
                    g.lev[l].nvert, g.s);
-  for (int l = 0; l < L; l++) launch_form_metrics(g.lev[l].d, g.lev[l].coor, g.lev[l].M, g.mtmp, g.s);
+  if (coords)
+    for (int l = 0; l < L; l++) launch_form_metrics(g.lev[l].d, g.lev[l].coor, g.lev[l].M, g.mtmp, g.s);
   for (int l = 0; l < L; l++) launch_restrict_weights(g.lev[l].N, g.lev[l].nvert, g.lev[l].rw32, g.lev[l].rw64, g.s);
   Level& F = g.lev[L - 1];
   launch_inverse_metric(F.d, F.M, F.nvert, g.minv, g.s);
@@ -2085,7 +2087,7 @@ int vfs_grid_create(vfs_ctx* ctx, const vfs_grid_desc* desc, int* grid_id) {
   if (cudaMemcpyAsync(F.coor, desc->coor, 3 * N * sizeof(double), cudaMemcpyHostToDevice, g.s) != cudaSuccess)
     return bail(cuda_fail(ctx, cudaGetLastError(), "upload"));
   r = grid_set_nvert(ctx, g, desc->nvert);
-  if (!r) r = grid_derive(ctx, g);
+  if (!r) r = grid_derive(ctx, g, true);
   if (r) return bail(r);
   const int id = ctx->next_id++;
   ctx->grids[id] = gp;
@@ -2110,7 +2112,7 @@ int vfs_grid_update_nvert(vfs_ctx* ctx, int grid, const double* nvert) {
   if (g->busy) return fail(ctx, VFS_ERR_BUSY, "the grid has a request in flight");
   CK(cudaSetDevice(ctx->device));
   int r = grid_set_nvert(ctx, *g, nvert);
-  if (!r) r = grid_derive(ctx, *g);
+  if (!r) r = grid_derive(ctx, *g, false);
   return r;
 }
 
@@ -2122,7 +2124,7 @@ int vfs_grid_update_coords(vfs_ctx* ctx, int grid, const double* coor) {
   CK(cudaSetDevice(ctx->device));
   Level& F = g->lev[g->L - 1];
   CK(cudaMemcpyAsync(F.coor, coor, 3 * ncell(g->d) * sizeof(double), cudaMemcpyHostToDevice, g->s));
-  return grid_derive(ctx, *g);
+  return grid_derive(ctx, *g, true);
 }
 
 namespace {
@@ -2215,10 +2217,11 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   Grid& g = *gp;
   CK(cudaSetDevice(ctx->device));
   const size_t N = ncell(g.d);
-  double* gt = nullptr;
-  unsigned* dmask = nullptr;
-  CK(cudaMalloc(&gt, 9 * N * sizeof(double)));
-  CK(cudaMalloc(&dmask, 2 * sizeof(unsigned)));
+  // scratch on the grid's own stream: the g tensor in the metric formation's
+  // buffer (9 N), the slot mask, range flag and region count among the scalars
+  double* gt = g.mtmp;
+  unsigned* dmask = (unsigned*)(g.scal + 32);
+  int* dregions = (int*)(g.scal + 34);
   CK(cudaMemsetAsync(dmask + 1, 0, sizeof(unsigned), g.s));
   for (int l = 0; l < g.L; l++) {
     Level& Lv = g.lev[l];
@@ -2244,29 +2247,34 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   CK(cudaMemcpyAsync(&range, dmask + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
   CK(cudaStreamSynchronize(g.s));
   g.half_ok = range == 0;
-  cudaFree(gt);
-  cudaFree(dmask);
-  // connected fluid regions of the finest level: one null vector each
-  {
-    std::vector<double> nv(N);
-    CK(cudaMemcpy(nv.data(), F.nvert, N * sizeof(double), cudaMemcpyDeviceToHost));
-    std::vector<char> fl(N, 0);
-    bool solid = false;
-    for (int k = 1; k < F.d.mz - 1; k++)
-      for (int j = 1; j < F.d.my - 1; j++)
-        for (int i = 1; i < F.d.mx - 1; i++) {
-          const size_t c = cidx(F.d, i, j, k);
-          fl[c] = nv[c] < 0.1;
-          solid = solid || !fl[c];
+  // connected fluid regions of the finest level: one null vector each.  They
+  // are counted on the device (the g tensor's buffer is free again); only a
+  // grid that bodies cut apart needs the labels.
+  g.ncomp = 1;
+  if (g.nfluid < (double)n_interior(F.d)) {
+    launch_region_count(F.d, F.nvert, (int*)gt, dregions, g.s);
+    int regions = 0;
+    CK(cudaMemcpyAsync(&regions, dregions, sizeof(int), cudaMemcpyDeviceToHost, g.s));
+    CK(cudaStreamSynchronize(g.s));
+    if (regions != 1) {
+      std::vector<double> nv(N);
+      CK(cudaMemcpy(nv.data(), F.nvert, N * sizeof(double), cudaMemcpyDeviceToHost));
+      std::vector<char> fl(N, 0);
+      for (int k = 1; k < F.d.mz - 1; k++)
+        for (int j = 1; j < F.d.my - 1; j++)
+          for (int i = 1; i < F.d.mx - 1; i++) {
+            const size_t c = cidx(F.d, i, j, k);
+            fl[c] = nv[c] < 0.1;
+          }
+      std::vector<int> lab;
+      g.ncomp = fluid_regions(F.d, fl, lab);
+      if (g.ncomp > 1) {
+        if (!g.comp) {
+          const int r = galloc(ctx, g, &g.comp, N);
+          if (r) return r;
         }
-    std::vector<int> lab;
-    g.ncomp = solid ? fluid_regions(F.d, fl, lab) : 1;
-    if (g.ncomp > 1) {
-      if (!g.comp) {
-        const int r = galloc(ctx, g, &g.comp, N);
-        if (r) return r;
+        CK(cudaMemcpy(g.comp, lab.data(), N * sizeof(int), cudaMemcpyHostToDevice));
       }
-      CK(cudaMemcpy(g.comp, lab.data(), N * sizeof(int), cudaMemcpyHostToDevice));
     }
   }
   // coarsest level: dense inverse of A + sigma e e^T when small enough
@@ -2304,21 +2312,17 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
     }
     if (nf > 0) {
       const double sigma = -(sabs / nf) / (double)nf;
-      double *W = nullptr, *fac = nullptr, *pval = nullptr;
-      int* piv = nullptr;
-      CK(cudaMalloc(&W, (size_t)n * 2 * n * sizeof(double)));
-      CK(cudaMalloc(&fac, (size_t)n * sizeof(double)));
-      CK(cudaMalloc(&pval, sizeof(double)));
-      CK(cudaMalloc(&piv, sizeof(int)));
+      double* W = nullptr;
+      CK(cudaMalloc(&W, dense_inverse_scratch(n) * sizeof(double)));
       int r = C.Binv ? VFS_OK : galloc(ctx, g, &C.Binv, (size_t)n * n);
       if (!r && !C.Binv32) r = galloc(ctx, g, &C.Binv32, (size_t)n * n);
       if (r) {
-        cudaFree(W); cudaFree(fac); cudaFree(pval); cudaFree(piv); cudaFree(ccomp);
+        cudaFree(W); cudaFree(ccomp);
         return r;
       }
-      launch_dense_inverse(C.d, C.mcoef, sigma, W, fac, piv, pval, C.Binv, C.Binv32, n, g.s, ccomp);
+      launch_dense_inverse(C.d, C.mcoef, sigma, W, C.Binv, C.Binv32, n, g.s, ccomp);
       cudaError_t e = cudaStreamSynchronize(g.s);
-      cudaFree(W); cudaFree(fac); cudaFree(pval); cudaFree(piv); cudaFree(ccomp);
+      cudaFree(W); cudaFree(ccomp);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "coarse inverse");
       C.nco = n;
     }

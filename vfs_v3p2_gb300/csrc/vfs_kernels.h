@@ -37,8 +37,11 @@ int launch_prolong_codes(const Dims& f, const Dims& c, int si, int sj, int sk, c
                          uint8_t* code, cudaStream_t s);
 // ccomp (nullable): labels of the level's connected fluid regions, one
 // sigma e_q e_q^T term per region
-int launch_dense_inverse(const Dims& d, const double* mcoef, double sigma, double* W, double* fac, int* piv, double* pval,
-                         double* Binv, float* Binv32, int n, cudaStream_t s, const int* ccomp = nullptr);
+int launch_dense_inverse(const Dims& d, const double* mcoef, double sigma, double* W, double* Binv, float* Binv32, int n,
+                         cudaStream_t s, const int* ccomp = nullptr);
+size_t dense_inverse_scratch(int n);  // doubles of W
+// number of connected fluid regions into *count (device); parent: N ints of scratch
+int launch_region_count(const Dims& d, const double* nvert, int* parent, int* count, cudaStream_t s);
 
 // ---- stencils and multigrid (k_mg.cu) ----
 // y = A x (FP64 accumulate; x FP64 or FP32); r = b - A x when b != nullptr.
