@@ -41,93 +41,119 @@ __device__ __forceinline__ void post_status(const KrylovState* st, int* hst) {
   h[1] = st->epoch;
   __threadfence_system();
 }
-// True in every thread of the block that arrives last (each block calls it
-// once, after its partials): that block sums the partials of all blocks in a
-// fixed order, so the result does not depend on which block it is, and a
-// separate one-block launch (3 us of a captured iteration) is saved.  The
-// ticket is back at zero when the block continues.
-__device__ __forceinline__ bool last_block(unsigned* ticket) {
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    if (last) *ticket = 0u;
-  }
-  __syncthreads();
-  if (last) __threadfence();
-  return last;
-}
 __device__ __forceinline__ bool met(const KrylovState* st, double r) {
   return r <= st->rtol * st->bnorm && (st->atol <= 0. || r <= st->atol);
 }
 
-// ||v||^2 partials; then finish: is_b ? bnorm : beta (+ g[0], done check).
-__global__ void __launch_bounds__(KB) k_sq_partials(const KrylovState* st, const double* __restrict__ v, size_t n,
-                                                     double* parts, int check_done) {
-  if (check_done && is_done(st)) return;
+// The norm of a new round's vectors from their partials, by one block: MODE 0
+// (beta alone: a restart's residual), 1 (bnorm alone: a warm start, whose
+// residual follows), 2 (both: a cold start, where r0 = aj b).  Clears the
+// Hessenberg matrix and g with the whole block.
+template <int MODE>
+__device__ __forceinline__ void norm_close(KrylovState* st, const double* parts, int nparts) {
   __shared__ double sh[32];
   double s = 0.;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    double a = v[t];
-    s = fma(a, a, s);
-  }
+  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += __ldcg(parts + p);
   s = block_sum(s, sh);
-  if (threadIdx.x == 0) parts[blockIdx.x] = s;
-}
-
-__global__ void k_norm_finish(KrylovState* st, const double* __restrict__ parts, int nparts, int is_b) {
-  if (!is_b && is_done(st)) return;
-  __shared__ double sh[32];
-  double s = 0.;
-  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += parts[p];
-  s = block_sum(s, sh);
-  if (!is_b) {  // clear the Hessenberg matrix and g with the whole block
+  if (MODE != 1) {
     const int m = st->m;
     for (int q = threadIdx.x; q <= m; q += blockDim.x) st->g[q] = 0.;
     for (int q = threadIdx.x; q < (m + 1) * m; q += blockDim.x) st->H[q] = 0.;
     __syncthreads();
   }
-  if (threadIdx.x == 0) {
-    double nrm = sqrt(s);
-    if (is_b) {
-      st->bnorm = nrm;
-      st->done = (nrm == 0.) ? 1 : 0;
-      st->it = 0;
-      st->j = 0;
-    } else {
-      st->beta = nrm;
-      st->resid = nrm;
-      st->g[0] = nrm;
-      st->j = 0;
-      st->inv_hn = nrm > 0. ? 1. / nrm : 0.;
-      st->vs[0] = 1.;  // V_0 is stored normalised
-      if (met(st, nrm)) st->done = 1;
+  if (threadIdx.x != 0) return;
+  const double nrm = sqrt(s);
+  if (MODE != 0) {
+    st->bnorm = nrm;
+    st->done = (nrm == 0.) ? 1 : 0;
+    st->it = 0;
+    st->j = 0;
+    if (nrm == 0. || MODE == 1) return;
+  }
+  st->beta = nrm;
+  st->resid = nrm;
+  st->g[0] = nrm;
+  st->j = 0;
+  st->inv_hn = nrm > 0. ? 1. / nrm : 0.;
+  st->vs[0] = 1.;  // V_0 is stored normalised
+  if (met(st, nrm)) st->done = 1;
+}
+
+// beta = ||r|| of a restart (or warm start): partials and, by the last block, the close.
+__global__ void __launch_bounds__(KB) k_beta(KrylovState* st, const double* __restrict__ v, size_t n, double* parts) {
+  if (is_done(st)) return;
+  __shared__ double sh[32];
+  double s = 0.;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    const double a = v[t];
+    s = fma(a, a, s);
+  }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) parts[blockIdx.x] = s;
+  if (last_block(st->ticket)) norm_close<0>(st, parts, gridDim.x);
+}
+int launch_beta(KrylovState* st, const double* r, size_t n, double* parts, cudaStream_t s) {
+  k_beta<<<krylov_nblocks(n), KB, 0, s>>>(st, r, n, parts); ++g_launches;
+  return (int)cudaGetLastError();
+}
+
+// Opening of a round: the aj-scaled right-hand side bs = aj b on the interior
+// (bs's ghosts are zero), its norm, and on a cold start the residual r0 = bs
+// as V_0 (scaled by launch_open_v) and its norm: one pass and one launch.
+template <bool COLD>
+__global__ void __launch_bounds__(KB) k_open_b(KrylovState* st, Dims d, const double* __restrict__ aj,
+                                               const double* __restrict__ b, double* __restrict__ bs,
+                                               double* __restrict__ V, double* parts) {
+  __shared__ double sh[32];
+  const int lane = threadIdx.x & 31, nw = gridDim.x * (KB / 32);
+  double s = 0.;
+  for (int r = blockIdx.x * (KB / 32) + (threadIdx.x >> 5); r < d.my * d.mz; r += nw) {
+    const int k = r / d.my, j = r - k * d.my;
+    const bool in = j > 0 && k > 0 && j < d.my - 1 && k < d.mz - 1;
+    const size_t o = (size_t)r * d.mx;
+    for (int i = lane; i < d.mx; i += 32) {
+      double v = 0.;
+      if (in && i > 0 && i < d.mx - 1) {
+        v = aj[o + i] * b[o + i];
+        bs[o + i] = v;
+        s = fma(v, v, s);
+      }
+      if (COLD) V[o + i] = v;
     }
   }
+  s = block_sum(s, sh);
+  if (threadIdx.x == 0) parts[blockIdx.x] = s;
+  if (last_block(st->ticket)) norm_close<COLD ? 2 : 1>(st, parts, gridDim.x);
 }
-
-int launch_norm_init(KrylovState* st, const double* r, size_t n, double* parts, int is_b, cudaStream_t s) {
-  const int nb = krylov_nblocks(n);
-  k_sq_partials<<<nb, KB, 0, s>>>(st, r, n, parts, !is_b); ++g_launches;
-  k_norm_finish<<<1, KB, 0, s>>>(st, parts, nb, is_b); ++g_launches;
+int launch_open_b(KrylovState* st, const Dims& d, const double* aj, const double* b, double* bs, double* V, bool cold,
+                  double* parts, cudaStream_t s) {
+  const int nb = krylov_nblocks(ncell(d));
+  if (cold) k_open_b<true><<<nb, KB, 0, s>>>(st, d, aj, b, bs, V, parts);
+  else k_open_b<false><<<nb, KB, 0, s>>>(st, d, aj, b, bs, V, parts);
+  ++g_launches;
   return (int)cudaGetLastError();
 }
 
-// v0 = r * (1 / beta)
-__global__ void k_scale_vec(const KrylovState* st, const double* __restrict__ r, double* __restrict__ v, size_t n) {
+// v0 = r / beta in place and the first preconditioner input T(v0) (times 1 / D
+// of the FP16 normalised operator when dinv is set); r's ghosts are zero.
+template <typename T>
+__global__ void __launch_bounds__(KB) k_open_v(const KrylovState* st, double* v, T* __restrict__ out, size_t n,
+                                               const float* __restrict__ dinv) {
   if (is_done(st)) return;
   const double f = st->inv_hn;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) v[t] = r[t] * f;
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
+    const double a = v[t] * f;
+    v[t] = a;
+    out[t] = dinv ? (T)a * (T)dinv[t] : (T)a;
+  }
 }
-int launch_vec_scale_first(KrylovState* st, const double* r, double* v0, size_t n, cudaStream_t s) {
-  k_scale_vec<<<krylov_nblocks(n) * 4, KB, 0, s>>>(st, r, v0, n); ++g_launches;
+template <typename T>
+int launch_open_v(const KrylovState* st, double* v, T* out, size_t n, const float* dinv, cudaStream_t s) {
+  k_open_v<T><<<krylov_nblocks(n) * 4, KB, 0, s>>>(st, v, out, n, dinv); ++g_launches;
   return (int)cudaGetLastError();
 }
-int launch_vnext(KrylovState* st, const double* w, double* vn, size_t n, cudaStream_t s) {
-  k_scale_vec<<<krylov_nblocks(n) * 4, KB, 0, s>>>(st, w, vn, n); ++g_launches;
-  return (int)cudaGetLastError();
-}
+template int launch_open_v<float>(const KrylovState*, double*, float*, size_t, const float*, cudaStream_t);
+template int launch_open_v<double>(const KrylovState*, double*, double*, size_t, const float*, cudaStream_t);
 
 // Multi-dot partials: parts[q * nblocks + b] = sum over block b's cells of
 // V_q . w for q < nv, up to DCH columns per sweep (w is re-read from L2).
@@ -474,9 +500,10 @@ int launch_lsq_update(KrylovState* st, cudaStream_t s) {
   return (int)cudaGetLastError();
 }
 
-// x += sum_q y_q Z_q over the closed columns.
+// x += sum_q y_q Z_q over the closed columns; the last block marks them as
+// applied (a later update adds nothing).
 template <typename T>
-__global__ void __launch_bounds__(KB) k_x_update(const KrylovState* st, const T* __restrict__ Z, size_t n, double* x) {
+__global__ void __launch_bounds__(KB) k_x_update(KrylovState* st, const T* __restrict__ Z, size_t n, double* x) {
   __shared__ double ys[72];
   const int J = st->j;
   for (int q = threadIdx.x; q < J; q += blockDim.x) ys[q] = st->y[q] * st->vs[q];
@@ -486,6 +513,7 @@ __global__ void __launch_bounds__(KB) k_x_update(const KrylovState* st, const T*
     for (int q = 0; q < J; q++) a = fma(ys[q], to_acc<double>(Z[(size_t)q * n + t]), a);
     x[t] = a;
   }
+  if (last_block(st->ticket) && threadIdx.x == 0) st->j = 0;
 }
 template <typename T>
 int launch_x_update(KrylovState* st, const T* Z, size_t n, double* x, cudaStream_t s) {
@@ -494,30 +522,6 @@ int launch_x_update(KrylovState* st, const T* Z, size_t n, double* x, cudaStream
 }
 template int launch_x_update<float>(KrylovState*, const float*, size_t, double*, cudaStream_t);
 template int launch_x_update<double>(KrylovState*, const double*, size_t, double*, cudaStream_t);
-
-// Mark the closed columns as applied (a later x update adds nothing).
-__global__ void k_restart_reset(KrylovState* st) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) st->j = 0;
-}
-int launch_restart_reset(KrylovState* st, cudaStream_t s) {
-  k_restart_reset<<<1, 32, 0, s>>>(st); ++g_launches;
-  return (int)cudaGetLastError();
-}
-
-// out = ||v||_2 (no Krylov state involved).
-__global__ void k_sqrt_sum(const double* __restrict__ parts, int nparts, double* out) {
-  __shared__ double sh[32];
-  double s = 0.;
-  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += parts[p];
-  s = block_sum(s, sh);
-  if (threadIdx.x == 0) *out = sqrt(s);
-}
-int launch_norm2(const double* v, size_t n, double* parts, double* out, cudaStream_t s) {
-  const int nb = krylov_nblocks(n);
-  k_sq_partials<<<nb, KB, 0, s>>>(nullptr, v, n, parts, 0); ++g_launches;
-  k_sqrt_sum<<<1, KB, 0, s>>>(parts, nb, out); ++g_launches;
-  return (int)cudaGetLastError();
-}
 
 // Next basis vector and multigrid input in one sweep: V_{j+1} = w / h_{j+1,j}
 // and out = T(V_{j+1}) over the interior; ghost entries of w are zero.

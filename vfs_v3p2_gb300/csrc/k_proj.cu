@@ -38,23 +38,47 @@ static inline int nblk(size_t n, int bs = 256) {
   return (int)(b ? b : 1);
 }
 
-// Sum per-block partials [nparts][q] in index order (one block).
-__global__ void k_finish_sums(const double* __restrict__ parts, int nparts, int nq, double* out) {
-  __shared__ double sh[32];
-  for (int q = 0; q < nq; q++) {
+// Rows (j, k) of the grid, a warp each: base cell o of the row, in: the row is
+// interior in j and k.  One division a row instead of two a cell, and a warp
+// reads consecutive cells.
+#define ROW_LOOP(d)                                                                                       \
+  const int _lane = threadIdx.x & 31, _rows = (d).my * (d).mz, _nw = gridDim.x * (RB / 32);             \
+  for (int _r = blockIdx.x * (RB / 32) + (threadIdx.x >> 5); _r < _rows; _r += _nw)
+#define ROW_DECOMP(d, j, k, o, in)                                                \
+  const int k = _r / (d).my, j = _r - k * (d).my;                               \
+  const size_t o = (size_t)_r * (d).mx;                                         \
+  const bool in = j > 0 && k > 0 && j < (d).my - 1 && k < (d).mz - 1
+
+static inline int row_blocks(const Dims& d) {
+  const int b = ((size_t)d.my * d.mz + RB / 32 - 1) / (RB / 32);
+  return b < 152 * 8 ? b : 152 * 8;
+}
+
+// Sums of NQ per-block partials (parts[q * nblocks + b]) in a fixed order, by
+// the last block: out[q].
+template <int NQ>
+__device__ __forceinline__ void finish_sums(const double* parts, double* out, double* sh) {
+  const int nb = gridDim.x;
+  for (int q = 0; q < NQ; q++) {
     double s = 0.;
-    for (int p = threadIdx.x; p < nparts; p += blockDim.x) s += parts[(size_t)p * nq + q];
+    for (int p = threadIdx.x; p < nb; p += blockDim.x) s += __ldcg(parts + (size_t)q * nb + p);
     s = block_sum(s, sh);
     if (threadIdx.x == 0) out[q] = s;
     __syncthreads();
   }
 }
-__global__ void k_finish_max(const double* __restrict__ parts, int nparts, double* out) {
-  __shared__ double sh[32];
-  double s = 0.;
-  for (int p = threadIdx.x; p < nparts; p += blockDim.x) s = fmax(s, parts[p]);
-  s = block_max(s, sh);
-  if (threadIdx.x == 0) *out = s;
+// Block maximum of integers that order like the values (max_abs), and the
+// maximum of all blocks' by the last one.
+__device__ __forceinline__ unsigned long long block_maxbits(unsigned long long v, double* sh) {
+  return (unsigned long long)block_max((long long)v, (long long*)sh);
+}
+__device__ __forceinline__ double finish_max(const double* parts, double* sh) {
+  unsigned long long m = 0ull;
+  for (int p = threadIdx.x; p < (int)gridDim.x; p += blockDim.x) {
+    const unsigned long long v = (unsigned long long)__double_as_longlong(__ldcg(parts + p));
+    m = v > m ? v : m;
+  }
+  return __longlong_as_double((long long)block_maxbits(m, sh));
 }
 
 // ---- AoS (reference Cmpnts) <-> SoA device layout ----
@@ -87,57 +111,64 @@ int launch_soa2aos(size_t n, const double* x, const double* y, const double* z, 
 // on fluid cells, periodic wrap of the minus faces; partial sums of b and of
 // the fluid count for the compatibility fix of PoissonRHS2 (poisson.c:1879-1903).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(RB) k_rhs(Dims d, Ucont u, const double* __restrict__ nvert, double dt, double st,
-                                            double coeff, double* b, double* parts) {
+__global__ void __launch_bounds__(RB) k_rhs(Dims d, Ucont u, const double* __restrict__ nvert,
+                                            const uint8_t* __restrict__ nb8, double scale, double* b, double* parts,
+                                            double* sc, unsigned* ticket) {
   __shared__ double sh[32];
   __shared__ unsigned shc[32];
   double lsum = 0.;
   unsigned lcnt = 0;  // fluid cells, counted on the integer pipe (exact)
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    double val = 0.;
-    if (interior(d, i, j, k) && !(nvert[_t] >= 0.1)) {
-      val -= u.x[_t];
-      if (i == 1 && d.ip) val += u.x[cidx(d, d.mx - 2, j, k)];
-      else val += u.x[cidx(d, i - 1, j, k)];
-      val -= u.y[_t];
-      if (j == 1 && d.jp) val += u.y[cidx(d, i, d.my - 2, k)];
-      else val += u.y[cidx(d, i, j - 1, k)];
-      val -= u.z[_t];
-      if (k == 1 && d.kp) val += u.z[cidx(d, i, j, d.mz - 2)];
-      else val += u.z[cidx(d, i, j, k - 1)];
-      val *= -1.0 / dt * st * coeff;
-      lsum += val;
-      lcnt += 1;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    const long long os = (j == 1 && d.jp) ? (long long)(d.my - 3) * d.mx : -(long long)d.mx;
+    const long long ob = (k == 1 && d.kp) ? (long long)(d.mz - 3) * d.my * d.mx : -(long long)d.my * d.mx;
+    for (int i = _lane; i < d.mx; i += 32) {
+      const size_t c = o + i;
+      double val = 0.;
+      if (in && i > 0 && i < d.mx - 1 && (nb8 ? nb8[c] == 0 : !at_least(nvert[c], 0.1))) {
+        // (0 - u_x) + u_x(i-1) is exactly the first difference
+        val = u.x[(i == 1 && d.ip) ? o + d.mx - 2 : c - 1] - u.x[c];
+        val -= u.y[c];
+        val += u.y[c + os];
+        val -= u.z[c];
+        val += u.z[c + ob];
+        val *= scale;
+        lsum += val;
+        lcnt += 1;
+      }
+      b[c] = val;
     }
-    b[_t] = val;
   }
   lsum = block_sum(lsum, sh);
   lcnt = block_sum(lcnt, shc);
   if (threadIdx.x == 0) {
-    parts[2 * blockIdx.x] = lsum;
-    parts[2 * blockIdx.x + 1] = (double)lcnt;
+    parts[blockIdx.x] = lsum;
+    parts[gridDim.x + blockIdx.x] = (double)lcnt;
   }
+  if (last_block(ticket)) finish_sums<2>(parts, sc, sh);
 }
 // b += -sum / count on fluid interior cells (sc = {sum, count}).
-__global__ void k_meanfix(Dims d, const double* __restrict__ nvert, const double* __restrict__ sc, double* b) {
+__global__ void __launch_bounds__(RB) k_meanfix(Dims d, const double* __restrict__ nvert, const double* __restrict__ sc,
+                                                double* b) {
   const double v = (sc[1] > 0.) ? -sc[0] / sc[1] : 0.;
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (interior(d, i, j, k) && nvert[_t] < 0.1) b[_t] += v;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32)
+      if (below(nvert[o + i], 0.1)) b[o + i] += v;
   }
 }
 int launch_rhs(const Dims& d, const Ucont& u, const double* nvert, double dt, double st, double coeff, int meanfix,
-               double* b, double* parts, double* sc, cudaStream_t s, const int* comp, int ncomp) {
-  const int nb = nblk(ncell(d), RB);
-  k_rhs<<<nb, RB, 0, s>>>(d, u, nvert, dt, st, coeff, b, parts); ++g_launches;
-  k_finish_sums<<<1, 256, 0, s>>>(parts, nb, 2, sc); ++g_launches;
+               double* b, double* parts, double* sc, unsigned* ticket, cudaStream_t s, const uint8_t* nb8, const int* comp,
+               int ncomp) {
+  const int nb = row_blocks(d);
+  k_rhs<<<nb, RB, 0, s>>>(d, u, nvert, nb8, -1.0 / dt * st * coeff, b, parts, sc, ticket); ++g_launches;
   if (meanfix && comp && ncomp > 1) {
     // one compatibility fix per connected fluid region (sums in sc[2..3])
-    return launch_remove_mean(d, nvert, b, parts, sc + 2, s, comp, ncomp);
+    return launch_remove_mean(d, nvert, b, parts, sc + 2, ticket, s, comp, ncomp);
   }
   if (meanfix) {
-    k_meanfix<<<nblk(ncell(d)), 256, 0, s>>>(d, nvert, sc, b);
+    k_meanfix<<<nb, RB, 0, s>>>(d, nvert, sc, b);
     ++g_launches;
   }
   return (int)cudaGetLastError();
@@ -158,87 +189,100 @@ __device__ __forceinline__ double nrm3(const double* v, size_t c) {
 // nb8 (nvert as bytes, every value an integer in [0, 127]) turns the FP64
 // interface tests into exact integer ones: nv < 0.1 <=> 0, nv > 0.1 <=> >= 1,
 // 0.1 < nv < 1.1 <=> 1.
+// Interface faces are few: a cell whose byte equals its three + neighbours'
+// has none, and a warp without any skips the FP64 reductions.
 __global__ void __launch_bounds__(RB) k_vflux(Dims d, int mode, int phase, Ucont u, const double* __restrict__ nv,
                                               const double* __restrict__ csi, const double* __restrict__ eta,
                                               const double* __restrict__ zet, const double* __restrict__ fa, double* parts,
-                                              const uint8_t* __restrict__ nb8) {
+                                              double* out, unsigned* ticket, const uint8_t* __restrict__ nb8) {
   __shared__ double sh[32];
   const double eps = 1.e-10, ibmval = 1.1;
   double flux = 0., area = 0.;
   double corr = 0.;
+  bool any = false;
   if (phase == 1) corr = (fa[1] > 1.e-15) ? fa[0] / fa[1] : 0.;
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (!interior(d, i, j, k)) continue;
-    const size_t c = _t;
-    const size_t ce = cidx(d, i + 1, j, k), cn = cidx(d, i, j + 1, k), ct = cidx(d, i, j, k + 1);
-    double* uf[3] = {u.x, u.y, u.z};
-    const double* mt[3] = {csi, eta, zet};
-    const size_t nb[3] = {ce, cn, ct};
-    const bool lim1[3] = {i < d.mx - 2, j < d.my - 2, k < d.mz - 2};
-    const bool lim0[3] = {i <= d.mx - 2, j <= d.my - 2, k <= d.mz - 2};
-    for (int f = 0; f < 3; f++) {
-      double* uu = uf[f];
-      if (mode == 1) {
+  double* uf[3] = {u.x, u.y, u.z};
+  const double* mt[3] = {csi, eta, zet};
+  const int off[3] = {1, d.mx, d.mx * d.my};
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32) {
+      const size_t c = o + i;
+      if (nb8) {
+        const int a = nb8[c];
+        if (a == nb8[c + off[0]] && a == nb8[c + off[1]] && a == nb8[c + off[2]]) continue;
+      }
+      const bool lim1[3] = {i < d.mx - 2, j < d.my - 2, k < d.mz - 2};
+#pragma unroll
+      for (int f = 0; f < 3; f++) {
+        double* uu = uf[f];
+        const size_t cf = c + off[f];
         bool plus, minus;
-        if (nb8) {
-          const int a = nb8[c], b = nb8[nb[f]];
-          plus = a == 0 && b == 1 && lim1[f];
-          minus = a == 1 && b == 0 && lim1[f];
-        } else {
-          plus = nv[c] < 0.1 && nv[nb[f]] > 0.1 && nv[nb[f]] < ibmval && lim1[f];
-          minus = nv[c] > 0.1 && nv[c] < ibmval && nv[nb[f]] < 0.1 && lim1[f];
-        }
-        if (!(plus || minus)) continue;
-        if (phase == 0) {
-          if (fabs(uu[c]) > eps) {
-            flux += plus ? uu[c] : -uu[c];
-            area += nrm3(mt[f], c);
-          } else uu[c] = 0.;
-        } else {
-          // phase 1: correct, and measure the corrected face at once (the
-          // same values and order as a separate measuring pass)
-          const double nr = nrm3(mt[f], c);
-          if (fabs(uu[c]) > eps) {
-            if (plus) uu[c] -= nr * corr;
-            else uu[c] += nr * corr;
+        if (mode == 1) {
+          if (nb8) {
+            const int a = nb8[c], b = nb8[cf];
+            plus = a == 0 && b == 1 && lim1[f];
+            minus = a == 1 && b == 0 && lim1[f];
+          } else {
+            plus = nv[c] < 0.1 && nv[cf] > 0.1 && nv[cf] < ibmval && lim1[f];
+            minus = nv[c] > 0.1 && nv[c] < ibmval && nv[cf] < 0.1 && lim1[f];
           }
-          flux += plus ? uu[c] : -uu[c];
-          area += nr;
-        }
-      } else {
-        bool plus, minus;
-        if (nb8) {
-          const int a = nb8[c], b = nb8[nb[f]];
-          plus = a == 0 && b != 0 && lim0[f];
-          minus = a != 0 && b == 0 && lim0[f];
+          if (!(plus || minus)) continue;
+          any = true;
+          if (phase == 0) {
+            if (fabs(uu[c]) > eps) {
+              flux += plus ? uu[c] : -uu[c];
+              area += nrm3(mt[f], c);
+            } else uu[c] = 0.;
+          } else {
+            // phase 1: correct, and measure the corrected face at once (the
+            // same values and order as a separate measuring pass)
+            const double nr = nrm3(mt[f], c);
+            if (fabs(uu[c]) > eps) {
+              if (plus) uu[c] -= nr * corr;
+              else uu[c] += nr * corr;
+            }
+            flux += plus ? uu[c] : -uu[c];
+            area += nr;
+          }
         } else {
-          plus = nv[c] < VFS_THR && nv[nb[f]] > VFS_THR && lim0[f];
-          minus = nv[c] > VFS_THR && nv[nb[f]] < VFS_THR && lim0[f];
+          if (nb8) {
+            const int a = nb8[c], b = nb8[cf];
+            plus = a == 0 && b != 0;
+            minus = a != 0 && b == 0;
+          } else {
+            plus = nv[c] < VFS_THR && nv[cf] > VFS_THR;
+            minus = nv[c] > VFS_THR && nv[cf] < VFS_THR;
+          }
+          if (!(plus || minus)) continue;
+          any = true;
+          if (phase == 1) uu[c] = 0.;  // and measured as such
+          flux += plus ? uu[c] : -uu[c];
+          area += nrm3(mt[f], c);
         }
-        if (!(plus || minus)) continue;
-        if (phase == 1) uu[c] = 0.;  // and measured as such
-        flux += plus ? uu[c] : -uu[c];
-        area += nrm3(mt[f], c);
       }
     }
   }
-  flux = block_sum(flux, sh);
-  area = block_sum(area, sh);
-  if (threadIdx.x == 0) {
-    parts[2 * blockIdx.x] = flux;
-    parts[2 * blockIdx.x + 1] = area;
+  if (__syncthreads_or(any)) {
+    flux = block_sum(flux, sh);
+    area = block_sum(area, sh);
   }
+  if (threadIdx.x == 0) {
+    parts[blockIdx.x] = flux;
+    parts[gridDim.x + blockIdx.x] = area;
+  }
+  if (last_block(ticket)) finish_sums<2>(parts, out, sh);
 }
 int launch_volume_flux(const Dims& d, int mode, const Ucont& u, const double* nvert, const double* M, double* parts,
-                       double* fa4, cudaStream_t s, const uint8_t* nb8) {
+                       double* fa4, unsigned* ticket, cudaStream_t s, const uint8_t* nb8) {
   const size_t N = ncell(d);
-  const int nb = nblk(N, RB);
+  const int nb = row_blocks(d);
   const double *csi = M + N * MP_CSI, *eta = M + N * MP_ETA, *zet = M + N * MP_ZET;
-  k_vflux<<<nb, RB, 0, s>>>(d, mode, 0, u, nvert, csi, eta, zet, fa4, parts, nb8); ++g_launches;
-  k_finish_sums<<<1, 256, 0, s>>>(parts, nb, 2, fa4); ++g_launches;
-  k_vflux<<<nb, RB, 0, s>>>(d, mode, 1, u, nvert, csi, eta, zet, fa4, parts, nb8); ++g_launches;
-  k_finish_sums<<<1, 256, 0, s>>>(parts, nb, 2, fa4 + 2); ++g_launches;
+  for (int phase = 0; phase < 2; phase++) {
+    k_vflux<<<nb, RB, 0, s>>>(d, mode, phase, u, nvert, csi, eta, zet, fa4, parts, fa4 + 2 * phase, ticket, nb8);
+    ++g_launches;
+  }
   return (int)cudaGetLastError();
 }
 
@@ -250,77 +294,120 @@ int launch_volume_flux(const Dims& d, int mode, const Ucont& u, const double* nv
 // (poisson.c:819-873, regions from FullyBlocked, poisson.c:1918-1998).
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(RB) k_fluid_sum(Dims d, const double* __restrict__ nvert, const double* __restrict__ x,
-                                                  double* parts, const int* __restrict__ comp, int q) {
+                                                  double* parts, double* sc, unsigned* ticket,
+                                                  const int* __restrict__ comp, int q) {
   __shared__ double sh[32];
   __shared__ unsigned shc[32];
   double s = 0.;
   unsigned n = 0;  // counted on the integer pipe (exact)
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (interior(d, i, j, k) && nvert[_t] < 0.1 && (!comp || comp[_t] == q)) {
-      s += x[_t];
-      n += 1;
-    }
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32)
+      if (below(nvert[o + i], 0.1) && (!comp || comp[o + i] == q)) {
+        s += x[o + i];
+        n += 1;
+      }
   }
   s = block_sum(s, sh);
   n = block_sum(n, shc);
   if (threadIdx.x == 0) {
-    parts[2 * blockIdx.x] = s;
-    parts[2 * blockIdx.x + 1] = (double)n;
+    parts[blockIdx.x] = s;
+    parts[gridDim.x + blockIdx.x] = (double)n;
   }
+  if (last_block(ticket)) finish_sums<2>(parts, sc, sh);
 }
-__global__ void k_sub_mean(Dims d, const double* __restrict__ nvert, const double* __restrict__ sc, double* x,
-                           const int* __restrict__ comp, int q) {
+int launch_fluid_sum(const Dims& d, const double* nvert, const double* x, double* parts, double* sc, unsigned* ticket,
+                     cudaStream_t s) {
+  k_fluid_sum<<<row_blocks(d), RB, 0, s>>>(d, nvert, x, parts, sc, ticket, nullptr, 0); ++g_launches;
+  return (int)cudaGetLastError();
+}
+__global__ void __launch_bounds__(RB) k_sub_mean(Dims d, const double* __restrict__ nvert, const double* __restrict__ sc,
+                                                 double* x, const int* __restrict__ comp, int q) {
   const double v = (sc[1] > 0.) ? -sc[0] / sc[1] : 0.;
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (interior(d, i, j, k) && nvert[_t] < 0.1 && (!comp || comp[_t] == q)) x[_t] += v;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32)
+      if (below(nvert[o + i], 0.1) && comp[o + i] == q) x[o + i] += v;
   }
 }
-int launch_remove_mean(const Dims& d, const double* nvert, double* x, double* parts, double* sc, cudaStream_t s,
-                       const int* comp, int ncomp) {
-  const int nb = nblk(ncell(d), RB);
-  const int nq = (comp && ncomp > 1) ? ncomp : 1;
-  const int* cm = nq > 1 ? comp : nullptr;
-  for (int q = 0; q < nq; q++) {
-    k_fluid_sum<<<nb, RB, 0, s>>>(d, nvert, x, parts, cm, q); ++g_launches;
-    k_finish_sums<<<1, 256, 0, s>>>(parts, nb, 2, sc); ++g_launches;
-    k_sub_mean<<<nblk(ncell(d)), 256, 0, s>>>(d, nvert, sc, x, cm, q); ++g_launches;
+int launch_remove_mean(const Dims& d, const double* nvert, double* x, double* parts, double* sc, unsigned* ticket,
+                       cudaStream_t s, const int* comp, int ncomp) {
+  const int nb = row_blocks(d);
+  for (int q = 0; q < ncomp; q++) {
+    k_fluid_sum<<<nb, RB, 0, s>>>(d, nvert, x, parts, sc, ticket, comp, q); ++g_launches;
+    k_sub_mean<<<nb, RB, 0, s>>>(d, nvert, sc, x, comp, q); ++g_launches;
   }
   return (int)cudaGetLastError();
 }
 
-// Convert_Phi2_Phi (poisson.c:97-185): zero on boundary and non-fluid cells.
-__global__ void k_phi_zero(Dims d, const double* __restrict__ nvert, double* phi) {
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (!interior(d, i, j, k) || (int)nvert[_t] > VFS_THR) phi[_t] = 0.;
+// v into interior cell (i, j, k) and into the ghost cells that mirror it
+// through periodic axes (poisson.c:146-181, 2580-2616).  The thread of the
+// source writes them, so a fill needs no launch after its update.
+__device__ __forceinline__ void put_mirrored(const Dims& d, double* a, int i, int j, int k, double v) {
+  a[cidx(d, i, j, k)] = v;
+  const int gi = d.ip ? (i == 1 ? d.mx - 1 : i == d.mx - 2 ? 0 : -1) : -1;
+  const int gj = d.jp ? (j == 1 ? d.my - 1 : j == d.my - 2 ? 0 : -1) : -1;
+  const int gk = d.kp ? (k == 1 ? d.mz - 1 : k == d.mz - 2 ? 0 : -1) : -1;
+  if (gi < 0 && gj < 0 && gk < 0) return;
+  for (int q = 1; q < 8; q++) {
+    const int x = q & 1 ? gi : i, y = q & 2 ? gj : j, z = q & 4 ? gk : k;
+    if (x >= 0 && y >= 0 && z >= 0) a[cidx(d, x, y, z)] = v;
   }
 }
-// Periodic ghost fill of a scalar (poisson.c:146-181, 2580-2616).
-__global__ void k_scalar_ghosts(Dims d, double* a) {
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    int ai = wrapi(i, d.mx, d.ip), bj = wrapi(j, d.my, d.jp), ck = wrapi(k, d.mz, d.kp);
-    if (ai != i || bj != j || ck != k) a[_t] = a[cidx(d, ai, bj, ck)];
+// A ghost cell that mirrors an interior one (its value comes from there).
+__device__ __forceinline__ bool mirrors(const Dims& d, int i, int j, int k) {
+  return interior(d, wrapi(i, d.mx, d.ip), wrapi(j, d.my, d.jp), wrapi(k, d.mz, d.kp));
+}
+
+// Remove_Nullspace's mean (sc = {sum, count}, nullable), Convert_Phi2_Phi
+// (poisson.c:97-185: zero on boundary and non-fluid cells) and the periodic
+// ghosts in one pass.
+__global__ void __launch_bounds__(RB) k_phi_finish(Dims d, const double* __restrict__ nvert, const double* __restrict__ sc,
+                                                   double* phi) {
+  const double v = (sc && sc[1] > 0.) ? -sc[0] / sc[1] : 0.;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    for (int i = _lane; i < d.mx; i += 32) {
+      if (in && i > 0 && i < d.mx - 1) {
+        const double nv = nvert[o + i];
+        double x = phi[o + i];
+        if (below(nv, 0.1)) x += v;
+        if (at_least(nv, 1.0)) x = 0.;  // (int)nv > 0.1
+        put_mirrored(d, phi, i, j, k, x);
+      } else if (!mirrors(d, i, j, k)) {
+        phi[o + i] = 0.;
+      }
+    }
   }
 }
-int launch_phi_finish(const Dims& d, const double* nvert, double* phi, cudaStream_t s) {
-  k_phi_zero<<<nblk(ncell(d)), 256, 0, s>>>(d, nvert, phi); ++g_launches;
-  k_scalar_ghosts<<<nblk(ncell(d)), 256, 0, s>>>(d, phi); ++g_launches;
+int launch_phi_finish(const Dims& d, const double* nvert, double* phi, const double* sc, cudaStream_t s) {
+  k_phi_finish<<<row_blocks(d), RB, 0, s>>>(d, nvert, sc, phi); ++g_launches;
   return (int)cudaGetLastError();
 }
 
-// UpdatePressure (poisson.c:2522-2548, non-PRIMITIVE branch, + ghost fill).
-__global__ void k_update_p(Dims d, const double* __restrict__ nvert, const double* __restrict__ phi, double* p) {
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (interior(d, i, j, k) && nvert[_t] < 0.1) p[_t] += phi[_t];
+// UpdatePressure (poisson.c:2522-2548, non-PRIMITIVE branch, + ghost fill): a
+// ghost whose mirror is a boundary cell of another axis copies that cell,
+// which the update leaves alone.
+__global__ void __launch_bounds__(RB) k_update_p(Dims d, const double* __restrict__ nvert, const double* __restrict__ phi,
+                                                 double* p) {
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    for (int i = _lane; i < d.mx; i += 32) {
+      if (in && i > 0 && i < d.mx - 1) {
+        double x = p[o + i];
+        if (below(nvert[o + i], 0.1)) x += phi[o + i];
+        put_mirrored(d, p, i, j, k, x);
+      } else if (!mirrors(d, i, j, k)) {
+        const size_t src = cidx(d, wrapi(i, d.mx, d.ip), wrapi(j, d.my, d.jp), wrapi(k, d.mz, d.kp));
+        if (src != o + i) p[o + i] = p[src];
+      }
+    }
   }
 }
 int launch_update_pressure(const Dims& d, const double* nvert, const double* phi, double* p, cudaStream_t s) {
-  k_update_p<<<nblk(ncell(d)), 256, 0, s>>>(d, nvert, phi, p); ++g_launches;
-  k_scalar_ghosts<<<nblk(ncell(d)), 256, 0, s>>>(d, p); ++g_launches;
+  k_update_p<<<row_blocks(d), RB, 0, s>>>(d, nvert, phi, p); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -632,18 +719,37 @@ int launch_projection_fast(const Dims& d, const double* pw, const uint16_t* pc, 
 }
 
 // periodic ghost sync of the flagged component (poisson.c:2398-2437) on
-// cells [c0, c1).  Every source is interior in all periodic directions, so
-// the sync never reads a cell it writes; the source of a cell on an interior
-// plane k lies on plane k.
-__global__ void k_ucont_ghosts(Dims d, size_t c0, size_t c1, Ucont u) {
-  RANGE_LOOP(c0, c1) {
-    DECOMP(d, i, j, k);
-    int a = wrapi(i, d.mx, d.ip), b = wrapi(j, d.my, d.jp), cc = wrapi(k, d.mz, d.kp);
-    if (a == i && b == j && cc == k) continue;
-    size_t s = cidx(d, a, b, cc);
-    if (a != i) u.x[_t] = u.x[s];
-    if (b != j) u.y[_t] = u.y[s];
-    if (cc != k) u.z[_t] = u.z[s];
+// planes [k0, k1): the i ghost planes of u.x, the j ghost planes of u.y and
+// the k ghost planes of u.z, no other cell.  Every source is interior in all
+// periodic directions, so the sync never reads a cell it writes; the source
+// of a cell on an interior plane k lies on plane k.
+__global__ void k_ucont_ghosts(Dims d, int k0, int k1, Ucont u) {
+  const int nk = k1 - k0, nx = d.ip ? 2 * d.my * nk : 0, ny = d.jp ? 2 * d.mx * nk : 0;
+  const int g0 = k0 == 0 ? 1 : 0, g1 = k1 == d.mz ? 1 : 0;  // k ghost planes in the range
+  const int nz = d.kp ? (g0 + g1) * d.mx * d.my : 0;
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nx + ny + nz; t += gridDim.x * blockDim.x) {
+    int i, j, k;
+    double* a;
+    if (t < nx) {
+      const int q = t >> 1;
+      i = t & 1 ? d.mx - 1 : 0;
+      j = q % d.my;
+      k = k0 + q / d.my;
+      a = u.x;
+    } else if (t < nx + ny) {
+      const int q = t - nx, r = q / d.mx;
+      i = q - r * d.mx;
+      j = r & 1 ? d.my - 1 : 0;
+      k = k0 + (r >> 1);
+      a = u.y;
+    } else {
+      const int q = t - nx - ny, r = q / d.mx;
+      i = q - r * d.mx;
+      j = r % d.my;
+      k = (r >= d.my || !g0) ? d.mz - 1 : 0;
+      a = u.z;
+    }
+    a[cidx(d, i, j, k)] = a[cidx(d, wrapi(i, d.mx, d.ip), wrapi(j, d.my, d.jp), wrapi(k, d.mz, d.kp))];
   }
 }
 
@@ -703,7 +809,10 @@ int launch_projection(const Dims& d, const double* pd, const double* M, const do
 int launch_ucont_ghosts(const Dims& d, const Ucont& u, int k0, int k1, cudaStream_t s) {
   const size_t P = (size_t)d.mx * d.my;
   if (k0 < 0 || k0 >= k1 || k1 > d.mz) return (int)cudaErrorInvalidValue;
-  k_ucont_ghosts<<<nblk((k1 - k0) * P), 256, 0, s>>>(d, k0 * P, k1 * P, u); ++g_launches;
+  const size_t n = (size_t)(d.ip ? 2 * d.my * (k1 - k0) : 0) + (d.jp ? 2 * d.mx * (k1 - k0) : 0) +
+                   (d.kp ? ((k0 == 0) + (k1 == d.mz)) * P : 0);
+  if (n == 0) return (int)cudaSuccess;
+  k_ucont_ghosts<<<nblk(n), 256, 0, s>>>(d, k0, k1, u); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -774,79 +883,95 @@ int launch_contra2cart(const Dims& d, const double* minv, const double* nvert, c
 // non-negative integers exceeds 0.1 exactly when one of them is nonzero, an
 // integer or of the bytes.
 __device__ __forceinline__ bool near_body(const Dims& d, const double* __restrict__ nvert,
-                                          const uint8_t* __restrict__ nb8, size_t c, int i, int j, int k) {
-  if (nb8)
-    return (nb8[c] | nb8[cidx(d, i, j, k + 1)] | nb8[cidx(d, i, j, k - 1)] | nb8[cidx(d, i, j + 1, k)] |
-            nb8[cidx(d, i, j - 1, k)] | nb8[cidx(d, i + 1, j, k)] | nb8[cidx(d, i - 1, j, k)]) != 0;
-  return nvert[c] + nvert[cidx(d, i, j, k + 1)] + nvert[cidx(d, i, j, k - 1)] + nvert[cidx(d, i, j + 1, k)] +
-             nvert[cidx(d, i, j - 1, k)] + nvert[cidx(d, i + 1, j, k)] + nvert[cidx(d, i - 1, j, k)] >
-         0.1;
+                                          const uint8_t* __restrict__ nb8, size_t c) {
+  const size_t sy = d.mx, sz = (size_t)d.mx * d.my;
+  if (nb8) return (nb8[c] | nb8[c + sz] | nb8[c - sz] | nb8[c + sy] | nb8[c - sy] | nb8[c + 1] | nb8[c - 1]) != 0;
+  const double n0 = nvert[c], nt = nvert[c + sz], nbk = nvert[c - sz], nn = nvert[c + sy], ns = nvert[c - sy],
+               ne = nvert[c + 1], nw = nvert[c - 1];
+  // all zero (bits, on the integer pipe) almost everywhere; else the reference's sum
+  if (((abs_bits(n0) | abs_bits(nt) | abs_bits(nbk)) | (abs_bits(nn) | abs_bits(ns)) | (abs_bits(ne) | abs_bits(nw))) == 0ull)
+    return false;
+  return n0 + nt + nbk + nn + ns + ne + nw > 0.1;
 }
 
+// What bounds it: the FP64 pipe, six operations a cell (the test for bodies and
+// the maximum run on the integer pipe: 256x128x128 83 -> TDIV us; a caller's
+// 151x67x93 arrays with doubles for nvert 44.5 -> TNOA us a call).
 __global__ void __launch_bounds__(RB) k_divergence(Dims d, Ucont u, const double* __restrict__ aj,
-                                                   const double* __restrict__ nvert, double* parts,
-                                                   const uint8_t* __restrict__ nb8 = nullptr) {
+                                                   const double* __restrict__ nvert, double* parts, double* out,
+                                                   unsigned* ticket, const uint8_t* __restrict__ nb8) {
   __shared__ double sh[32];
-  double mxv = 0.;
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (!interior(d, i, j, k)) continue;
-    const size_t c = _t;
-    if (near_body(d, nvert, nb8, c, i, j, k)) continue;
-    const double v = fabs((u.x[c] - u.x[cidx(d, i - 1, j, k)] + u.y[c] - u.y[cidx(d, i, j - 1, k)] + u.z[c] -
-                           u.z[cidx(d, i, j, k - 1)]) * aj[c]);
-    mxv = fmax(mxv, v);
+  unsigned long long mxv = 0ull;
+  const size_t sy = d.mx, sz = (size_t)d.mx * d.my;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32) {
+      const size_t c = o + i;
+      const double v = (u.x[c] - u.x[c - 1] + u.y[c] - u.y[c - sy] + u.z[c] - u.z[c - sz]) * aj[c];
+      if (!near_body(d, nvert, nb8, c)) max_abs(mxv, v);
+    }
   }
-  mxv = block_max(mxv, sh);
-  if (threadIdx.x == 0) parts[blockIdx.x] = mxv;
+  mxv = block_maxbits(mxv, sh);
+  if (threadIdx.x == 0) parts[blockIdx.x] = __longlong_as_double((long long)mxv);
+  if (!last_block(ticket)) return;
+  const double m = finish_max(parts, sh);
+  if (threadIdx.x == 0) *out = m;
 }
 int launch_divergence(const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* parts, double* out,
-                      cudaStream_t s, const uint8_t* nb8) {
-  const int nb = nblk(ncell(d), RB);
-  k_divergence<<<nb, RB, 0, s>>>(d, u, aj, nvert, parts, nb8); ++g_launches;
-  k_finish_max<<<1, 256, 0, s>>>(parts, nb, out); ++g_launches;
+                      unsigned* ticket, cudaStream_t s, const uint8_t* nb8) {
+  k_divergence<<<row_blocks(d), RB, 0, s>>>(d, u, aj, nvert, parts, out, ticket, nb8); ++g_launches;
   return (int)cudaGetLastError();
 }
 
-// max |r| over the cells the Divergence check keeps (main.c:1279-1349: the
-// cell and its six face neighbours free of nvert): with st = 1 the projection
-// leaves div u = dt / coeff * r there for the aj-scaled residual r.
-__global__ void __launch_bounds__(RB) k_masked_absmax(Dims d, const double* __restrict__ r, const double* __restrict__ nvert,
-                                                      double* parts, const uint8_t* __restrict__ nb8) {
+// ||r|| over the array and max |r| over the cells the Divergence check keeps
+// (main.c:1279-1349: the cell and its six face neighbours free of nvert): with
+// st = 1 the projection leaves div u = dt / coeff * r there for the aj-scaled
+// residual r (whose ghosts are zero).
+__global__ void __launch_bounds__(RB) k_norm_absmax(Dims d, const double* __restrict__ r, const double* __restrict__ nvert,
+                                                    double* parts, double* out, unsigned* ticket,
+                                                    const uint8_t* __restrict__ nb8) {
   __shared__ double sh[32];
-  double mxv = 0.;
-  GRID_LOOP(d) {
-    DECOMP(d, i, j, k);
-    if (!interior(d, i, j, k)) continue;
-    const size_t c = _t;
-    if (near_body(d, nvert, nb8, c, i, j, k)) continue;
-    mxv = fmax(mxv, fabs(r[c]));
+  unsigned long long mxv = 0ull;
+  double s = 0.;
+  ROW_LOOP(d) {
+    ROW_DECOMP(d, j, k, o, in);
+    if (!in) continue;
+    for (int i = 1 + _lane; i < d.mx - 1; i += 32) {
+      const double v = r[o + i];
+      s = fma(v, v, s);
+      if (!near_body(d, nvert, nb8, o + i)) max_abs(mxv, v);
+    }
   }
-  mxv = block_max(mxv, sh);
-  if (threadIdx.x == 0) parts[blockIdx.x] = mxv;
+  s = block_sum(s, sh);
+  mxv = block_maxbits(mxv, sh);
+  if (threadIdx.x == 0) {
+    parts[gridDim.x + blockIdx.x] = s;
+    parts[blockIdx.x] = __longlong_as_double((long long)mxv);
+  }
+  if (!last_block(ticket)) return;
+  const double m = finish_max(parts, sh);
+  finish_sums<1>(parts + gridDim.x, out, sh);
+  if (threadIdx.x == 0) {
+    out[0] = sqrt(out[0]);
+    out[1] = m;
+  }
 }
-int launch_masked_absmax(const Dims& d, const double* r, const double* nvert, double* parts, double* out, cudaStream_t s,
-                         const uint8_t* nb8) {
-  const int nb = nblk(ncell(d), RB);
-  k_masked_absmax<<<nb, RB, 0, s>>>(d, r, nvert, parts, nb8); ++g_launches;
-  k_finish_max<<<1, 256, 0, s>>>(parts, nb, out); ++g_launches;
+int launch_norm_absmax(const Dims& d, const double* r, const double* nvert, double* parts, double* out, unsigned* ticket,
+                       cudaStream_t s, const uint8_t* nb8) {
+  k_norm_absmax<<<row_blocks(d), RB, 0, s>>>(d, r, nvert, parts, out, ticket, nb8); ++g_launches;
   return (int)cudaGetLastError();
 }
-
-int launch_finish_sums(const double* parts, int nparts, int nq, double* out, cudaStream_t s) {
-  k_finish_sums<<<1, 256, 0, s>>>(parts, nparts, nq, out); ++g_launches;
-  return (int)cudaGetLastError();
-}
-
-int partial_blocks(const Dims& d) { return nblk(ncell(d), RB); }
 
 // ---- allocation-free divergence check (static device scratch) ----
 // The block maxima of k_divergence live in this file-scope array instead of
-// a grid's partials buffer.  nblk() caps a launch at 152 * 16 blocks, so the
-// array always holds one partial per block; every block writes its partial
-// before k_finish_max reads it, so nothing in it has to start at zero.
+// a grid's partials buffer.  row_blocks() caps a launch at 152 * 8 blocks, so
+// the array always holds one partial per block; every block writes its
+// partial before the last one reads it, so none of them has to start at zero.
+// The ticket behind them does: it starts there and every launch leaves it
+// there.
 constexpr int STATIC_PARTS = 152 * 16;
-static __device__ __align__(256) double g_static_parts[STATIC_PARTS];
+static __device__ __align__(256) double g_static_parts[STATIC_PARTS + 1];
 
 int divergence_max_static(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
                           cudaStream_t s, const char** why) {
@@ -881,13 +1006,12 @@ int divergence_max_static(int device, const Dims& d, const Ucont& u, const doubl
     }
     parts = addr[device];
   }
-  const int nb = nblk(ncell(d), RB);
-  if (nb > STATIC_PARTS) {  // unreachable while nblk caps the grid; kept as the stated limit
+  const int nb = row_blocks(d);
+  if (nb > STATIC_PARTS) {  // unreachable while row_blocks caps the grid; kept as the stated limit
     *why = "more block partials than the static scratch holds";
     return 1;
   }
-  k_divergence<<<nb, RB, 0, s>>>(d, u, aj, nvert, parts); ++g_launches;
-  k_finish_max<<<1, 256, 0, s>>>(parts, nb, out); ++g_launches;
+  k_divergence<<<nb, RB, 0, s>>>(d, u, aj, nvert, parts, out, (unsigned*)(parts + STATIC_PARTS), nullptr); ++g_launches;
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     *why = cudaGetErrorString(e);

@@ -160,6 +160,44 @@ __device__ __forceinline__ T block_max(T v, T* sh) {
   return v;
 }
 
+// True in every thread of the block that arrives last (each block calls it
+// once, after its partials): that block sums the partials of all blocks in a
+// fixed order, so the result does not depend on which block it is, and a
+// separate one-block launch is saved.  The
+// ticket is back at zero when the block continues.
+__device__ __forceinline__ bool last_block(unsigned* ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0u;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+// Tests of doubles on the integer pipe (the FP64 pipe takes 16 cycles a warp
+// for each comparison).  below(v, c): v < c for a positive constant c (false
+// for NaN); zero_bits: v is +0 or -0; abs_bits: |v| as an integer that orders
+// like it, for maxima (ABS_INF and below are numbers, NaNs are above).
+constexpr unsigned long long ABS_INF = 0x7FF0000000000000ull;
+__device__ __forceinline__ unsigned long long abs_bits(double v) {
+  return (unsigned long long)__double_as_longlong(v) & 0x7FFFFFFFFFFFFFFFull;
+}
+__device__ __forceinline__ bool below(double v, double c) {
+  return __double_as_longlong(v) < __double_as_longlong(c) && abs_bits(v) <= ABS_INF;
+}
+__device__ __forceinline__ bool at_least(double v, double c) {  // v >= c for a positive constant c
+  return __double_as_longlong(v) >= __double_as_longlong(c) && abs_bits(v) <= ABS_INF;
+}
+__device__ __forceinline__ bool zero_bits(double v) { return abs_bits(v) == 0ull; }
+// Running maximum of |v| that ignores NaNs, as fmax does.
+__device__ __forceinline__ void max_abs(unsigned long long& m, double v) {
+  const unsigned long long a = abs_bits(v);
+  if (a <= ABS_INF && a > m) m = a;
+}
+
 // Exact binary32 -> binary64 widening on the integer pipe, without branches.
 // IEEE 754 fixes the result field by field: a normal number's exponent is
 // rebiased by 1023 - 127 = 896 and its 23-bit fraction becomes the top of the

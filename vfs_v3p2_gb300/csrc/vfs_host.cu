@@ -206,8 +206,10 @@ struct Grid {
   unsigned long long ig_kernels = 0;  // kernels per replay
   double ig_omega = 0.;
   double nfluid = 0.;  // fluid interior cells of the finest level
+  bool bodies = false;  // some nvert is nonzero
   size_t bytes = 0;
   std::vector<void*> allocs;
+  unsigned* ticket() const { return (unsigned*)(scal + 48); }  // arrived blocks of a reduction (0 between launches)
   Ucont U() const { size_t N = ncell(d); return Ucont{u, u + N, u + 2 * N}; }
 };
 
@@ -782,9 +784,8 @@ template <typename T>
 void fg_open_cycle(Grid& g, const vfs_solve_params& p, cudaStream_t s) {
   const size_t N = ncell(g.d);
   Level& F = g.lev[g.L - 1];
-  dbg("v0", 0, launch_vec_scale_first(g.st, g.V, g.V, N, s), s);
-  dbg("scale_in", 0,
-      launch_scale_in<T>(F.d, nullptr, g.V, bbuf<T>(F), &g.st->done, s, dinv_sel<T>(F, mgcfg(p, g.L - 1, g.half_ok).half)), s);
+  dbg("open_v", 0,
+      launch_open_v<T>(g.st, g.V, bbuf<T>(F), N, dinv_sel<T>(F, mgcfg(p, g.L - 1, g.half_ok).half), s), s);
 }
 
 template <typename T>
@@ -816,12 +817,12 @@ int fg_start(vfs_ctx* ctx, Fgmres& f, double atol, bool warm) {
   CK(cudaMemcpyAsync(g.st, &h, sizeof(h), cudaMemcpyHostToDevice, s));
   if (!warm) CK(cudaMemsetAsync(g.phi, 0, N * sizeof(double), s));
   Level& F = g.lev[g.L - 1];
-  dbg("scale_rhs", 0, launch_scale_in<double>(F.d, F.M + F.N * MP_AJ, g.b, g.bs, nullptr, s), s);
-  dbg("bnorm", 0, launch_norm_init(g.st, g.bs, N, g.parts, 1, s), s);
   // r0 = aj b - A phi; from a cold start phi = 0 and r0 = aj b exactly
-  if (warm) dbg("residual0", 0, apply_outer(g, g.phi, g.bs, g.V, &g.st->done, s), s);
-  else CK(cudaMemcpyAsync(g.V, g.bs, N * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  dbg("beta", 0, launch_norm_init(g.st, g.V, N, g.parts, 0, s), s);
+  dbg("open_b", 0, launch_open_b(g.st, F.d, F.M + F.N * MP_AJ, g.b, g.bs, g.V, !warm, g.parts, s), s);
+  if (warm) {
+    dbg("residual0", 0, apply_outer(g, g.phi, g.bs, g.V, &g.st->done, s), s);
+    dbg("beta", 0, launch_beta(g.st, g.V, N, g.parts, s), s);
+  }
   fg_open_cycle<T>(g, p, s);
   g.hstat[0] = 0;
   f.it = 0;
@@ -980,14 +981,13 @@ void fg_cycle_end(Grid& g, const vfs_solve_params& p, bool last, cudaStream_t s,
     Probed pr(VFS_PROBE_ALL, s, "k_x_update", g.L - 1, (double)N * (ncols * (double)sizeof(T) + 16.0));
     dbg("x_update", 0, launch_x_update<T>(g.st, zbase<T>(g), N, g.phi, s), s);
   }
-  dbg("restart_reset", 0, launch_restart_reset(g.st, s), s);
   if (last) return;
   {
     Level& F = g.lev[g.L - 1];
     Probed pr(VFS_PROBE_ALL, s, "k_apply64 (residual)", g.L - 1, (double)n_interior(F.d) * (8.0 * popcount(F.mask) + 24.0));
     apply_outer(g, g.phi, g.bs, g.V, &g.st->done, s);
   }
-  launch_norm_init(g.st, g.V, N, g.parts, 0, s);
+  launch_beta(g.st, g.V, N, g.parts, s);
   fg_open_cycle<T>(g, p, s);
 }
 
@@ -1203,8 +1203,7 @@ int job_check_enqueue(vfs_ctx* ctx, Job& J) {
   }
   {
     Probed pr(VFS_PROBE_ALL, s, "k_norm2 + k_masked_absmax", g.L - 1, (double)N * (8.0 + 8.0 + (g.nb8 ? 1.0 : 8.0)));
-    dbg("norm2", 0, launch_norm2(g.w, N, g.parts, g.scal + 16, s), s);
-    dbg("masked_max", 0, launch_masked_absmax(F.d, g.w, F.nvert, g.parts, g.scal + 17, s, g.nb8), s);
+    dbg("norm_absmax", 0, launch_norm_absmax(F.d, g.w, F.nvert, g.parts, g.scal + 16, g.ticket(), s, g.nb8), s);
   }
   CK(cudaMemcpyAsync(g.hk, g.st, sizeof(KrylovState), cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(g.hv, g.scal + 16, 2 * sizeof(double), cudaMemcpyDeviceToHost, s));
@@ -1241,13 +1240,18 @@ int job_check_eval(vfs_ctx* ctx, Job& J) {
     Level& F = g.lev[g.L - 1];
     const size_t N = ncell(g.d);
     {
-      // per region: nvert and phi read; nvert and phi read, phi written
-      Probed pr(VFS_PROBE_ALL, s, "k_fluid_sum + k_sub_mean", g.L - 1, (double)N * 40.0 * g.ncomp);
-      dbg("remove_mean", 0, launch_remove_mean(F.d, F.nvert, g.phi, g.parts, g.scal, s, g.comp, g.ncomp), s);
+      // the fluid mean of one region is subtracted where phi is finished (nvert
+      // and phi read); several regions take a sum and a subtraction each
+      Probed pr(VFS_PROBE_ALL, s, "k_fluid_sum + k_sub_mean", g.L - 1, (double)N * (g.ncomp > 1 ? 40.0 * g.ncomp : 16.0));
+      if (g.ncomp > 1)
+        dbg("remove_mean", 0,
+            launch_remove_mean(F.d, F.nvert, g.phi, g.parts, g.scal, g.ticket(), s, g.comp, g.ncomp), s);
+      else dbg("fluid_sum", 0, launch_fluid_sum(F.d, F.nvert, g.phi, g.parts, g.scal, g.ticket(), s), s);
     }
     {
-      Probed pr(VFS_PROBE_ALL, s, "k_phi_zero + ghosts", g.L - 1, (double)N * 16.0);
-      dbg("phi_finish", 0, launch_phi_finish(F.d, F.nvert, g.phi, s), s);
+      // nvert and phi read, phi written
+      Probed pr(VFS_PROBE_ALL, s, "k_phi_zero + ghosts", g.L - 1, (double)N * 24.0);
+      dbg("phi_finish", 0, launch_phi_finish(F.d, F.nvert, g.phi, g.ncomp > 1 ? nullptr : g.scal, s), s);
     }
     CK(cudaEventRecord(g.t1, s));
     if (J.post) {
@@ -1830,6 +1834,8 @@ int grid_set_nvert(vfs_ctx* ctx, Grid& g, const double* nvert) {
     for (int j = 1; j < d.my - 1; j++)
       for (int i = 1; i < d.mx - 1; i++)
         if (nvert[cidx(d, i, j, k)] < 0.1) g.nfluid += 1.;
+  g.bodies = false;
+  for (size_t c = 0; c < N && !g.bodies; c++) g.bodies = nvert[c] != 0.;
   std::vector<uint8_t> nbh(N);
   bool integral = true;
   for (size_t c = 0; c < N && integral; c++) {
@@ -2390,7 +2396,7 @@ int vfs_volume_flux(vfs_ctx* ctx, int grid, double out[4]) {
   if (int r_ = check_idle(ctx, gp)) return r_;
   Grid& g = *gp;
   Level& F = g.lev[g.L - 1];
-  launch_volume_flux(F.d, g.immersed ? 1 : 0, g.U(), F.nvert, F.M, g.parts, g.scal, g.s, g.nb8);
+  launch_volume_flux(F.d, g.immersed ? 1 : 0, g.U(), F.nvert, F.M, g.parts, g.scal, g.ticket(), g.s, g.nb8);
   if (out) CK(cudaMemcpyAsync(out, g.scal, 4 * sizeof(double), cudaMemcpyDeviceToHost, g.s));
   CK(cudaStreamSynchronize(g.s));
   return VFS_OK;
@@ -2407,7 +2413,7 @@ int vfs_poisson_rhs(vfs_ctx* ctx, int grid, double dt, double st, double coeff, 
   g.dt = dt;
   g.st_ = st;
   g.coeff = coeff;
-  launch_rhs(F.d, g.U(), F.nvert, dt, st, coeff, meanfix, g.b, g.parts, g.scal + 4, g.s, g.comp, g.ncomp);
+  launch_rhs(F.d, g.U(), F.nvert, dt, st, coeff, meanfix, g.b, g.parts, g.scal + 4, g.ticket(), g.s, g.nb8, g.comp, g.ncomp);
   double sc[2];
   CK(cudaMemcpyAsync(sc, g.scal + 4, 2 * sizeof(double), cudaMemcpyDeviceToHost, g.s));
   CK(cudaStreamSynchronize(g.s));
@@ -2498,7 +2504,7 @@ int vfs_divergence_max(vfs_ctx* ctx, int grid, double* out) {
   if (int r_ = check_idle(ctx, gp)) return r_;
   Grid& g = *gp;
   Level& F = g.lev[g.L - 1];
-  launch_divergence(F.d, g.U(), F.M + F.N * MP_AJ, F.nvert, g.parts, g.scal + 8, g.s, g.nb8);
+  launch_divergence(F.d, g.U(), F.M + F.N * MP_AJ, F.nvert, g.parts, g.scal + 8, g.ticket(), g.s, g.nb8);
   CK(cudaMemcpyAsync(out, g.scal + 8, sizeof(double), cudaMemcpyDeviceToHost, g.s));
   CK(cudaStreamSynchronize(g.s));
   return VFS_OK;
@@ -2520,14 +2526,17 @@ void step_pre(Grid& g, double dt, double st, double coeff) {
     // two passes over the fluid mask (the interface faces' fluxes and metric
     // norms are few)
     Probed pr(VFS_PROBE_ALL, g.s, "k_vflux (2 passes)", g.L - 1, 2.0 * N * nvb);
-    dbg("volume_flux", 0, launch_volume_flux(F.d, g.immersed ? 1 : 0, g.U(), F.nvert, F.M, g.parts, g.scal, g.s, g.nb8),
-        g.s);
+    // without a nonzero nvert there is no interface face: nothing to balance
+    if (g.bodies)
+      dbg("volume_flux", 0,
+          launch_volume_flux(F.d, g.immersed ? 1 : 0, g.U(), F.nvert, F.M, g.parts, g.scal, g.ticket(), g.s, g.nb8), g.s);
   }
   {
     // U (3 components) and nvert read, b written; the mean fix reads nvert and
     // b and writes b
     Probed pr(VFS_PROBE_ALL, g.s, "k_rhs + k_meanfix", g.L - 1, N * (40.0 + 24.0 * g.ncomp));
-    dbg("rhs", 0, launch_rhs(F.d, g.U(), F.nvert, dt, st, coeff, 1, g.b, g.parts, g.scal + 4, g.s, g.comp, g.ncomp),
+    dbg("rhs", 0,
+        launch_rhs(F.d, g.U(), F.nvert, dt, st, coeff, 1, g.b, g.parts, g.scal + 4, g.ticket(), g.s, g.nb8, g.comp, g.ncomp),
         g.s);
   }
 }
@@ -2616,8 +2625,8 @@ int step_post(Grid& g, double dt, double st, double coeff, bool exact, double* u
   {
     // U, aj and the nvert bytes (or doubles) read
     Probed pr(VFS_PROBE_ALL, g.s, "k_divergence", g.L - 1, Nd * (24.0 + 8.0 + (g.nb8 ? 1.0 : 8.0)));
-    dbg("divergence", 0, launch_divergence(F.d, g.U(), F.M + F.N * MP_AJ, F.nvert, g.parts, g.scal + 8, g.s, g.nb8),
-        g.s);
+    dbg("divergence", 0,
+        launch_divergence(F.d, g.U(), F.M + F.N * MP_AJ, F.nvert, g.parts, g.scal + 8, g.ticket(), g.s, g.nb8), g.s);
   }
   if (p_out || u_out) {
     ok(cudaEventRecord(g.ev_cs, g.cs));

@@ -13,21 +13,27 @@ struct Ucont {
   double *x, *y, *z;
 };
 
-int partial_blocks(const Dims& d);
-int launch_finish_sums(const double* parts, int nparts, int nq, double* out, cudaStream_t s);
+// ticket (of the reductions below): an unsigned that is 0 between launches; the
+// launches that share one are ordered.
 int launch_aos2soa(size_t n, const double* aos, double* x, double* y, double* z, cudaStream_t s);
 int launch_soa2aos(size_t n, const double* x, const double* y, const double* z, double* aos, cudaStream_t s);
 // comp / ncomp: labels 0..ncomp-1 of the connected fluid regions (nullptr
 // when the fluid is one region): the compatibility fix and the mean removal
 // then act per region.  sc holds 4 doubles for launch_rhs.
 int launch_rhs(const Dims& d, const Ucont& u, const double* nvert, double dt, double st, double coeff, int meanfix,
-               double* b, double* parts, double* sc, cudaStream_t s, const int* comp = nullptr, int ncomp = 1);
+               double* b, double* parts, double* sc, unsigned* ticket, cudaStream_t s, const uint8_t* nb8 = nullptr,
+               const int* comp = nullptr, int ncomp = 1);
 int launch_volume_flux(const Dims& d, int mode, const Ucont& u, const double* nvert, const double* M, double* parts,
-                       double* fa4, cudaStream_t s,
-                       const uint8_t* nb8 = nullptr);
-int launch_remove_mean(const Dims& d, const double* nvert, double* x, double* parts, double* sc, cudaStream_t s,
-                       const int* comp = nullptr, int ncomp = 1);
-int launch_phi_finish(const Dims& d, const double* nvert, double* phi, cudaStream_t s);
+                       double* fa4, unsigned* ticket, cudaStream_t s, const uint8_t* nb8 = nullptr);
+// subtracts each region's fluid mean from x
+int launch_remove_mean(const Dims& d, const double* nvert, double* x, double* parts, double* sc, unsigned* ticket,
+                       cudaStream_t s, const int* comp, int ncomp);
+// sum and count of x over the fluid (sc[0..1])
+int launch_fluid_sum(const Dims& d, const double* nvert, const double* x, double* parts, double* sc, unsigned* ticket,
+                     cudaStream_t s);
+// phi of a solve: the mean of sc subtracted on the fluid (sc nullable), zero on
+// boundary and solid cells, periodic ghosts
+int launch_phi_finish(const Dims& d, const double* nvert, double* phi, const double* sc, cudaStream_t s);
 int launch_update_pressure(const Dims& d, const double* nvert, const double* phi, double* p, cudaStream_t s);
 int launch_proj_dots(const Dims& d, const double* M, double* pd, cudaStream_t s);
 // nb8: nvert as bytes when every value is an integer in [0, 127] (exact
@@ -56,11 +62,12 @@ int launch_inverse_metric(const Dims& d, const double* M, const double* nvert, d
 // allocation); returns 0, 1 (argument) or 2 (CUDA) and sets *why on error.
 int divergence_max_static(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
                           cudaStream_t s, const char** why);
-int launch_masked_absmax(const Dims& d, const double* r, const double* nvert, double* parts, double* out, cudaStream_t s,
-                         const uint8_t* nb8 = nullptr);
+// out[0] = ||r||_2 over the array, out[1] = max |r| over the cells the
+// divergence check keeps
+int launch_norm_absmax(const Dims& d, const double* r, const double* nvert, double* parts, double* out, unsigned* ticket,
+                       cudaStream_t s, const uint8_t* nb8 = nullptr);
 int launch_divergence(const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* parts, double* out,
-                      cudaStream_t s,
-                      const uint8_t* nb8 = nullptr);
+                      unsigned* ticket, cudaStream_t s, const uint8_t* nb8 = nullptr);
 
 // ---- FGMRES device state (k_krylov.cu) ----
 // One flexible GMRES(m) solve keeps all of its scalars on the device so an
@@ -89,8 +96,14 @@ struct KrylovState {
 
 // parts must hold nblocks * (m + 2) doubles.
 int krylov_nblocks(size_t n);
-int launch_norm_init(KrylovState* st, const double* r, size_t n, double* parts, int is_b, cudaStream_t s);
-int launch_vec_scale_first(KrylovState* st, const double* r, double* v0, size_t n, cudaStream_t s);
+// a round's opening: bs = aj b, bnorm, and on a cold start V_0 = bs with beta
+int launch_open_b(KrylovState* st, const Dims& d, const double* aj, const double* b, double* bs, double* V, bool cold,
+                  double* parts, cudaStream_t s);
+// beta of a warm start's or restart's residual r
+int launch_beta(KrylovState* st, const double* r, size_t n, double* parts, cudaStream_t s);
+// v = r / beta in place and out = T(v)
+template <typename T>
+int launch_open_v(const KrylovState* st, double* v, T* out, size_t n, const float* dinv, cudaStream_t s);
 int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
                     cudaStream_t s);
 // close: the launch's last block closes the Arnoldi column (what
@@ -113,11 +126,8 @@ int launch_vnext_in(KrylovState* st, const double* w, double* vn, T* out, size_t
 template <typename T>
 int launch_apply64_krylov(const OpView<double>& A, const T* z, T* Z, const KrylovState* st, double* w, cudaStream_t s);
 int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, int* hst, cudaStream_t s);
-int launch_vnext(KrylovState* st, const double* w, double* vn, size_t n, cudaStream_t s);
 int launch_lsq_update(KrylovState* st, cudaStream_t s);
 template <typename T>
 int launch_x_update(KrylovState* st, const T* Z, size_t n, double* x, cudaStream_t s);
-int launch_restart_reset(KrylovState* st, cudaStream_t s);
-int launch_norm2(const double* v, size_t n, double* parts, double* out, cudaStream_t s);
 
 }  // namespace vfs
