@@ -49,9 +49,12 @@ static inline int nblk(size_t n, int bs = 256) {
   const size_t o = (size_t)_r * (d).mx;                                         \
   const bool in = j > 0 && k > 0 && j < (d).my - 1 && k < (d).mz - 1
 
-static inline int row_blocks(const Dims& d) {
+// Blocks of a reduction (four per SM: a block's FP64 sums and the fence before
+// its ticket cost as much as several rows; 256x128x128 divergence 84 us at 16,
+// 76 at 8, 72 at 4) and of an update without one (eight).
+static inline int row_blocks(const Dims& d, int per_sm = 4) {
   const int b = ((size_t)d.my * d.mz + RB / 32 - 1) / (RB / 32);
-  return b < 152 * 8 ? b : 152 * 8;
+  return b < 152 * per_sm ? b : 152 * per_sm;
 }
 
 // Sums of NQ per-block partials (parts[q * nblocks + b]) in a fixed order, by
@@ -125,16 +128,17 @@ __global__ void __launch_bounds__(RB) k_rhs(Dims d, Ucont u, const double* __res
     for (int i = _lane; i < d.mx; i += 32) {
       const size_t c = o + i;
       double val = 0.;
-      if (in && i > 0 && i < d.mx - 1 && (nb8 ? nb8[c] == 0 : !at_least(nvert[c], 0.1))) {
+      if (in && i > 0 && i < d.mx - 1) {  // the fluid test by select, so that no load waits for it
+        const bool fluid = nb8 ? nb8[c] == 0 : !at_least(nvert[c], 0.1);
         // (0 - u_x) + u_x(i-1) is exactly the first difference
-        val = u.x[(i == 1 && d.ip) ? o + d.mx - 2 : c - 1] - u.x[c];
-        val -= u.y[c];
-        val += u.y[c + os];
-        val -= u.z[c];
-        val += u.z[c + ob];
-        val *= scale;
+        double v = u.x[(i == 1 && d.ip) ? o + d.mx - 2 : c - 1] - u.x[c];
+        v -= u.y[c];
+        v += u.y[c + os];
+        v -= u.z[c];
+        v += u.z[c + ob];
+        val = fluid ? v * scale : 0.;
         lsum += val;
-        lcnt += 1;
+        lcnt += fluid;
       }
       b[c] = val;
     }
@@ -168,7 +172,7 @@ int launch_rhs(const Dims& d, const Ucont& u, const double* nvert, double dt, do
     return launch_remove_mean(d, nvert, b, parts, sc + 2, ticket, s, comp, ncomp);
   }
   if (meanfix) {
-    k_meanfix<<<nb, RB, 0, s>>>(d, nvert, sc, b);
+    k_meanfix<<<row_blocks(d, 8), RB, 0, s>>>(d, nvert, sc, b);
     ++g_launches;
   }
   return (int)cudaGetLastError();
@@ -211,7 +215,8 @@ __global__ void __launch_bounds__(RB) k_vflux(Dims d, int mode, int phase, Ucont
       const size_t c = o + i;
       if (nb8) {
         const int a = nb8[c];
-        if (a == nb8[c + off[0]] && a == nb8[c + off[1]] && a == nb8[c + off[2]]) continue;
+        // (no short circuit: the four loads go together)
+        if (((a ^ nb8[c + off[0]]) | (a ^ nb8[c + off[1]]) | (a ^ nb8[c + off[2]])) == 0) continue;
       }
       const bool lim1[3] = {i < d.mx - 2, j < d.my - 2, k < d.mz - 2};
 #pragma unroll
@@ -383,7 +388,7 @@ __global__ void __launch_bounds__(RB) k_phi_finish(Dims d, const double* __restr
   }
 }
 int launch_phi_finish(const Dims& d, const double* nvert, double* phi, const double* sc, cudaStream_t s) {
-  k_phi_finish<<<row_blocks(d), RB, 0, s>>>(d, nvert, sc, phi); ++g_launches;
+  k_phi_finish<<<row_blocks(d, 8), RB, 0, s>>>(d, nvert, sc, phi); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -407,7 +412,7 @@ __global__ void __launch_bounds__(RB) k_update_p(Dims d, const double* __restric
   }
 }
 int launch_update_pressure(const Dims& d, const double* nvert, const double* phi, double* p, cudaStream_t s) {
-  k_update_p<<<row_blocks(d), RB, 0, s>>>(d, nvert, phi, p); ++g_launches;
+  k_update_p<<<row_blocks(d, 8), RB, 0, s>>>(d, nvert, phi, p); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -895,8 +900,8 @@ __device__ __forceinline__ bool near_body(const Dims& d, const double* __restric
 }
 
 // What bounds it: the FP64 pipe, six operations a cell (the test for bodies and
-// the maximum run on the integer pipe: 256x128x128 83 -> TDIV us; a caller's
-// 151x67x93 arrays with doubles for nvert 44.5 -> TNOA us a call).
+// the maximum run on the integer pipe: 256x128x128 83 -> 72 us; a caller's
+// 151x67x93 arrays with doubles for nvert 44.6 -> 28.7 us a call).
 __global__ void __launch_bounds__(RB) k_divergence(Dims d, Ucont u, const double* __restrict__ aj,
                                                    const double* __restrict__ nvert, double* parts, double* out,
                                                    unsigned* ticket, const uint8_t* __restrict__ nb8) {
@@ -965,7 +970,7 @@ int launch_norm_absmax(const Dims& d, const double* r, const double* nvert, doub
 
 // ---- allocation-free divergence check (static device scratch) ----
 // The block maxima of k_divergence live in this file-scope array instead of
-// a grid's partials buffer.  row_blocks() caps a launch at 152 * 8 blocks, so
+// a grid's partials buffer.  row_blocks() caps a launch at 152 * 4 blocks, so
 // the array always holds one partial per block; every block writes its
 // partial before the last one reads it, so none of them has to start at zero.
 // The ticket behind them does: it starts there and every launch leaves it
