@@ -144,7 +144,7 @@ __global__ void __launch_bounds__(KB) k_open_v(const KrylovState* st, double* v,
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const double a = v[t] * f;
     v[t] = a;
-    out[t] = dinv ? (T)a * (T)dinv[t] : (T)a;
+    out[t] = dinv ? from_double<T>(a) * (T)dinv[t] : from_double<T>(a);
   }
 }
 template <typename T>
@@ -190,6 +190,7 @@ __device__ __forceinline__ int warp_sum8_index(int lane) { return (lane & 16 ? 4
 // stride of the block partials in four chains, then the warp tree.
 __device__ __forceinline__ void dots_finish(KrylovState* st, const double* parts, int nparts, int nv, int pass) {
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const double m = column_scale(st).m;
   for (int q = threadIdx.x >> 5; q < nv; q += nw) {
     const double* pq = parts + (size_t)q * nparts;
     double s[4] = {0., 0., 0., 0.};
@@ -198,7 +199,7 @@ __device__ __forceinline__ void dots_finish(KrylovState* st, const double* parts
       for (int u = 0; u < 4; u++)
         if (p + 32 * u < nparts) s[u] += __ldcg(pq + p + 32 * u);
     }
-    const double t = warp_sum((s[0] + s[1]) + (s[2] + s[3])) * st->vs[q];
+    const double t = warp_sum((s[0] + s[1]) + (s[2] + s[3])) * st->vs[q] * m;
     if (lane == 0) {
       st->h[q] = t;
       st->hacc[q] = (pass == 1) ? t : st->hacc[q] + t;
@@ -289,7 +290,7 @@ __device__ __forceinline__ void arnoldi_close(KrylovState* st, const double* par
   }
   s = block_sum(s, sh);  // (its barriers also order the staging)
   if (threadIdx.x != 0) return;
-  const double hn = sqrt(s);
+  const double nw = sqrt(s), hn = nw * column_scale(st).m;  // of the stored column, and its value's
   double* Hc = st->H + (size_t)j * (m + 1);
   hc[j + 1] = hn;
   for (int q = 0; q < j; q++) {
@@ -309,7 +310,7 @@ __device__ __forceinline__ void arnoldi_close(KrylovState* st, const double* par
   st->g[j] = c * st->g[j];
   st->resid = fabs(st->g[j + 1]);
   st->hn = hn;
-  st->inv_hn = hn > 0. ? 1. / hn : 0.;
+  st->inv_hn = nw > 0. ? 1. / nw : 0.;
   st->vs[j + 1] = st->orth2 ? 1. : st->inv_hn;  // CGS2 normalises the column in k_vnext_in
   st->j = j + 1;
   st->it += 1;
@@ -341,7 +342,8 @@ __global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double*
   nv = nv_of(st, nv);
   __shared__ double sh[32];
   __shared__ double hs[72];
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q];
+  const double m = column_scale(st).m;
+  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q] / m;
   __syncthreads();
   double s = 0.;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
@@ -378,7 +380,8 @@ __global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, c
   const int nv = st->j + 1;
   __shared__ double sh[32];
   __shared__ double hs[72];
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q];
+  const double m = column_scale(st).m;
+  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q] / m;
   __syncthreads();
   double* vn = V + (size_t)nv * n;
   double s = 0.;
@@ -396,8 +399,8 @@ __global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, c
     }
     vn[t] = a0;
     vn[t + stride] = a1;
-    out[t] = dinv ? (T)a0 * (T)dinv[t] : (T)a0;
-    out[t + stride] = dinv ? (T)a1 * (T)dinv[t + stride] : (T)a1;
+    out[t] = dinv ? from_double<T>(a0) * (T)dinv[t] : from_double<T>(a0);
+    out[t + stride] = dinv ? from_double<T>(a1) * (T)dinv[t + stride] : from_double<T>(a1);
     s = fma(a0, a0, s);
     s = fma(a1, a1, s);
   }
@@ -406,7 +409,7 @@ __global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, c
 #pragma unroll 4
     for (int q = 0; q < nv; q++) a = fma(-hs[q], V[(size_t)q * n + t], a);
     vn[t] = a;
-    out[t] = dinv ? (T)a * (T)dinv[t] : (T)a;
+    out[t] = dinv ? from_double<T>(a) * (T)dinv[t] : from_double<T>(a);
     s = fma(a, a, s);
   }
   s = block_sum(s, sh);
@@ -438,7 +441,8 @@ __global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const do
   if (nv <= NV0 || nv > NV) return;
   __shared__ double hs[NV];
   __shared__ double red[KB / 32][NV];
-  for (int q = threadIdx.x; q < NV; q += blockDim.x) hs[q] = q < nv ? st->h[q] * st->vs[q] : 0.;
+  const double m = column_scale(st).m;
+  for (int q = threadIdx.x; q < NV; q += blockDim.x) hs[q] = q < nv ? st->h[q] * st->vs[q] / m : 0.;
   __syncthreads();
   double acc[NV];
 #pragma unroll
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(KB) k_vnext_in(const KrylovState* st, const do
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const double v = w[t] * f;
     vn[t] = v;
-    out[t] = dinv ? (T)v * (T)dinv[t] : (T)v;
+    out[t] = dinv ? from_double<T>(v) * (T)dinv[t] : from_double<T>(v);
   }
 }
 template <typename T>

@@ -35,22 +35,33 @@ __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_apply64(OpView<dou
   }
 }
 
+// The instantiation of a slot set.
+#define BY_SLOTS(mask, CALL)                 \
+  do {                                       \
+    if (fits_ch(mask)) CALL(MASK_CH);        \
+    else if (fits_tr(mask)) CALL(MASK_TR);   \
+    else CALL(MASK_ALL);                     \
+  } while (0)
+
 int launch_apply64(const OpView<double>& A, const double* x, const double* b, double* y, cudaStream_t s) {
-  if (fits_ch(A.mask)) k_apply64<MASK_CH, double><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y);
-  else k_apply64<MASK_ALL, double><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y);
+#define CALL(M) k_apply64<M, double><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y)
+  BY_SLOTS(A.mask, CALL);
+#undef CALL
   ++g_launches;
   return (int)cudaGetLastError();
 }
 int launch_apply64_xf(const OpView<double>& A, const float* x, const double* b, double* y, cudaStream_t s) {
-  if (fits_ch(A.mask)) k_apply64<MASK_CH, float><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y);
-  else k_apply64<MASK_ALL, float><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y);
+#define CALL(M) k_apply64<M, float><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, x, b, y)
+  BY_SLOTS(A.mask, CALL);
+#undef CALL
   ++g_launches;
   return (int)cudaGetLastError();
 }
 
 // Outer operator inside the Krylov iteration: z (multigrid precision) is the
 // V-cycle applied to the stored column V_j, so the flexible direction of the
-// basis vector vs_j V_j is vs_j z; w = vs_j (A z) in FP64, and z is copied to
+// basis vector vs_j V_j is vs_j z; w = vs_j (A z) in FP64 (with FP32
+// directions over the rest of the scale, column_scale), and z is copied to
 // its Krylov slot Z[st->j] (the solution update applies vs_j again); z[c] is
 // loaded for the stencil's centre anyway.
 template <unsigned MASK, typename T>
@@ -59,18 +70,29 @@ __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_apply64_krylov(OpV
   if (skipped(A.skip)) return;
   T* zj = Z + (size_t)st->j * ncell(A.d);
   const double vs = st->vs[st->j];
+  const float p2 = column_scale(st).p2;
   TILE_LOOP_Z(A.d, plane_block(A.flip, blockIdx.z, gridDim.z)) {
-    const double s = stencil_clamped<MASK, double>(A.d, A.coef, z, i, j, k);
+    double cv[19];
+    T xv[19];
+    stencil_gather<MASK>(A.d, A.coef, z, min(i, A.d.mx - 2), min(j, A.d.my - 2), k, cv, xv);
+    const T zc = xv[CP];
+    if constexpr (sizeof(T) == 4) {
+#pragma unroll
+      for (int m = 0; m < 19; m++)
+        if (MASK & (1u << m)) xv[m] *= p2;
+    }
+    const double s = stencil_dot<MASK, double>(cv, xv);
     if (!_in) continue;
     const size_t c = cidx(A.d, i, j, k);
-    w[c] = vs * s;
-    zj[c] = z[c];
+    w[c] = sizeof(T) == 4 ? s : vs * s;
+    zj[c] = zc;
   }
 }
 template <typename T>
 int launch_apply64_krylov(const OpView<double>& A, const T* z, T* Z, const KrylovState* st, double* w, cudaStream_t s) {
-  if (fits_ch(A.mask)) k_apply64_krylov<MASK_CH, T><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, z, Z, st, w);
-  else k_apply64_krylov<MASK_ALL, T><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, z, Z, st, w);
+#define CALL(M) k_apply64_krylov<M, T><<<tile_grid(A.d), dim3(TX, TY), 0, s>>>(A, z, Z, st, w)
+  BY_SLOTS(A.mask, CALL);
+#undef CALL
   ++g_launches;
   return (int)cudaGetLastError();
 }

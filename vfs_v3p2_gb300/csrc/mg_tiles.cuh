@@ -47,6 +47,10 @@ __device__ __forceinline__ int plane_block(int flip, int b, int n) { return flip
 // time every load of a stencil is issued before its FMAs (no per-slot
 // branch), which keeps ~2 x slots loads in flight per cell.
 constexpr unsigned MASK_ALL = 0x7FFFFu;
+// MASK_TR: no i-k cross terms (terrain-following lines over uniform x and z),
+// 15 slots: the FP64 product, whose pipe a slot's FMA occupies (512x256x256:
+// 1217 us on all 19).
+constexpr unsigned MASK_TR = MASK_ALL & ~((1u << TE) | (1u << BE) | (1u << TW) | (1u << BW));
 constexpr unsigned MASK_CH = (1u << CP) | (1u << EP) | (1u << WP) | (1u << NP) | (1u << SP) | (1u << TP) | (1u << BP) |
                              (1u << TE) | (1u << BE) | (1u << TW) | (1u << BW);
 
@@ -173,6 +177,7 @@ __device__ __forceinline__ TA stencil_clamped(const Dims& d, const TC* __restric
   return stencil_dot<MASK, TA>(cv, xv);
 }
 
+__host__ __forceinline__ bool fits_tr(unsigned mask) { return (mask & ~MASK_TR) == 0u; }
 __host__ __forceinline__ bool fits_ch(unsigned mask) { return (mask & ~MASK_CH) == 0u; }
 
 // Storage tag of the FP32 multigrid's face form (OpView::ffi ...): the row

@@ -233,6 +233,41 @@ __host__ __device__ __forceinline__ double widen(float f) {
   return d;
 #endif
 }
+// binary64 -> binary32, to nearest even, on the integer pipe for every value
+// whose result is a normal number or overflows, and for zeros; subnormal
+// results, infinities and NaNs take the hardware conversion (a branch no
+// Krylov vector's cell normally takes).
+__host__ __device__ __forceinline__ float narrow(double v) {
+#ifdef __CUDA_ARCH__
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+#else
+  unsigned long long b;
+  memcpy(&b, &v, sizeof b);
+#endif
+  const unsigned hi = (unsigned)(b >> 32), lo = (unsigned)b;
+  const unsigned e = (hi >> 20) & 0x7ffu, sgn = hi & 0x80000000u;
+  unsigned r;
+  if (e - 897u <= 253u) {  // 2^-126 <= |v| < 2^128
+    const unsigned m = ((hi & 0xfffffu) << 3) | (lo >> 29), rest = lo & 0x1fffffffu;
+    r = (sgn | ((e - 896u) << 23) | m) + ((rest + 0x0fffffffu + (m & 1u)) >> 29);
+  } else if ((b << 1) == 0ull) {
+    r = sgn;
+  } else {
+    return (float)v;
+  }
+#ifdef __CUDA_ARCH__
+  return __uint_as_float(r);
+#else
+  float f;
+  memcpy(&f, &r, sizeof f);
+  return f;
+#endif
+}
+template <typename T>
+__device__ __forceinline__ T from_double(double v) { return (T)v; }
+template <>
+__device__ __forceinline__ float from_double<float>(double v) { return narrow(v); }
+
 // Operand conversion into an accumulator type (widen() for float -> double).
 template <typename TA, typename TX_>
 __device__ __forceinline__ TA to_acc(TX_ v) { return (TA)v; }

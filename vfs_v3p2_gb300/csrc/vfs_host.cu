@@ -808,6 +808,7 @@ int fg_start(vfs_ctx* ctx, Fgmres& f, double atol, bool warm) {
   h.hacc = a; a += p.restart + 2;
   h.vs = a;
   h.orth2 = p.orth == VFS_ORTH_CGS2;
+  h.f32 = sizeof(T) == 4;
   h.epoch = ++g.epoch;
   f.epoch = h.epoch;
   if (!g.st) {

@@ -91,8 +91,27 @@ struct KrylovState {
   double* hacc;   // m+1 accumulated dots of the column
   double* vs;     // m+1 column scales: basis vector q is vs[q] * V_q
   int orth2;      // 1: CGS2 (columns stored normalised, vs = 1)
+  int f32;        // 1: FP32 directions (see column_scale)
   unsigned ticket[1];  // blocks of the running reduction that have arrived (0 between launches)
 };
+
+// The scale vs[j] of the column that opens an iteration, split as p2 m: with
+// FP32 directions the product A z takes the power of two p2 into z (exact, on
+// the FP32 pipe) and leaves the rest m, in [1, 2), to the few scalars that
+// follow, so that it needs no FP64 multiply a cell (one of its twelve
+// operations on 11 slots).  The vectors of the iteration are then 1 / m times
+// their values: w = A z p2, dots times m, and the column stored from it.
+struct ColumnScale {
+  float p2;
+  double m;
+};
+__device__ __forceinline__ ColumnScale column_scale(const KrylovState* st) {
+  const double vs = st->vs[st->j];
+  if (!st->f32) return {1.f, 1.};
+  int e = (int)((__double_as_longlong(vs) >> 52) & 0x7ff) - 1023;
+  e = e < -120 ? -120 : (e > 120 ? 120 : e);  // a float either way; m then takes the rest
+  return {__int_as_float((e + 127) << 23), vs * __longlong_as_double((long long)(1023 - e) << 52)};
+}
 
 // parts must hold nblocks * (m + 2) doubles.
 int krylov_nblocks(size_t n);
