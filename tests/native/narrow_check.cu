@@ -1,7 +1,8 @@
 // Host-side check of vfs::narrow (the integer-pipe binary64 -> binary32
 // rounding of the Krylov kernels) against the compiler's conversion: around
 // every binary32 value of a stride the points and midpoints where rounding
-// turns, pseudo-random doubles over all exponents, and the special classes.
+// turns, pseudo-random doubles over all exponents, and the special classes;
+// and of vfs::widen_normal over the same values.
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -15,6 +16,17 @@ static void check(unsigned long long u) {
   n++;
   if (std::memcmp(&a, &b, 4) != 0 && !(a != a && b != b)) bad++;
 }
+// widen_normal agrees with the conversion unless it says special, and says so
+// exactly for subnormals, infinities and NaNs.
+static void check_normal(float f) {
+  unsigned u;
+  std::memcpy(&u, &f, 4);
+  const unsigned e = (u >> 23) & 0xffu, m = u & 0x7fffffu;
+  bool special = false;
+  const double a = vfs::widen_normal(f, special), b = (double)f;
+  n++;
+  if (special != (e == 0xffu || (e == 0u && m != 0u)) || (!special && std::memcmp(&a, &b, 8) != 0)) bad++;
+}
 static void around(double d) {
   unsigned long long u;
   std::memcpy(&u, &d, 8);
@@ -27,6 +39,7 @@ int main(int argc, char** argv) {
     const unsigned u = (unsigned)t;
     float f, g;
     std::memcpy(&f, &u, 4);
+    check_normal(f);
     const unsigned v = u + 1;
     std::memcpy(&g, &v, 4);
     if (f != f || g != g) continue;
@@ -44,6 +57,11 @@ int main(int argc, char** argv) {
                                         0x7ff8000000000000ull, 0x47efffffe0000000ull, 0x47efffffefffffffull,
                                         0x47effffff0000000ull, 0x3810000000000000ull, 0x380fffffffffffffull};
   for (unsigned long long u : special) check(u);
+  for (unsigned u : {0u, 0x80000000u, 1u, 0x007fffffu, 0x00800000u, 0x7f7fffffu, 0x7f800000u, 0x7fc00000u, 0xff800000u}) {
+    float f;
+    std::memcpy(&f, &u, 4);
+    check_normal(f);
+  }
   std::printf("checked %llu values, %llu mismatches\n", n, bad);
   return bad ? 1 : 0;
 }

@@ -265,9 +265,17 @@ __global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* 
   if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, pass);
 }
 
+// Blocks of the dots: a warp's reduction of eight columns takes nine FP64 adds
+// whatever its cells, so two blocks per SM until a thread has eight cells
+// (104x40x72, 21 columns: 30.4 us a launch at two cells a thread, 23.6 so).
+static int dots_nblocks(size_t n) {
+  const size_t two = (n + KB * 2 - 1) / (KB * 2), eight = (n + KB * 8 - 1) / (KB * 8);
+  const size_t b = eight > 152 * 2 ? eight : (two < 152 * 2 ? two : 152 * 2);
+  return (int)(b > 152 * 4 ? 152 * 4 : (b ? b : 1));
+}
 int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
                     cudaStream_t s) {
-  k_multidot<<<krylov_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, pass); ++g_launches;
+  k_multidot<<<dots_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, pass); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -513,8 +521,19 @@ __global__ void __launch_bounds__(KB) k_x_update(KrylovState* st, const T* __res
   for (int q = threadIdx.x; q < J; q += blockDim.x) ys[q] = st->y[q] * st->vs[q];
   __syncthreads();
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    double a = x[t];
-    for (int q = 0; q < J; q++) a = fma(ys[q], to_acc<double>(Z[(size_t)q * n + t]), a);
+    const double x0 = x[t];
+    double a = x0;
+    bool special = false;
+#pragma unroll 4
+    for (int q = 0; q < J; q++) {
+      const T z = Z[(size_t)q * n + t];
+      if constexpr (sizeof(T) == 4) a = fma(ys[q], widen_normal(z, special), a);
+      else a = fma(ys[q], z, a);
+    }
+    if (special) {
+      a = x0;
+      for (int q = 0; q < J; q++) a = fma(ys[q], to_acc<double>(Z[(size_t)q * n + t]), a);
+    }
     x[t] = a;
   }
   if (last_block(st->ticket) && threadIdx.x == 0) st->j = 0;

@@ -64,6 +64,10 @@ int launch_apply64_xf(const OpView<double>& A, const float* x, const double* b, 
 // directions over the rest of the scale, column_scale), and z is copied to
 // its Krylov slot Z[st->j] (the solution update applies vs_j again); z[c] is
 // loaded for the stencil's centre anyway.
+template <typename T>
+__device__ T slot_value(const Dims& d, const T* x, int i, int j, int k, int m) {
+  return x[cidx(d, wrapi(i + slot_di(m), d.mx, d.ip), wrapi(j + slot_dj(m), d.my, d.jp), wrapi(k + slot_dk(m), d.mz, d.kp))];
+}
 template <unsigned MASK, typename T>
 __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_apply64_krylov(OpView<double> A, const T* __restrict__ z, T* __restrict__ Z,
                                                            const KrylovState* st, double* __restrict__ w) {
@@ -74,14 +78,30 @@ __global__ void __launch_bounds__(TX* TY, VFS_STENCIL_MINB) k_apply64_krylov(OpV
   TILE_LOOP_Z(A.d, plane_block(A.flip, blockIdx.z, gridDim.z)) {
     double cv[19];
     T xv[19];
-    stencil_gather<MASK>(A.d, A.coef, z, min(i, A.d.mx - 2), min(j, A.d.my - 2), k, cv, xv);
+    const int ic = min(i, A.d.mx - 2), jc = min(j, A.d.my - 2);
+    stencil_gather<MASK>(A.d, A.coef, z, ic, jc, k, cv, xv);
     const T zc = xv[CP];
-    if constexpr (sizeof(T) == 4) {
+    double s = 0.;
+    if constexpr (sizeof(T) == 4 && MASK == MASK_CH) {
 #pragma unroll
       for (int m = 0; m < 19; m++)
-        if (MASK & (1u << m)) xv[m] *= p2;
+        if (MASK & (1u << m)) s = fma(cv[m], widen(xv[m] * p2), s);
+    } else if constexpr (sizeof(T) == 4) {
+      // 15 slots and more: the full widening's integer operations would bound
+      // the kernel (512x256x256: 995 -> 930 us; on 11 slots the branch costs
+      // what it saves, 98 -> 101 us)
+      bool special = false;
+#pragma unroll
+      for (int m = 0; m < 19; m++)
+        if (MASK & (1u << m)) s = fma(cv[m], widen_normal(xv[m] * p2, special), s);
+      if (special) {  // subnormals or worse: the row again, gathered again (no registers held for it)
+        s = 0.;
+        for (int m = 0; m < 19; m++)
+          if (MASK & (1u << m)) s = fma(A.coef[(size_t)m * ncell(A.d) + cidx(A.d, ic, jc, k)], widen(slot_value(A.d, z, ic, jc, k, m) * p2), s);
+      }
+    } else {
+      s = stencil_dot<MASK, double>(cv, xv);
     }
-    const double s = stencil_dot<MASK, double>(cv, xv);
     if (!_in) continue;
     const size_t c = cidx(A.d, i, j, k);
     w[c] = sizeof(T) == 4 ? s : vs * s;

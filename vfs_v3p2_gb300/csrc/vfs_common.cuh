@@ -233,6 +233,30 @@ __host__ __device__ __forceinline__ double widen(float f) {
   return d;
 #endif
 }
+// widen() of normal numbers and zeros in 8 integer operations instead of 25;
+// special is set when f is neither (the caller then sums again with widen()).
+// A row of the outer operator widens 11 to 19 values, and at 25 operations each
+// the integer pipe took as long as the FP64 one.
+__host__ __device__ __forceinline__ double widen_normal(float f, bool& special) {
+#ifdef __CUDA_ARCH__
+  const unsigned u = __float_as_uint(f);
+#else
+  unsigned u;
+  memcpy(&u, &f, sizeof u);
+#endif
+  const unsigned t = u & 0x7fffffffu;
+  special |= t - 0x00800000u >= 0x7f000000u && t != 0u;
+  const unsigned hi = (u & 0x80000000u) | (t != 0u ? (t >> 3) + 0x38000000u : 0u);
+#ifdef __CUDA_ARCH__
+  return __hiloint2double((int)hi, (int)(u << 29));
+#else
+  const unsigned long long bits = (unsigned long long)hi << 32 | (u << 29);
+  double d;
+  memcpy(&d, &bits, sizeof d);
+  return d;
+#endif
+}
+
 // binary64 -> binary32, to nearest even, on the integer pipe for every value
 // whose result is a normal number or overflows, and for zeros; subnormal
 // results, infinities and NaNs take the hardware conversion (a branch no
