@@ -577,6 +577,10 @@ __host__ __device__ inline size_t smooth_smem(int tw, int nj) {
   return (size_t)3 * tw * nj * sizeof(T);
 }
 
+// Tiles are a power of two wide: column and row of a tile cell by mask and
+// shift (a run-time division is 25 instructions, twice a cell).
+__device__ __forceinline__ int tile_shift(int tw) { return 31 - __clz(tw); }
+
 // Phase 1 of the sweep on the face form (FP32): U cells per thread batch,
 // every load issued before the arithmetic; writes su, sp, sl of the tile.
 // From a zero guess (ZG) the residual is b and only the j faces and aj are
@@ -588,13 +592,14 @@ __device__ __forceinline__ void face_phase1(const OpView<float>& A, const float*
   const Dims d = A.d;
   const int nj = d.my - 2, sy = d.mx, sz = d.mx * d.my;
   const int okB = ((k == 1 && d.kp) ? d.mz - 3 : -1) * sz, okT = ((k == d.mz - 2 && d.kp) ? 3 - d.mz : 1) * sz;
+  const int sh = tile_shift(tw);
   for (int base = threadIdx.x; base < tw * nj; base += U * VFS_SMOOTH_NT) {
     FaceData f[U];
     float xv[U][11], bb[U], inv[U];
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int idx = min(base + u * VFS_SMOOTH_NT, tw * nj - 1);
-      const int il = idx % tw, jl = idx / tw;
+      const int il = idx & (tw - 1), jl = idx >> sh;
       const int i = min(i0 + il, d.mx - 2), j = 1 + jl;
       const int c = k * sz + j * sy + i;
       const int oiW = (i == 1 && d.ip) ? d.mx - 3 : -1, oiE = (i == d.mx - 2 && d.ip) ? 3 - d.mx : 1;
@@ -628,10 +633,10 @@ __device__ __forceinline__ void face_phase1(const OpView<float>& A, const float*
     for (int u = 0; u < U; u++) {
       const int idx = base + u * VFS_SMOOTH_NT;
       if (idx >= tw * nj) break;
-      const int jl = idx / tw;
+      const int jl = idx >> sh;
       f[u].cc = face_code(f[u].aj);
       f[u].aj = face_aj(f[u].aj);
-      const bool live = (i0 + idx % tw <= d.mx - 2) && f[u].aj != 0.f;
+      const bool live = (i0 + (idx & (tw - 1)) <= d.mx - 2) && f[u].aj != 0.f;
       float x11[19];  // slot-indexed view of the 11 values (TE, BE, TW, BW: the stencil slots)
       if (!ZG) {
         x11[CP] = xv[u][0]; x11[EP] = xv[u][1]; x11[WP] = xv[u][2]; x11[NP] = xv[u][3]; x11[SP] = xv[u][4];
@@ -661,6 +666,7 @@ __device__ __forceinline__ void face_phase1_all(const OpView<float>& A, const fl
   const size_t N = ncell(d);
   const float* __restrict__ csp = A.coef + (size_t)SP * N;
   const float* __restrict__ cnp = A.coef + (size_t)NP * N;
+  const int sh = tile_shift(tw);
   for (int base = threadIdx.x; base < tw * nj; base += U * VFS_SMOOTH_NT) {
     FaceData f[U];
     FaceX e[U];
@@ -668,7 +674,7 @@ __device__ __forceinline__ void face_phase1_all(const OpView<float>& A, const fl
 #pragma unroll
     for (int u = 0; u < U; u++) {
       const int idx = min(base + u * VFS_SMOOTH_NT, tw * nj - 1);
-      const int il = idx % tw, jl = idx / tw;
+      const int il = idx & (tw - 1), jl = idx >> sh;
       const int i = min(i0 + il, d.mx - 2), j = 1 + jl;
       const int c = k * sz + j * sy + i;
       if (ZG) {
@@ -685,9 +691,9 @@ __device__ __forceinline__ void face_phase1_all(const OpView<float>& A, const fl
     for (int u = 0; u < U; u++) {
       const int idx = base + u * VFS_SMOOTH_NT;
       if (idx >= tw * nj) break;
-      const int jl = idx / tw;
+      const int jl = idx >> sh;
       const float aj = face_aj(f[u].aj);
-      const bool live = (i0 + idx % tw <= d.mx - 2) && aj != 0.f;
+      const bool live = (i0 + (idx & (tw - 1)) <= d.mx - 2) && aj != 0.f;
       float ax = 0.f;
       if (!ZG) {
         ax = face_row_all(f[u], e[u], xv[u], av[u], cv[u]);
@@ -730,6 +736,7 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
   const int i0 = 1 + bx * TW;
   const int k = 1 + by;
   constexpr int U = UU;
+  const int sh = tile_shift(TW);
   // L2 prefetch of the rows a warp will stream PF iterations later: the
   // loads in flight are bounded by registers (4 bytes each), the prefetches
   // are not, so they keep more of HBM's latency-bandwidth product busy.  One
@@ -793,7 +800,7 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
     // (few registers a cell: the serial chain of round trips is a quarter).
     // TW divides the block: a thread keeps its column (il) and steps rows by
     // jstep; its cell and coefficient offsets advance by one row pitch.
-    const int il = threadIdx.x % TW, jl0 = threadIdx.x / TW, jstep = VFS_SMOOTH_NT / TW;
+    const int il = threadIdx.x & (TW - 1), jl0 = threadIdx.x >> sh, jstep = VFS_SMOOTH_NT >> sh;
     const int ic = min(i0 + il, d.mx - 2);
     const bool col_in = i0 + il <= d.mx - 2;
     const int c1 = k * d.mx * d.my + d.mx + ic;  // cell (ic, 1, k)
@@ -891,7 +898,7 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
   #pragma unroll
       for (int u = 0; u < U; u++) {
         const int idx = min(base + u * VFS_SMOOTH_NT, TW * nj - 1);
-        const int il = idx % TW, jl = idx / TW;
+        const int il = idx & (TW - 1), jl = idx >> sh;
         const int i = min(i0 + il, d.mx - 2), j = 1 + jl;
         const int c = k * d.mx * d.my + j * d.mx + i;
         if (xi) {
@@ -912,8 +919,8 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
       for (int u = 0; u < U; u++) {
         const int idx = base + u * VFS_SMOOTH_NT;
         if (idx >= TW * nj) break;
-        const int jl = idx / TW;
-        const bool live = (i0 + idx % TW <= d.mx - 2) && (NRM || to_acc<T>(cv[u][CP]) != T(0));
+        const int jl = idx >> sh;
+        const bool live = (i0 + (idx & (TW - 1)) <= d.mx - 2) && (NRM || to_acc<T>(cv[u][CP]) != T(0));
         const T ax = xi ? row_dot<MASK, T>(cv[u], xv[u]) : T(0);
         const T a = jl > 0 ? to_acc<T>(cv[u][SP]) : T(0), cn = jl < nj - 1 ? to_acc<T>(cv[u][NP]) : T(0);
         su[idx] = live ? (bb[u] - ax) * inv[u] : T(0);
@@ -924,14 +931,21 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
     }
   }
   __syncthreads();
-  if (threadIdx.x < TW) line_solve<T>(su, sp, sl, nj, TW, threadIdx.x);
+  // a pitch known at compile time: one warp's issue is the solve's time, and a
+  // run-time pitch takes three integer products a row
+  if (threadIdx.x < TW) {
+    if (TW == 32) line_solve<T>(su, sp, sl, nj, 32, threadIdx.x);
+    else if (TW == 16) line_solve<T>(su, sp, sl, nj, 16, threadIdx.x);
+    else if (TW == 8) line_solve<T>(su, sp, sl, nj, 8, threadIdx.x);
+    else line_solve<T>(su, sp, sl, nj, TW, threadIdx.x);
+  }
   __syncthreads();
   // Phase 3, unrolled so that the old values of several cells are loaded
   // together (columns past the last one are clamped and not stored).
   constexpr int U3 = VFS_SMOOTH_U3;
 #pragma unroll U3
   for (int idx = threadIdx.x; idx < TW * nj; idx += VFS_SMOOTH_NT) {
-    const int il = idx % TW, jl = idx / TW;
+    const int il = idx & (TW - 1), jl = idx >> sh;
     const int i = min(i0 + il, d.mx - 2), j = 1 + jl;
     const int c = k * d.mx * d.my + j * d.mx + i;
     const T x0 = xi ? __ldg(xi + c) : T(0);
