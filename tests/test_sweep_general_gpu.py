@@ -19,6 +19,8 @@ CASES = {
     "rows_over_3_one_level": (62, 23, 110, 1, (0, 0, 0), [(3.1, 0.4, 1.5, 0.3)]),
     "periodic": (32, 32, 152, 2, (1, 1, 1), [(3.1, 0.4, 1.5, 0.3)]),
     "long_lines": (60, 256, 160, 3, (1, 0, 1), ()),
+    # a sheared grid: the i and k faces have each other's cross term as well
+    "sheared": (62, 23, 110, 1, (0, 0, 0), [(3.1, 0.4, 1.5, 0.3)]),
 }
 
 
@@ -26,6 +28,8 @@ CASES = {
 def test_warp_rows_equal_single_cells(gpu_ctx, name):
     ni, nj, nk, levels, per, sph = CASES[name]
     coor = synth.terrain_coords(ni, nj, nk, 2.5)
+    if name == "sheared":
+        coor[: nk + 1, : nj + 1, : ni + 1, 0] += 0.3 * coor[: nk + 1, : nj + 1, : ni + 1, 2]
     nv = synth.sphere_nvert(coor, sph, *per) if sph else np.zeros((nk + 2, nj + 2, ni + 2))
     gid = gpu_ctx.grid_create(coor, nv, levels, 1 if sph else 0, periodic=per)
     try:

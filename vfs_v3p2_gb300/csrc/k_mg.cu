@@ -177,7 +177,9 @@ __global__ void __launch_bounds__(VFS_SMOOTH_NT, PAIR ? VFS_SMOOTH_MINB_HALF : (
 // The face-form sweeps with warp-row neighbours: 30-column tiles; two rows a
 // warp and four blocks per SM on the 11-slot form (smooth_tile_w), four rows
 // and two blocks on the general one (smooth_tile_wg; 512x256x256: 674 us one
-// cell per thread, 1 row 638, 2 rows 619, 4 rows 554, 16 warps a block 599).
+// cell per thread, 1 row 638, 2 rows 619, 4 rows 554, 16 warps a block 599;
+// 513 without the i-k cross terms where the operator has none, XIK -- the
+// restriction gained nothing from that, 384 -> 397 us, and reads them all).
 // What limits both is L1: the line arrays leave 56 KB of it per SM, and a load
 // in flight holds its lines (4 KB more shared memory a block, padded lines,
 // cost 48 -> 69 us and 554 -> 838 us).
@@ -188,23 +190,27 @@ __global__ void __launch_bounds__(VFS_SMOOTH_NT, VFS_SMOOTH_W_MINB)
   extern __shared__ unsigned char smraw[];
   smooth_tile_w<VFS_SMOOTH_W_U>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), smraw);
 }
+template <bool XIK>
 __global__ void __launch_bounds__(VFS_SMOOTH_NT, 2)
     k_smooth_wg(OpView<float> A, const float* __restrict__ lf, const float* __restrict__ xi,
                 const float* __restrict__ b, float* __restrict__ xo, float omega) {
   if (skipped(A.skip)) return;
   extern __shared__ float sm[];
-  smooth_tile_wg<4>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), sm);
+  smooth_tile_wg<4, XIK>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), sm);
 }
 static int smooth_w_launch(const OpView<float>& A, const float* lf, const float* xi, const float* b, float* xo,
                            float omega, cudaStream_t s) {
   static const cudaError_t attr = [] {
-    const cudaError_t e = cudaFuncSetAttribute(k_smooth_w, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_smooth_wg, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024);
+    const auto large = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(k_smooth_w, large, 100 * 1024);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_smooth_wg<false>, large, 100 * 1024);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_smooth_wg<true>, large, 100 * 1024);
   }();
   if (attr != cudaSuccess) return (int)attr;
   const dim3 g((A.d.mx - 2 + SMOOTH_W_TW - 1) / SMOOTH_W_TW, A.d.mz - 2);
   const size_t sm = smooth_smem<float>(32, A.d.my - 2);
-  if (A.ffc) k_smooth_wg<<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
+  if (A.ffc && fits_tr(A.mask)) k_smooth_wg<false><<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
+  else if (A.ffc) k_smooth_wg<true><<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
   else k_smooth_w<<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
   ++g_launches;
   return (int)cudaGetLastError();

@@ -305,32 +305,44 @@ __device__ __forceinline__ float face_cross(float w, float ctr, float up, float 
 // weights, the j cross terms of the i and k faces (the pair at j-1 or j+1
 // unless the regime takes the centre pair) and the j faces' cross terms
 // whose centre pair is the pair they take.  SIDED: some cross term takes a
-// centre pair (its codes are read); else every code is 0.
-template <bool SIDED>
+// centre pair (its codes are read); else every code is 0.  XIK: the i and k
+// faces have each other's cross term (an operator without it, MASK_TR, has
+// none above the drop threshold); else v's i-k corners and the code bits of
+// aj are not read.
+template <bool SIDED, bool XIK>
 __device__ __forceinline__ float face_row_gen(const FaceData& f, const FaceX& e, const float* x, float& s, float& n) {
   const float xc = x[CP], xe = x[EP], xw = x[WP], xn = x[NP], xs = x[SP], xt = x[TP], xb = x[BP];
-  const float xte = x[TE], xbe = x[BE], xtw = x[TW], xbw = x[BW];
   const float xne = x[NE], xse = x[SE], xnw = x[NW], xsw = x[SW], xtn = x[TN], xbn = x[BN], xts = x[TS], xbs = x[BS];
-  const float ce = xc + xe, te = xt + xte, be = xb + xbe;  // pairs along the +i face of c
-  const float wc = xw + xc, tw = xtw + xt, bw = xbw + xb;  // of c-i
-  const float ct = xc + xt, ete = xe + xte, wtw = xw + xtw;  // along the +k face of c
-  const float bc = xb + xc, eb = xbe + xe, wb = xbw + xw;    // of c-k
-  float pi = te - be, pw = tw - bw, pk = ete - wtw, pb = eb - wb;
-  if (SIDED) {
-    pi = ((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be);
-    pw = ((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw);
-    pk = ((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw);
-    pb = ((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb);
+  // the centre pairs along the +i faces of c and c-i and the +k faces of c and c-k
+  const float ce = xc + xe, wc = xw + xc, ct = xc + xt, bc = xb + xc;
+  float ai, aw, ak, ab;  // i-k cross terms of those faces
+  if constexpr (XIK) {
+    const float xte = x[TE], xbe = x[BE], xtw = x[TW], xbw = x[BW];
+    const float te = xt + xte, be = xb + xbe, tw = xtw + xt, bw = xbw + xb;
+    const float ete = xe + xte, wtw = xw + xtw, eb = xbe + xe, wb = xbw + xw;
+    float pi = te - be, pw = tw - bw, pk = ete - wtw, pb = eb - wb;
+    if (SIDED) {
+      pi = ((f.cc & 1u) ? ce : te) - ((f.cc & 2u) ? ce : be);
+      pw = ((f.cw & 1u) ? wc : tw) - ((f.cw & 2u) ? wc : bw);
+      pk = ((f.cc & 4u) ? ct : ete) - ((f.cc & 8u) ? ct : wtw);
+      pb = ((f.cb & 4u) ? bc : eb) - ((f.cb & 8u) ? bc : wb);
+    }
+    ai = f.fic.y * pi;
+    aw = f.fiw.y * pw;
+    ak = f.fkc.y * pk;
+    ab = f.fkb.y * pb;
+  } else {
+    ai = aw = ak = ab = 0.f;
   }
-  const float Fic = face_cross<SIDED>(e.ijc, ce, xn + xne, xs + xse, fmaf(f.fic.x, xe - xc, f.fic.y * pi));
-  const float Fiw = face_cross<SIDED>(e.ijw, wc, xnw + xn, xsw + xs, fmaf(f.fiw.x, xc - xw, f.fiw.y * pw));
+  const float Fic = face_cross<SIDED>(e.ijc, ce, xn + xne, xs + xse, fmaf(f.fic.x, xe - xc, ai));
+  const float Fiw = face_cross<SIDED>(e.ijw, wc, xnw + xn, xsw + xs, fmaf(f.fiw.x, xc - xw, aw));
   const float cn = xc + xn, sc = xs + xc;  // along the +j faces of c and c-j
   const float Fjc = face_cross<SIDED>(e.jkc, cn, xt + xtn, xb + xbn,
                                       face_cross<SIDED>(e.jic, cn, xe + xne, xw + xnw, f.gjc * (xn - xc)));
   const float Fjs = face_cross<SIDED>(e.jks, sc, xts + xt, xbs + xb,
                                       face_cross<SIDED>(e.jis, sc, xse + xe, xsw + xw, f.gjs * (xc - xs)));
-  const float Fkc = face_cross<SIDED>(e.kjc, ct, xn + xtn, xs + xts, fmaf(f.fkc.x, xt - xc, f.fkc.y * pk));
-  const float Fkb = face_cross<SIDED>(e.kjb, bc, xbn + xn, xbs + xs, fmaf(f.fkb.x, xc - xb, f.fkb.y * pb));
+  const float Fkc = face_cross<SIDED>(e.kjc, ct, xn + xtn, xs + xts, fmaf(f.fkc.x, xt - xc, ak));
+  const float Fkb = face_cross<SIDED>(e.kjb, bc, xbn + xn, xbs + xs, fmaf(f.fkb.x, xc - xb, ab));
   if (SIDED) {
     auto nq1 = [](float w) { return (face_xc(w) & 1u) ? 0.f : face_xw(w); };  // upper pair at +1
     auto nq2 = [](float w) { return (face_xc(w) & 2u) ? 0.f : face_xw(w); };  // lower pair at -1
@@ -348,11 +360,13 @@ __device__ __forceinline__ float face_row_gen(const FaceData& f, const FaceX& e,
 }
 // As in face_row, the one-sided cases (beside bodies and walls) are branched
 // around elsewhere.
+template <bool XIK = true>
 __device__ __forceinline__ float face_row_all(const FaceData& f, const FaceX& e, const float* x, float& s, float& n) {
-  const unsigned q = face_xc(e.ijc) | face_xc(e.ijw) | face_xc(e.jic) | face_xc(e.jkc) | face_xc(e.jis) |
-                     face_xc(e.jks) | face_xc(e.kjc) | face_xc(e.kjb);
-  if (q | (f.cc & 0xFu) | (f.cw & 3u) | (f.cb & 0xCu)) return face_row_gen<true>(f, e, x, s, n);
-  return face_row_gen<false>(f, e, x, s, n);
+  unsigned q = face_xc(e.ijc) | face_xc(e.ijw) | face_xc(e.jic) | face_xc(e.jkc) | face_xc(e.jis) |
+               face_xc(e.jks) | face_xc(e.kjc) | face_xc(e.kjb);
+  if (XIK) q |= (f.cc & 0xFu) | (f.cw & 3u) | (f.cb & 0xCu);
+  if (q) return face_row_gen<true, XIK>(f, e, x, s, n);
+  return face_row_gen<false, XIK>(f, e, x, s, n);
 }
 // face_gather plus the cross weights of c, c-i, c-j, c-k and the eight x
 // values face_row leaves out (NE SE NW SW TN BN TS BS), periodic wraps as in
@@ -1125,7 +1139,7 @@ __device__ __forceinline__ void put_line(float* su, float* sp, float* sl, int jl
 }
 
 // Rows jb .. jb + U - 1 of a tile, every load issued before any arithmetic.
-template <int U>
+template <int U, bool XIK>
 __device__ __forceinline__ void warp_rows(const OpView<float>& A, const WarpTile& p, const float* __restrict__ lf,
                                           const float* __restrict__ x, const float* __restrict__ b, float* su, float* sp,
                                           float* sl, int jb) {
@@ -1154,7 +1168,7 @@ __device__ __forceinline__ void warp_rows(const OpView<float>& A, const WarpTile
     gj[u + 1] = p.comp ? ldb(A.ffj, c) : 0.f;
     fkc[u] = p.comp ? ldb(A.ffk, 2u * c) : make_float2(0.f, 0.f);
     fkb[u] = p.comp ? ldb(A.ffk, 2u * (c + p.okB)) : make_float2(0.f, 0.f);
-    ajb[u] = p.comp ? ldb(A.faj, c + p.okB) : 0.f;
+    ajb[u] = XIK && p.comp ? ldb(A.faj, c + p.okB) : 0.f;
     cr[u + 1] = ldb(A.ffc, 4u * c);
     kjb[u] = p.comp ? ldb(reinterpret_cast<const float*>(A.ffc), 4u * (c + p.okB) + 12u) : 0.f;
     bb[u] = p.comp ? ldb(b, c) : 0.f;
@@ -1179,19 +1193,22 @@ __device__ __forceinline__ void warp_rows(const OpView<float>& A, const WarpTile
     v[WP] = cw[u + 1];
     v[TP] = xt[u + 1];
     v[BP] = xb[u + 1];
-    v[TE] = from_e(v[TP]);
-    v[TW] = from_w(v[TP]);
-    v[BE] = from_e(v[BP]);
-    v[BW] = from_w(v[BP]);
+    if constexpr (XIK) {
+      v[TE] = from_e(v[TP]);
+      v[TW] = from_w(v[TP]);
+      v[BE] = from_e(v[BP]);
+      v[BW] = from_w(v[BP]);
+      f.fiw.y = from_w(fic[u].y);
+      f.cw = face_code(from_w(ajr[u]));
+    }
     f.fic = fic[u];
-    f.fiw = make_float2(from_w(fic[u].x), from_w(fic[u].y));
+    f.fiw.x = from_w(fic[u].x);
     f.fkc = fkc[u];
     f.fkb = fkb[u];
     f.gjc = gj[u + 1];
     f.gjs = gj[u];
     f.aj = face_aj(ajr[u]);
     f.cc = face_code(ajr[u]);
-    f.cw = face_code(from_w(ajr[u]));
     f.cb = face_code(ajb[u]);
     const bool live = p.comp && f.aj != 0.f;
     v[SE] = ce[u];
@@ -1204,14 +1221,14 @@ __device__ __forceinline__ void warp_rows(const OpView<float>& A, const WarpTile
     v[BN] = xb[u + 2];
     const FaceX e{cr[u + 1].x, from_w(cr[u + 1].x), cr[u + 1].y, cr[u + 1].z, cr[u].y, cr[u].z, cr[u + 1].w, kjb[u]};
     float s, n;
-    const float ax = face_row_all(f, e, v, s, n);
+    const float ax = face_row_all<XIK>(f, e, v, s, n);
     put_line(su, sp, sl, jl, nj, live, bb[u] - ax, inv[u], s * f.aj, n * f.aj);
   }
 }
 
 // A tile of the sweep: residuals by all warps, column solves by the first, the
 // write by all.
-template <int U>
+template <int U, bool XIK>
 __device__ __forceinline__ void smooth_tile_wg(const OpView<float>& A, const float* __restrict__ lf,
                                               const float* __restrict__ xi, const float* __restrict__ b,
                                               float* __restrict__ xo, float omega, int bx, int by, float* su) {
@@ -1219,7 +1236,7 @@ __device__ __forceinline__ void smooth_tile_wg(const OpView<float>& A, const flo
   const int nj = A.d.my - 2, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float *sp = su + 32 * nj, *sl = sp + 32 * nj;
   const WarpTile p = warp_tile(A.d, bx, by);
-  for (int jb = warp * U; jb < nj; jb += NW * U) warp_rows<U>(A, p, lf, xi, b, su, sp, sl, jb);
+  for (int jb = warp * U; jb < nj; jb += NW * U) warp_rows<U, XIK>(A, p, lf, xi, b, su, sp, sl, jb);
   __syncthreads();
   if (warp == 0) line_solve<float>(su, sp, sl, nj, 32, lane);
   __syncthreads();
