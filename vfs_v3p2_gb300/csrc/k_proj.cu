@@ -564,10 +564,13 @@ __global__ void __launch_bounds__(128) k_projection(Dims d, size_t c0, size_t c1
 // per cross term two code bits choosing its upper and lower pair (the pair
 // beside the face, or the face's own pair for a one-sided difference).  The
 // step then applies, per face, U -= (wN dn + wA (Up_A - Lo_A) + wB (Up_B -
-// Lo_B)) dt st / coeff with FMAs: at most 33 FP64 operations per cell
-// instead of about 60, and no nvert loads.  The same
-// products in a different order: the result differs from the reference's
-// operation order by rounding (<= 1e-14 relative).
+// Lo_B)) dt st / coeff with FMAs and no nvert loads: 9 FP64 operations per
+// cell and 4 per cross term in use, at most 33, instead of about 60 (they
+// bound the kernel).  The same products in a
+// different order: the result differs from the reference's operation order
+// by rounding (<= 1e-14 relative).  used: bit q is set where some weight
+// pw[q] is not zero (grids uniform along an axis have whole arrays of zero
+// cross weights, which the step does not read).
 // pw: [9][N] (i face: normal, j cross, k cross | j face: normal, i cross,
 // k cross | k face: normal, i cross, j cross); pc: two bits per cross term
 // in that order (bit 0: the upper pair is the face's own, bit 1: the lower),
@@ -576,8 +579,10 @@ __global__ void __launch_bounds__(128) k_projection(Dims d, size_t c0, size_t c1
 // ---------------------------------------------------------------------------
 __global__ void k_proj_weights(Dims d, const double* __restrict__ pd, const double* __restrict__ iaj,
                                const double* __restrict__ jaj, const double* __restrict__ kaj,
-                               const double* __restrict__ nvert, double* __restrict__ pw, uint16_t* __restrict__ pc) {
+                               const double* __restrict__ nvert, double* __restrict__ pw, uint16_t* __restrict__ pc,
+                               unsigned* __restrict__ used) {
   const size_t N = ncell(d);
+  unsigned mine = 0;
   const int mx = d.mx, my = d.my, mz = d.mz, ip = d.ip, jp = d.jp, kp = d.kp;
   const double THR = VFS_THR;
   GRID_LOOP(d) {
@@ -646,15 +651,21 @@ __global__ void k_proj_weights(Dims d, const double* __restrict__ pd, const doub
 #undef GT2
 #undef LT2
 #pragma unroll
-    for (int q = 0; q < 9; q++) pw[(size_t)q * N + c] = w[q];
+    for (int q = 0; q < 9; q++) {
+      pw[(size_t)q * N + c] = w[q];
+      if (w[q] != 0.) mine |= 1u << q;
+    }
     pc[c] = (uint16_t)code;
   }
+  mine = __reduce_or_sync(0xFFFFFFFFu, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicOr(used, mine);
 }
 
 int launch_proj_weights(const Dims& d, const double* pd, const double* M, const double* nvert, double* pw, uint16_t* pc,
-                        cudaStream_t s) {
+                        unsigned* used, cudaStream_t s) {
   const size_t N = ncell(d);
-  k_proj_weights<<<nblk(N), 256, 0, s>>>(d, pd, M + N * MP_IAJ, M + N * MP_JAJ, M + N * MP_KAJ, nvert, pw, pc);
+  VFS_CUDA_OK(cudaMemsetAsync(used, 0, sizeof(unsigned), s));
+  k_proj_weights<<<nblk(N), 256, 0, s>>>(d, pd, M + N * MP_IAJ, M + N * MP_JAJ, M + N * MP_KAJ, nvert, pw, pc, used);
   ++g_launches;
   return (int)cudaGetLastError();
 }
@@ -662,9 +673,14 @@ int launch_proj_weights(const Dims& d, const double* pd, const double* M, const 
 // U -= sc (wN dn + wA (Up_A - Lo_A) + wB (Up_B - Lo_B)) on the projected
 // faces of the cells [c0, c1) (interior planes; the face bits are set on
 // interior cells only, and the normal difference wraps only on a periodic
-// seam, where alone the last face is projected); a cross term of weight 0
-// loads nothing; every phi read lies in the array (ghost layers included).
-__global__ void __launch_bounds__(128) k_projection_fast(Dims d, size_t c0, size_t c1, const double* __restrict__ pw,
+// seam, where alone the last face is projected).  All loads but the cross
+// terms' wait for nothing, and those only for the code; every phi read lies in
+// the array: the seven points of any cell of an interior plane do, the cross
+// terms' are read by interior cells.  The FP64 pipe bounds it (branches for
+// the one-sided and zero terms ran 23 operations where 17 are needed):
+// 256x128x128 (i-k terms only) 234 -> 164 us, 512x256x256 2361 -> 1833.
+__global__ void __launch_bounds__(128) k_projection_fast(Dims d, size_t c0, size_t c1, unsigned used,
+                                                         const double* __restrict__ pw,
                                                          const uint16_t* __restrict__ pc,
                                                          const double* __restrict__ phi, double sc, Ucont u) {
   const size_t N = ncell(d);
@@ -674,41 +690,39 @@ __global__ void __launch_bounds__(128) k_projection_fast(Dims d, size_t c0, size
     DECOMP(d, i, j, k);
     const int c = (int)_t;
     const unsigned code = pc[c];
-    // pair difference: (upper or own pair) - (lower or own pair), pairs along offset o from cells a, b
-    auto pair = [&](int a, int b, int o, unsigned bits) -> double {
-      const double own = phi[a] + phi[b];
-      const double up = (bits & 1u) ? own : phi[a + o] + phi[b + o];
-      const double lo = (bits & 2u) ? own : phi[a - o] + phi[b - o];
-      return up - lo;
+    double w[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) w[q] = (used >> q) & 1u ? pw[(size_t)q * N + c] : 0.;
+    const double pc0 = phi[c];
+    const double pe = phi[i == mx - 2 ? c + 3 - mx : c + 1];
+    const double pn = phi[j == my - 2 ? c + (3 - my) * sy : c + sy];
+    const double pt = phi[k == mz - 2 ? c + (3 - mz) * sz : c + sz];
+    const double ux = u.x[c], uy = u.y[c], uz = u.z[c];
+    // t + weight (upper - lower pair of c and c + e along o) for cross term q;
+    // a one-sided term takes the face's own pair by offset, not by branch or
+    // select of sums (both cost FP64 operations), and a face that is not
+    // projected or a zero weight takes none
+    auto cross = [&](int q, double t, unsigned face, int e, int o, unsigned bits) -> double {
+      if (!((used >> q) & 1u)) return t;
+      const int up = (face && !(bits & 1u)) ? o : 0, lo = (face && !(bits & 2u)) ? -o : 0, ee = face ? e : 0;
+      const double s = fma(w[q], (phi[c + up] - phi[c + lo]) + (phi[c + ee + up] - phi[c + ee + lo]), t);
+      return zero_bits(w[q]) ? t : s;
     };
-    if (code & (1u << 12)) {
-      const double wn = pw[c], wa = pw[N + c], wb = pw[2 * N + c];
-      const int e = (i == mx - 2) ? c + 3 - mx : c + 1;
-      double t = wn * (phi[e] - phi[c]);
-      if (wa != 0.) t = fma(wa, pair(c, c + 1, sy, code & 3u), t);
-      if (wb != 0.) t = fma(wb, pair(c, c + 1, sz, (code >> 2) & 3u), t);
-      u.x[c] = fma(-t, sc, u.x[c]);
-    }
-    if (code & (1u << 13)) {
-      const double wn = pw[3 * N + c], wa = pw[4 * N + c], wb = pw[5 * N + c];
-      const int e = (j == my - 2) ? c + (3 - my) * sy : c + sy;
-      double t = wn * (phi[e] - phi[c]);
-      if (wa != 0.) t = fma(wa, pair(c, c + sy, 1, (code >> 4) & 3u), t);
-      if (wb != 0.) t = fma(wb, pair(c, c + sy, sz, (code >> 6) & 3u), t);
-      u.y[c] = fma(-t, sc, u.y[c]);
-    }
-    if (code & (1u << 14)) {
-      const double wn = pw[6 * N + c], wa = pw[7 * N + c], wb = pw[8 * N + c];
-      const int e = (k == mz - 2) ? c + (3 - mz) * sz : c + sz;
-      double t = wn * (phi[e] - phi[c]);
-      if (wa != 0.) t = fma(wa, pair(c, c + sz, 1, (code >> 8) & 3u), t);
-      if (wb != 0.) t = fma(wb, pair(c, c + sz, sy, (code >> 10) & 3u), t);
-      u.z[c] = fma(-t, sc, u.z[c]);
-    }
+    const unsigned fi = code & (1u << 12), fj = code & (1u << 13), fk = code & (1u << 14);
+    double tx = w[0] * (pe - pc0), ty = w[3] * (pn - pc0), tz = w[6] * (pt - pc0);
+    tx = cross(1, tx, fi, 1, sy, code);
+    tx = cross(2, tx, fi, 1, sz, code >> 2);
+    ty = cross(4, ty, fj, sy, 1, code >> 4);
+    ty = cross(5, ty, fj, sy, sz, code >> 6);
+    tz = cross(7, tz, fk, sz, 1, code >> 8);
+    tz = cross(8, tz, fk, sz, sy, code >> 10);
+    if (fi) u.x[c] = fma(-tx, sc, ux);
+    if (fj) u.y[c] = fma(-ty, sc, uy);
+    if (fk) u.z[c] = fma(-tz, sc, uz);
   }
 }
 
-int launch_projection_fast(const Dims& d, const double* pw, const uint16_t* pc, const double* phi, double dt, double st,
+int launch_projection_fast(const Dims& d, unsigned used, const double* pw, const uint16_t* pc, const double* phi, double dt, double st,
                            double coeff, const Ucont& u, cudaStream_t s, int k0, int k1) {
   const size_t P = (size_t)d.mx * d.my;
   if (k1 < 0) k1 = d.mz;
@@ -717,7 +731,7 @@ int launch_projection_fast(const Dims& d, const double* pw, const uint16_t* pc, 
   if (p0 < p1) {
     const size_t c0 = p0 * P, c1 = p1 * P;
     const double sc = dt * st / coeff;
-    k_projection_fast<<<nblk(c1 - c0, 128), 128, 0, s>>>(d, c0, c1, pw, pc, phi, sc, u);
+    k_projection_fast<<<(unsigned)((c1 - c0 + 127) / 128), 128, 0, s>>>(d, c0, c1, used, pw, pc, phi, sc, u);
     ++g_launches;
   }
   return launch_ucont_ghosts(d, u, k0, k1, s);

@@ -159,6 +159,7 @@ struct Grid {
   Level lev[MAXLEV];
   double* pd = nullptr;
   double* pw = nullptr;     // projection face weights (9, see launch_proj_weights)
+  unsigned pw_used = 0x1FF;  // bit q: some weight pw[q] is not zero
   uint16_t* pc = nullptr;   // projection cross-term codes
   double* minv = nullptr;   // per-cell inverse metric / 2 (9, row-major), Contra2Cart
   uint8_t* nb8 = nullptr;   // nvert as bytes when all are integers in [0, 127], else null
@@ -2225,7 +2226,7 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   CK(cudaSetDevice(ctx->device));
   const size_t N = ncell(g.d);
   // scratch on the grid's own stream: the g tensor in the metric formation's
-  // buffer (9 N), the slot mask, range flag and region count among the scalars
+  // buffer (9 N), the slot mask, range flag, nonzero weights and region count among the scalars
   double* gt = g.mtmp;
   unsigned* dmask = (unsigned*)(g.scal + 32);
   int* dregions = (int*)(g.scal + 34);
@@ -2249,9 +2250,10 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
                                  g.lev[l - 1].mcoef, g.lev[l].rwh, g.s);
   Level& F = g.lev[g.L - 1];
   launch_proj_dots(F.d, F.M, g.pd, g.s);
-  launch_proj_weights(F.d, g.pd, F.M, F.nvert, g.pw, g.pc, g.s);
+  launch_proj_weights(F.d, g.pd, F.M, F.nvert, g.pw, g.pc, dmask + 2, g.s);
   unsigned range = 0;
   CK(cudaMemcpyAsync(&range, dmask + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
+  CK(cudaMemcpyAsync(&g.pw_used, dmask + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
   CK(cudaStreamSynchronize(g.s));
   g.half_ok = range == 0;
   // connected fluid regions of the finest level: one null vector each.  They
@@ -2470,7 +2472,7 @@ int vfs_projection_faces(vfs_ctx* ctx, int grid, double dt, double st, double co
   Grid& g = *gp;
   if (!g.lhs) return fail(ctx, VFS_ERR_STATE, "vfs_poisson_lhs must run before the projection");
   Level& F = g.lev[g.L - 1];
-  launch_projection_fast(F.d, g.pw, g.pc, g.phi, dt, st, coeff, g.U(), g.s);
+  launch_projection_fast(F.d, g.pw_used, g.pw, g.pc, g.phi, dt, st, coeff, g.U(), g.s);
   launch_contra2cart(F.d, g.minv, F.nvert, g.U(), g.ucat, g.s);
   CK(cudaStreamSynchronize(g.s));
   return VFS_OK;
@@ -2564,13 +2566,14 @@ int step_post(Grid& g, double dt, double st, double coeff, bool exact, double* u
     dbg("update_pressure", 0, launch_update_pressure(F.d, F.nvert, g.phi, g.p, g.s), g.s);
   }
   // projection: the 9 metric products, 3 face Jacobians, nvert bytes (or
-  // doubles) and phi read, U read and written; on face weights: the 9
-  // weights, the code and phi read, U read and written
-  const double proj_b = exact ? 9 * 8.0 + 24.0 + (g.nb8 ? 1.0 : 8.0) + 8.0 + 48.0 : 9 * 8.0 + 2.0 + 8.0 + 48.0;
+  // doubles) and phi read, U read and written; on face weights: the
+  // weight arrays in use, the code and phi read, U read and written
+  const double proj_b = exact ? 9 * 8.0 + 24.0 + (g.nb8 ? 1.0 : 8.0) + 8.0 + 48.0
+                              : popcount(g.pw_used) * 8.0 + 2.0 + 8.0 + 48.0;
   const char* proj_name = exact ? "k_projection" : "k_projection_fast";
   auto project = [&](int k0, int k1) {
     return exact ? launch_projection(F.d, g.pd, F.M, F.nvert, g.nb8, g.phi, dt, st, coeff, g.U(), g.s, k0, k1)
-                 : launch_projection_fast(F.d, g.pw, g.pc, g.phi, dt, st, coeff, g.U(), g.s, k0, k1);
+                 : launch_projection_fast(F.d, g.pw_used, g.pw, g.pc, g.phi, dt, st, coeff, g.U(), g.s, k0, k1);
   };
   if (p_out) {
     ok(cudaEventRecord(g.ev_p, g.s));
