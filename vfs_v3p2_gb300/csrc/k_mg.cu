@@ -317,23 +317,30 @@ int launch_smooth(const OpView<T>& A, const T* lf, const T* xi, const T* b, T* x
 // forms a_j/m_j and c'_j = c_j/m_j from its own coefficients, so that the
 // forward substitution is y_j = r_j/m_j - (a_j/m_j) y_{j-1} and the backward
 // one delta_j = y_j - c'_j delta_{j+1}.  Non-fluid cells are identity rows;
-// j-periodic seam couplings stay off the line.
+// j-periodic seam couplings stay off the line.  The FP64 factors eliminate
+// from both ends to the middle row: above it m_j = b_j - c_j
+// a'_{j+1} with a'_j = a_j / m_j, and the middle row has both terms.
 template <typename T>
 __global__ void k_line_factors(Dims d, const double* __restrict__ mcoef, T* __restrict__ lf) {
   const size_t N = ncell(d);
   const int ni = d.mx - 2, nk = d.mz - 2;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ni * nk; t += gridDim.x * blockDim.x) {
     const int i = 1 + t % ni, k = 1 + t / ni;
-    double cprev = 0.;
-    for (int j = 1; j < d.my - 1; j++) {
+    const int jm = sizeof(T) == 8 ? 1 + line_mid(d.my - 2) : d.my - 2;  // the rows above jm are eliminated upwards
+    double cprev = 0., aprev = 0.;
+    for (int q = 1; q < d.my - 1; q++) {
+      const int j = q < jm ? q : d.my - 2 - (q - jm);  // 1 .. jm - 1, my - 2 .. jm + 1, jm
       const size_t c = cidx(d, i, j, k);
       double a = (j > 1) ? mcoef[(size_t)SP * N + c] : 0.;
       double bb = mcoef[c];
       double cc = (j < d.my - 2) ? mcoef[(size_t)NP * N + c] : 0.;
       if (bb == 0.) { a = 0.; bb = 1.; cc = 0.; }
-      const double m = bb - a * cprev;
+      double m = bb;
+      if (j <= jm) m -= a * cprev;
+      if (j >= jm) m -= cc * aprev;
       const double inv = 1. / m;
-      cprev = cc * inv;
+      if (j < jm) cprev = cc * inv;
+      else aprev = a * inv;
       lf[c] = (T)inv;
     }
   }

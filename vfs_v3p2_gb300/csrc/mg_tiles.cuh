@@ -744,6 +744,62 @@ __device__ __forceinline__ void face_phase1_all(const OpView<float>& A, const fl
 // ZG: the zero-initial-guess sweep (xi == nullptr), its own instantiation so
 // that its phase 1 (four cells a batch) leaves the others' registers alone.
 
+// FP64 lines are solved from both ends towards the middle row line_mid and
+// back (their factors eliminate rows below it downwards and rows above it
+// upwards, see k_line_factors): two threads a column, so the serial chain is
+// half as long and a 16-column tile fills a warp (the FP64 pipe takes a
+// warp's 16 cycles whatever its live lanes).
+__host__ __device__ __forceinline__ int line_mid(int nj) { return nj / 2; }
+// Recurrence y = r - f y over n rows st apart, in place in r.
+__device__ __forceinline__ double line_pass(double* r, const double* f, int st, int n, double y) {
+  constexpr int B = 4;
+  for (; n >= B; n -= B) {
+    double a[B], v[B];
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      a[u] = f[u * st];
+      v[u] = r[u * st];
+    }
+#pragma unroll
+    for (int u = 0; u < B; u++) {
+      y = fma(-a[u], y, v[u]);
+      r[u * st] = y;
+    }
+    r += B * st;
+    f += B * st;
+  }
+  for (; n > 0; n--) {
+    y = fma(-*f, y, *r);
+    *r = y;
+    r += st;
+    f += st;
+  }
+  return y;
+}
+// All threads of the block call it; the two ends meet through sp's first and
+// sl's last row, which the way back does not read.
+__device__ __forceinline__ void line_solve_ends(double* su, double* sp, double* sl, int nj, int TW, int sh) {
+  const int il = threadIdx.x & (TW - 1), up = threadIdx.x >> sh, M = line_mid(nj);
+  const int n = up ? nj - 1 - M : M, o = up ? (nj - 1) * TW + il : il, st = up ? -TW : TW, m = M * TW + il;
+  double r = 0., a = 0., c = 0.;
+  if (up < 2) {
+    r = su[m];
+    a = sp[m];
+    c = sl[m];
+    double* const meet = (up ? sl : sp) + o;
+    const double y = line_pass(su + o, (up ? sl : sp) + o, st, n, 0.);
+    if (n > 0) *meet = y;
+  }
+  __syncthreads();
+  if (up < 2) {
+    const double lo = M > 0 ? sp[il] : 0., hi = M < nj - 1 ? sl[(nj - 1) * TW + il] : 0.;
+    const double x = fma(-c, hi, fma(-a, lo, r));
+    if (up == 0) su[m] = x;
+    const int q = m - st;  // outwards from the middle
+    line_pass(su + q, (up ? sp : sl) + q, -st, n, x);
+  }
+}
+
 // One tile of the sweep: columns i0 = 1 + bx TW .. of plane k = 1 + by,
 // staged in smraw (3 TW nj values of T).
 template <unsigned MASK, typename T, typename TC, bool PAIR, int UU, bool ZG>
@@ -963,7 +1019,9 @@ __device__ __forceinline__ void smooth_tile(const OpView<T>& A, const T* __restr
   __syncthreads();
   // a pitch known at compile time: one warp's issue is the solve's time, and a
   // run-time pitch takes three integer products a row
-  if (threadIdx.x < TW) {
+  if constexpr (sizeof(T) == 8) {
+    line_solve_ends(su, sp, sl, nj, TW, sh);
+  } else if (threadIdx.x < TW) {
     if (TW == 32) line_solve<T>(su, sp, sl, nj, 32, threadIdx.x);
     else if (TW == 16) line_solve<T>(su, sp, sl, nj, 16, threadIdx.x);
     else if (TW == 8) line_solve<T>(su, sp, sl, nj, 8, threadIdx.x);
