@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(256) k_group_gemv(const GroupItem<T>* __restri
   const GroupItem<T>& it = group_item(items, n);
   if (skipped(it.skip)) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  gemv_tile<T>(it.A.d, it.Binv, it.n, it.b, it.y, (const T*)nullptr, blockIdx.x - it.start, (T*)smraw);
+  const int r0 = 8 * (blockIdx.x - it.start);
+  gemv_tile<T>(it.A.d, it.Binv, it.n, it.b, it.y, (const T*)nullptr, r0, min(r0 + 8, it.n), (T*)smraw);
 }
 
 template <typename K>
