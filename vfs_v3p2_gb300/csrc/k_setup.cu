@@ -732,22 +732,20 @@ __global__ void k_prolong_codes(Dims f, Dims c, int si, int sj, int sk, const do
 // ccomp (labels of the level's connected fluid regions) the term is
 // sigma * sum_q e_q e_q^T, one per region, so B stays nonsingular when
 // bodies cut the level apart.  Unknowns
-// are the interior cells packed as ((k-1)*nj + (j-1))*ni + (i-1).  Work
-// matrix W = [B | I], n x 2n, row-major FP64; Gauss-Jordan with partial
-// pivoting, one pivot per launch sequence.
+// are the interior cells packed as ((k-1)*nj + (j-1))*ni + (i-1).  W: n x n,
+// row-major FP64.
 // ---------------------------------------------------------------------------
 __global__ void k_dense_build(Dims d, const double* __restrict__ mcoef, double sigma, double* W, int n,
                               const int* __restrict__ ccomp) {
   const size_t N = ncell(d);
   const int ni = d.mx - 2, nj = d.my - 2;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)n * 2 * n; t += (size_t)gridDim.x * blockDim.x) {
-    int r = (int)(t / (2 * (size_t)n)), col = (int)(t % (2 * (size_t)n));
+  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)n * n; t += (size_t)gridDim.x * blockDim.x) {
+    int r = (int)(t / n), col = (int)(t % n);
     int i = 1 + r % ni, j = 1 + (r / ni) % nj, k = 1 + r / (ni * nj);
     size_t c = cidx(d, i, j, k);
     bool fr = mcoef[c] != 0.;  // CP slot of a fluid row is nonzero
     double v = 0.;
-    if (col >= n) v = (col - n == r) ? 1. : 0.;
-    else {
+    {
       int i2 = 1 + col % ni, j2 = 1 + (col / ni) % nj, k2 = 1 + col / (ni * nj);
       size_t c2 = cidx(d, i2, j2, k2);
       bool fc = mcoef[c2] != 0.;
@@ -767,91 +765,123 @@ __global__ void k_dense_build(Dims d, const double* __restrict__ mcoef, double s
   }
 }
 
-// One block opens elimination step p: pivot search in column p (rows p on; the
-// largest magnitude, the first of equals), rows p and the pivot's swapped, row
-// p scaled by 1 / pivot, and the column's factors saved.  W was written by
-// other blocks of the running launch, so it is read past L1.  In the left half
-// only columns from p on are live (those before are unit vectors by now).
-__device__ void gj_open(double* W, int n, int p, double* fac) {
-  __shared__ double bv[32];
-  __shared__ int bi[32];
-  __shared__ double pinv;
-  const size_t w = 2 * (size_t)n;
-  double best = -1.;
-  int arg = p;
-  for (int r = p + threadIdx.x; r < n; r += blockDim.x) {
-    const double v = fabs(__ldcg(W + (size_t)r * w + p));
-    if (v > best) { best = v; arg = r; }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ov = __shfl_down_sync(0xffffffffu, best, o);
-    const int oa = __shfl_down_sync(0xffffffffu, arg, o);
-    if (ov > best || (ov == best && oa < arg)) { best = ov; arg = oa; }
-  }
-  if ((threadIdx.x & 31) == 0) { bv[threadIdx.x >> 5] = best; bi[threadIdx.x >> 5] = arg; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    for (int q = 1; q < nw; q++)
-      if (bv[q] > bv[0] || (bv[q] == bv[0] && bi[q] < bi[0])) { bv[0] = bv[q]; bi[0] = bi[q]; }
-    pinv = 1. / __ldcg(W + (size_t)bi[0] * w + p);
-  }
-  __syncthreads();
-  const int q = bi[0];
-  const double inv = pinv;
-  for (size_t c = p + threadIdx.x; c < w; c += blockDim.x) {
-    const double x = __ldcg(W + (size_t)p * w + c), y = __ldcg(W + (size_t)q * w + c);
-    if (q != p) __stcg(W + (size_t)q * w + c, x);
-    __stcg(W + (size_t)p * w + c, y * inv);
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) fac[r] = r == p ? 0. : __ldcg(W + (size_t)r * w + p);
+// Gauss-Jordan inversion in place, b columns a step (partial pivoting, rows
+// swapped; the inverse's columns are put back in order at the end).  For the
+// panel of columns p0 .. p0 + b - 1, one block applies the b elimination
+// steps to the panel alone (staged in shared memory, one thread per row):
+// with the row order src it ends as N, whose rows p0 + s hold the inverse of
+// the pivot block and whose other rows hold minus their multipliers.  Every
+// other column is then x'[r] = (r outside the panel's rows ? x[src r] : 0) +
+// sum_t N[r][t] x[src (p0 + t)], a rank-b product over all SMs into the other
+// of two matrices.  Two launches for b columns: at one launch a column the
+// chain of launches bounded it (432 rows: 4.2 ms).
+constexpr int GJ_B = 16;
+// Columns a step: a power of two whose panel fits a block's shared memory.
+static int gj_width(int n) {
+  int b = GJ_B;
+  while (b > 1 && (size_t)b * n * sizeof(double) > 192 * 1024) b >>= 1;
+  return b;
 }
-__global__ void __launch_bounds__(1024) k_gj_open(double* W, int n, double* fac, unsigned* ticket) {
-  if (threadIdx.x == 0) *ticket = 0u;
-  gj_open(W, n, 0, fac);
+// Candidate pivots in order: the larger magnitude, the first of equals.
+__device__ __forceinline__ void gj_better(unsigned long long& v, int& r, unsigned long long ov, int orow) {
+  if (ov > v || (ov == v && orow < r)) { v = ov; r = orow; }
 }
-
-// Step p: every row minus its factor times row p (a block per row, columns
-// where row p is zero left out: half of them on average, the identity columns
-// of rows not yet used); the block that arrives last opens step p + 1.  One
-// launch a step instead of four: what bounds a small level's inverse is the
-// chain of launches (96x48x48, 432 rows: set-up 11.3 -> 6.6 ms with the region
-// count below).
-__global__ void __launch_bounds__(256) k_gj_step(double* W, int n, int p, double* fac, unsigned* ticket) {
-  __shared__ bool last;
-  const int w = 2 * n;
-  const double* __restrict__ Wp = W + (size_t)p * w;
-  for (int r = blockIdx.x; r < n; r += gridDim.x) {
-    const double f = fac[r];
-    if (f == 0.) continue;
-    double* Wr = W + (size_t)r * w;
-    for (int c = p + 1 + threadIdx.x; c < w; c += blockDim.x) {
-      const double b = Wp[c];
-      if (b != 0.) Wr[c] -= f * b;
+__global__ void __launch_bounds__(1024) k_gj_panel(const double* __restrict__ A, int n, int p0, int b, double* __restrict__ Np,
+                                                   int* __restrict__ src, int* __restrict__ perm) {
+  extern __shared__ double P[];  // [b][n]
+  __shared__ double prow[GJ_B];
+  __shared__ unsigned long long cv[32];
+  __shared__ int cr[32], swap_row;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  for (int q = tid; q < n * b; q += blockDim.x) P[(q % b) * n + q / b] = A[(size_t)(q / b) * n + p0 + q % b];
+  for (int r = tid; r < n; r += blockDim.x) src[r] = r;
+  __syncthreads();
+  // the block's candidates for column t among its rows from lo on
+  auto candidates = [&](int t, int lo) {
+    unsigned long long v = 0ull;
+    int row = n;
+    for (int r = tid; r < n; r += blockDim.x)
+      if (r >= lo) gj_better(v, row, abs_bits(P[t * n + r]) + 1ull, r);
+    for (int o = 16; o > 0; o >>= 1)
+      gj_better(v, row, __shfl_down_sync(0xffffffffu, v, o), __shfl_down_sync(0xffffffffu, row, o));
+    if (lane == 0) { cv[warp] = v; cr[warp] = row; }
+  };
+  candidates(0, p0);
+  for (int t = 0; t < b; t++) {
+    const int p = p0 + t;
+    __syncthreads();
+    if (warp == 0) {  // pivot row q: swapped with row p, scaled into prow
+      unsigned long long v = lane < nw ? cv[lane] : 0ull;
+      int q = lane < nw ? cr[lane] : n;
+      for (int o = 16; o > 0; o >>= 1) gj_better(v, q, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, q, o));
+      const double inv = 1. / P[t * n + q];
+      __syncwarp();
+      if (lane < b) {
+        const double x = P[lane * n + p], y = P[lane * n + q];
+        if (q != p) P[lane * n + q] = x;
+        prow[lane] = lane == t ? inv : y * inv;
+      }
+      if (lane == 0) {
+        swap_row = src[p];  // (src is this block's alone)
+        src[p] = src[q];
+        src[q] = q != p ? swap_row : src[p];
+      }
     }
+    __syncthreads();
+    for (int r = tid; r < n; r += blockDim.x) {
+      const double f = P[t * n + r];
+#pragma unroll 4
+      for (int c = 0; c < b; c++)
+        P[c * n + r] = r == p ? prow[c] : fma(-f, prow[c], c == t ? 0. : P[c * n + r]);
+    }
+    // (a thread's candidates are rows it has just written)
+    if (t + 1 < b) candidates(t + 1, p + 1);
   }
-  if (p == n - 1) return;
-  __threadfence();
   __syncthreads();
-  if (threadIdx.x == 0) {
-    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    if (last) *ticket = 0u;
+  for (int q = tid; q < n * b; q += blockDim.x) Np[q] = P[(q % b) * n + q / b];
+  // the rows' original numbers after the swaps; perm is staged in the panel's room
+  int* was = reinterpret_cast<int*>(P);
+  __syncthreads();
+  for (int r = tid; r < n; r += blockDim.x) was[r] = p0 == 0 ? r : perm[r];
+  __syncthreads();
+  for (int r = tid; r < n; r += blockDim.x) perm[r] = was[src[r]];
+}
+// 16 rows x 64 columns a block, four rows of one column a thread.
+__global__ void __launch_bounds__(256) k_gj_update(const double* __restrict__ A, double* __restrict__ out, int n, int p0,
+                                                   int b, const double* __restrict__ Np, const int* __restrict__ src) {
+  const int c = blockIdx.x * 64 + (threadIdx.x & 63), r0 = blockIdx.y * 16 + (threadIdx.x >> 6) * 4;
+  if (c >= n) return;
+  const bool panel = c >= p0 && c < p0 + b;
+  double x[GJ_B], acc[4];
+#pragma unroll
+  for (int t = 0; t < GJ_B; t++) x[t] = t < b && !panel ? A[(size_t)src[p0 + t] * n + c] : 0.;
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const int r = r0 + u;
+    acc[u] = 0.;
+    if (r >= n) continue;
+    if (panel) acc[u] = Np[(size_t)r * b + c - p0];
+    else if (r < p0 || r >= p0 + b) acc[u] = A[(size_t)src[r] * n + c];
   }
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  gj_open(W, n, p + 1, fac);
+#pragma unroll
+  for (int u = 0; u < 4; u++) {
+    const int r = r0 + u;
+    if (r >= n) break;
+#pragma unroll
+    for (int t = 0; t < GJ_B; t++)
+      if (t < b) acc[u] = fma(Np[(size_t)r * b + t], x[t], acc[u]);
+    out[(size_t)r * n + c] = acc[u];
+  }
 }
 
-// Copy the right half of W (the inverse) into Binv (FP64) and Binv32.
-__global__ void k_gj_extract(const double* W, int n, double* B, float* B32) {
-  const size_t w = 2 * (size_t)n;
+// The inverse's columns in order into Binv (FP64) and Binv32.
+__global__ void k_gj_extract(const double* __restrict__ W, int n, const int* __restrict__ perm, double* __restrict__ B,
+                             float* __restrict__ B32) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)n * n; t += (size_t)gridDim.x * blockDim.x) {
-    size_t r = t / n, c = t % n;
-    double v = W[r * w + n + c];
-    B[t] = v;
-    B32[t] = (float)v;
+    const size_t q = t / n * n + perm[t % n];
+    const double v = W[t];
+    B[q] = v;
+    B32[q] = (float)v;
   }
 }
 
@@ -968,20 +998,27 @@ int launch_prolong_codes(const Dims& f, const Dims& c, int si, int sj, int sk, c
   return (int)cudaGetLastError();
 }
 
-// W: dense_inverse_scratch(n) doubles (the augmented matrix, n factors, a ticket).
-size_t dense_inverse_scratch(int n) { return (size_t)n * 2 * n + n + 1; }
+// W: dense_inverse_scratch(n) doubles (two matrices, the panel, two row orders).
+size_t dense_inverse_scratch(int n) { return 2 * (size_t)n * n + (size_t)n * GJ_B + n; }
 int launch_dense_inverse(const Dims& d, const double* mcoef, double sigma, double* W, double* Binv, float* Binv32, int n,
                          cudaStream_t s, const int* ccomp) {
-  const size_t w = 2 * (size_t)n;
-  double* fac = W + (size_t)n * w;
-  unsigned* ticket = (unsigned*)(fac + n);
-  k_dense_build<<<nblk((size_t)n * w), 256, 0, s>>>(d, mcoef, sigma, W, n, ccomp); ++g_launches;
-  k_gj_open<<<1, 1024, 0, s>>>(W, n, fac, ticket); ++g_launches;
-  const int nb = n < 152 * 8 ? n : 152 * 8;  // (1024 threads a block: 432 rows 4.3 -> 6.8 ms)
-  for (int p = 0; p < n; p++) {
-    k_gj_step<<<nb, 256, 0, s>>>(W, n, p, fac, ticket); ++g_launches;
+  const size_t nn = (size_t)n * n;
+  double *A = W, *out = W + nn, *Np = out + nn;
+  int *src = (int*)(Np + (size_t)n * GJ_B), *perm = src + n;
+  const int b = gj_width(n);
+  const size_t sm = (size_t)b * n * sizeof(double);
+  VFS_CUDA_OK(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sm > 48 * 1024 ? sm : 48 * 1024)));
+  const int nt = n >= 1024 ? 1024 : (n + 31) / 32 * 32;
+  k_dense_build<<<nblk(nn), 256, 0, s>>>(d, mcoef, sigma, A, n, ccomp); ++g_launches;
+  for (int p0 = 0; p0 < n; p0 += b) {
+    const int w = n - p0 < b ? n - p0 : b;
+    k_gj_panel<<<1, nt, sm, s>>>(A, n, p0, w, Np, src, perm); ++g_launches;
+    k_gj_update<<<dim3((n + 63) / 64, (n + 15) / 16), 256, 0, s>>>(A, out, n, p0, w, Np, src); ++g_launches;
+    double* const t = A;
+    A = out;
+    out = t;
   }
-  k_gj_extract<<<nblk((size_t)n * n), 256, 0, s>>>(W, n, Binv, Binv32); ++g_launches;
+  k_gj_extract<<<nblk(nn), 256, 0, s>>>(A, n, perm, Binv, Binv32); ++g_launches;
   return (int)cudaGetLastError();
 }
 

@@ -2324,17 +2324,19 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
     }
     if (nf > 0) {
       const double sigma = -(sabs / nf) / (double)nf;
-      double* W = nullptr;
-      CK(cudaMalloc(&W, dense_inverse_scratch(n) * sizeof(double)));
+      // scratch: the g tensor's buffer where it is large enough
+      double* own = nullptr;
+      if (dense_inverse_scratch(n) > 9 * N) CK(cudaMalloc(&own, dense_inverse_scratch(n) * sizeof(double)));
+      double* const W = own ? own : gt;
       int r = C.Binv ? VFS_OK : galloc(ctx, g, &C.Binv, (size_t)n * n);
       if (!r && !C.Binv32) r = galloc(ctx, g, &C.Binv32, (size_t)n * n);
       if (r) {
-        cudaFree(W); cudaFree(ccomp);
+        cudaFree(own); cudaFree(ccomp);
         return r;
       }
       launch_dense_inverse(C.d, C.mcoef, sigma, W, C.Binv, C.Binv32, n, g.s, ccomp);
       cudaError_t e = cudaStreamSynchronize(g.s);
-      cudaFree(W); cudaFree(ccomp);
+      cudaFree(own); cudaFree(ccomp);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "coarse inverse");
       C.nco = n;
     }
