@@ -320,6 +320,9 @@ int launch_smooth(const OpView<T>& A, const T* lf, const T* xi, const T* b, T* x
 // j-periodic seam couplings stay off the line.  The FP64 factors eliminate
 // from both ends to the middle row: above it m_j = b_j - c_j
 // a'_{j+1} with a'_j = a_j / m_j, and the middle row has both terms.
+// Rows whose coefficients a thread of the line factors loads together (the
+// recurrence waits for its divisions, not for memory).
+constexpr int LF_U = 8;
 template <typename T>
 __global__ void k_line_factors(Dims d, const double* __restrict__ mcoef, T* __restrict__ lf) {
   const size_t N = ncell(d);
@@ -328,20 +331,31 @@ __global__ void k_line_factors(Dims d, const double* __restrict__ mcoef, T* __re
     const int i = 1 + t % ni, k = 1 + t / ni;
     const int jm = sizeof(T) == 8 ? 1 + line_mid(d.my - 2) : d.my - 2;  // the rows above jm are eliminated upwards
     double cprev = 0., aprev = 0.;
-    for (int q = 1; q < d.my - 1; q++) {
-      const int j = q < jm ? q : d.my - 2 - (q - jm);  // 1 .. jm - 1, my - 2 .. jm + 1, jm
-      const size_t c = cidx(d, i, j, k);
-      double a = (j > 1) ? mcoef[(size_t)SP * N + c] : 0.;
-      double bb = mcoef[c];
-      double cc = (j < d.my - 2) ? mcoef[(size_t)NP * N + c] : 0.;
-      if (bb == 0.) { a = 0.; bb = 1.; cc = 0.; }
-      double m = bb;
-      if (j <= jm) m -= a * cprev;
-      if (j >= jm) m -= cc * aprev;
-      const double inv = 1. / m;
-      if (j < jm) cprev = cc * inv;
-      else aprev = a * inv;
-      lf[c] = (T)inv;
+    const int nj = d.my - 2;
+    auto row = [&](int q) { return q < jm ? q : nj - (q - jm); };  // 1 .. jm - 1, my - 2 .. jm + 1, jm
+    for (int q0 = 1; q0 <= nj; q0 += LF_U) {
+      double av[LF_U], bv[LF_U], cv[LF_U];
+#pragma unroll
+      for (int u = 0; u < LF_U; u++) {
+        const size_t c = cidx(d, i, row(min(q0 + u, nj)), k);
+        av[u] = mcoef[(size_t)SP * N + c];
+        bv[u] = mcoef[c];
+        cv[u] = mcoef[(size_t)NP * N + c];
+      }
+#pragma unroll
+      for (int u = 0; u < LF_U; u++) {
+        if (q0 + u > nj) break;
+        const int j = row(q0 + u);
+        double a = (j > 1) ? av[u] : 0., bb = bv[u], cc = (j < nj) ? cv[u] : 0.;
+        if (bb == 0.) { a = 0.; bb = 1.; cc = 0.; }
+        double m = bb;
+        if (j <= jm) m -= a * cprev;
+        if (j >= jm) m -= cc * aprev;
+        const double inv = 1. / m;
+        if (j < jm) cprev = cc * inv;
+        else aprev = a * inv;
+        lf[cidx(d, i, j, k)] = (T)inv;
+      }
     }
   }
 }
@@ -374,6 +388,7 @@ __global__ void k_half_operator(Dims d, const double* __restrict__ mcoef, __half
     const size_t hc = hidx(d, i, j, k);
     const double D = mcoef[c];
     double delta = 0.;
+#pragma unroll  // (the slots' loads and divisions side by side: 62 us a level of any size one after the other)
     for (int m = 1; m < 19; m++) {
       const double a = D != 0. ? mcoef[(size_t)m * n + c] / D : 0.;
       if (!(fabs(a) <= 6.e4)) atomicOr(range, 1u);
@@ -405,19 +420,36 @@ __global__ void k_line_factors_half(Dims d, const __half* __restrict__ h, const 
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ni * nk; t += gridDim.x * blockDim.x) {
     const int i = 1 + t % ni, k = 1 + t / ni;
     double cprev = 0.;
-    for (int j = 1; j < d.my - 1; j++) {
-      const size_t c = cidx(d, i, j, k), hc = hidx(d, i, j, k);
-      if (mcoef[c] == 0.) {
-        lf[c] = 0.f;
-        cprev = 0.;
-        continue;
+    const int nj = d.my - 2;
+    for (int j0 = 1; j0 <= nj; j0 += LF_U) {
+      double Dv[LF_U];
+      __half av[LF_U], bv[LF_U], cv[LF_U];
+#pragma unroll
+      for (int u = 0; u < LF_U; u++) {
+        const int j = min(j0 + u, nj);
+        const size_t hc = hidx(d, i, j, k);
+        Dv[u] = mcoef[cidx(d, i, j, k)];
+        av[u] = h[(size_t)SP * hs + hc];
+        bv[u] = h[hc];
+        cv[u] = h[(size_t)NP * hs + hc];
       }
-      const double a = (j > 1) ? (double)__half2float(h[(size_t)SP * hs + hc]) : 0.;
-      const double bb = 1. + (double)__half2float(h[hc]);
-      const double cc = (j < d.my - 2) ? (double)__half2float(h[(size_t)NP * hs + hc]) : 0.;
-      const double inv = 1. / (bb - a * cprev);
-      cprev = cc * inv;
-      lf[c] = (float)inv;
+#pragma unroll
+      for (int u = 0; u < LF_U; u++) {
+        const int j = j0 + u;
+        if (j > nj) break;
+        const size_t c = cidx(d, i, j, k);
+        if (Dv[u] == 0.) {
+          lf[c] = 0.f;
+          cprev = 0.;
+          continue;
+        }
+        const double a = (j > 1) ? (double)__half2float(av[u]) : 0.;
+        const double bb = 1. + (double)__half2float(bv[u]);
+        const double cc = (j < nj) ? (double)__half2float(cv[u]) : 0.;
+        const double inv = 1. / (bb - a * cprev);
+        cprev = cc * inv;
+        lf[c] = (float)inv;
+      }
     }
   }
 }

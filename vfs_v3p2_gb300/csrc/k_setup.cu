@@ -684,7 +684,8 @@ __global__ void k_nvert_product(Dims f, Dims c, int si, int sj, int sk, const do
 // nvert in place in k, j, i order.  A cell's test reads its i-1, j-1, k-1
 // neighbours after and its i+1, j+1, k+1 neighbours before their own update,
 // so processing the anti-diagonal planes i + j + k = s in increasing s
-// reproduces the sequential result exactly.  One launch per plane.
+// reproduces the sequential result exactly: by one block on the values as
+// bytes in shared memory where they fit, else one launch per plane.
 __global__ void k_nvert_sandwich(Dims c, int s, double* nc) {
   const int ni = c.mx - 2, nj = c.my - 2;
   // enumerate (i, j) on plane s, k = s - i - j
@@ -697,6 +698,25 @@ __global__ void k_nvert_sandwich(Dims c, int s, double* nc) {
       if (nc[cidx(c, i + 1, j, k)] + nc[cidx(c, i - 1, j, k)] > 1.1 && nc[cidx(c, i, j + 1, k)] + nc[cidx(c, i, j - 1, k)] > 1.1 &&
           nc[cidx(c, i, j, k + 1)] + nc[cidx(c, i, j, k - 1)] > 1.1)
         nc[q] = 1.;
+    }
+  }
+}
+// The values are 0 or 1 and the frame's are 0 (k_nvert_product).
+__global__ void __launch_bounds__(1024) k_nvert_sandwich_block(Dims c, double* nc) {
+  extern __shared__ uint8_t v[];
+  const int n = (int)ncell(c), ni = c.mx - 2, nj = c.my - 2, sy = c.mx, sz = c.mx * c.my;
+  for (int q = threadIdx.x; q < n; q += blockDim.x) v[q] = !zero_bits(nc[q]);
+  const int smax = ni + nj + c.mz - 2;
+  for (int s = 3; s <= smax; s++) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < ni * nj; t += blockDim.x) {
+      const int i = 1 + t % ni, j = 1 + t / ni, k = s - i - j;
+      if (k < 1 || k > c.mz - 2) continue;
+      const int q = k * sz + j * sy + i;
+      if (!v[q] && v[q + 1] && v[q - 1] && v[q + sy] && v[q - sy] && v[q + sz] && v[q - sz]) {
+        v[q] = 1;
+        nc[q] = 1.;
+      }
     }
   }
 }
@@ -888,16 +908,27 @@ __global__ void k_gj_extract(const double* __restrict__ W, int n, const int* __r
 // ---------------------------------------------------------------------------
 // Connected regions of the fluid cells (nvert < 0.1 on the interior) through
 // shared faces, periodic wrap included, counted by union-find: every cell is
-// hooked to its +i, +j and +k fluid neighbours, the root of a region being its
-// smallest cell.  parent: N ints.  Almost every grid is one region, and the
-// count is all that one needs; counted on the host it took 5 ms of a 96x48x48
-// grid's set-up.
+// hooked to its neighbours' region, the root of a region being its smallest
+// cell.  A warp starts each row's runs of fluid cells as one tree each, so that
+// two neighbouring rows are united once for each stretch that their runs share
+// (united cell by cell it took 0.75 ms of a 96x48x48 grid's set-up, counted on
+// the host 5 ms).  parent: N ints.  Almost every grid is one region, and the
+// count is all that one needs.
 // ---------------------------------------------------------------------------
-__global__ void k_region_init(Dims d, const double* __restrict__ nvert, int* parent, int* count) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < ncell(d); t += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(t % d.mx), j = (int)((t / d.mx) % d.my), k = (int)(t / ((size_t)d.mx * d.my));
-    parent[t] = interior(d, i, j, k) && nvert[t] < 0.1 ? (int)t : -1;
-    if (t == 0) *count = 0;
+__global__ void __launch_bounds__(256) k_region_init(Dims d, const double* __restrict__ nvert, int* parent, int* count) {
+  const int lane = threadIdx.x & 31;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
+  for (int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; row < d.my * d.mz; row += (gridDim.x * blockDim.x) >> 5) {
+    const int j = row % d.my, k = row / d.my, o = row * d.mx;
+    int open = -1;  // first cell of the run that reaches the last chunk's end
+    for (int i0 = 0; i0 < d.mx; i0 += 32) {
+      const int i = i0 + lane;
+      const bool fl = i < d.mx && interior(d, i, j, k) && below(nvert[o + i], 0.1);
+      const unsigned m = __ballot_sync(0xffffffffu, fl), gaps = ~m & ((1u << lane) - 1u);
+      const int first = gaps ? i0 + 32 - __clz(gaps) : (open >= 0 ? open : i0);
+      if (i < d.mx) parent[o + i] = fl ? o + first : -1;
+      open = __shfl_sync(0xffffffffu, fl ? first : -1, 31);
+    }
   }
 }
 __device__ __forceinline__ int region_root(volatile int* parent, int a) {
@@ -920,12 +951,13 @@ __global__ void k_region_unite(Dims d, int* parent) {
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < ncell(d); t += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(t % d.mx), j = (int)((t / d.mx) % d.my), k = (int)(t / ((size_t)d.mx * d.my));
     if (!interior(d, i, j, k) || parent[t] < 0) continue;
-    const int in = i == d.mx - 2 ? (d.ip ? 1 : 0) : i + 1, jn = j == d.my - 2 ? (d.jp ? 1 : 0) : j + 1,
-              kn = k == d.mz - 2 ? (d.kp ? 1 : 0) : k + 1;
-    const size_t nb[3] = {cidx(d, in, j, k), cidx(d, i, jn, k), cidx(d, i, j, kn)};
-    const bool ok[3] = {in > 0, jn > 0, kn > 0};
-    for (int q = 0; q < 3; q++)
-      if (ok[q] && parent[nb[q]] >= 0) region_unite(parent, (int)t, (int)nb[q]);
+    const int jn = j == d.my - 2 ? (d.jp ? 1 : 0) : j + 1, kn = k == d.mz - 2 ? (d.kp ? 1 : 0) : k + 1;
+    const size_t nb[2] = {cidx(d, i, jn, k), cidx(d, i, j, kn)};
+    const bool ok[2] = {jn > 0, kn > 0}, run = i > 1 && parent[t - 1] >= 0;
+    for (int q = 0; q < 2; q++)  // (the stretch's first cell unites the two runs)
+      if (ok[q] && parent[nb[q]] >= 0 && !(run && parent[nb[q] - 1] >= 0)) region_unite(parent, (int)t, (int)nb[q]);
+    const size_t seam = t - i + 1;
+    if (d.ip && i == d.mx - 2 && parent[seam] >= 0) region_unite(parent, (int)t, (int)seam);
   }
 }
 __global__ void k_region_count(size_t n, const int* __restrict__ parent, int* count) {
@@ -988,7 +1020,12 @@ int launch_coarsen(const Dims& f, const Dims& c, int si, int sj, int sk, const d
   k_nvert_product<<<nblk(ncell(c)), 256, 0, s>>>(f, c, si, sj, sk, nv_f, nv_c); ++g_launches;
   const int smax = (c.mx - 2) + (c.my - 2) + (c.mz - 2);
   const size_t plane = (size_t)(c.mx - 2) * (c.my - 2);
-  for (int sd = 3; sd <= smax; sd++) k_nvert_sandwich<<<nblk(plane), 256, 0, s>>>(c, sd, nv_c); ++g_launches;
+  if (ncell(c) <= 200 * 1024) {  // (96x48x48 and its levels: 162 launches)
+    VFS_CUDA_OK(cudaFuncSetAttribute(k_nvert_sandwich_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    k_nvert_sandwich_block<<<1, 1024, ncell(c), s>>>(c, nv_c); ++g_launches;
+  } else {
+    for (int sd = 3; sd <= smax; sd++) { k_nvert_sandwich<<<nblk(plane), 256, 0, s>>>(c, sd, nv_c); ++g_launches; }
+  }
   return (int)cudaGetLastError();
 }
 
