@@ -387,10 +387,11 @@ __global__ void k_half_operator(Dims d, const double* __restrict__ mcoef, __half
     const int i = (int)(c % d.mx), j = (int)((c / d.mx) % d.my), k = (int)(c / ((size_t)d.mx * d.my));
     const size_t hc = hidx(d, i, j, k);
     const double D = mcoef[c];
+    const double inv = D != 0. ? 1. / D : 0.;  // (one division, not 18: they bound it)
     double delta = 0.;
-#pragma unroll  // (the slots' loads and divisions side by side: 62 us a level of any size one after the other)
+#pragma unroll
     for (int m = 1; m < 19; m++) {
-      const double a = D != 0. ? mcoef[(size_t)m * n + c] / D : 0.;
+      const double a = mcoef[(size_t)m * n + c] * inv;
       if (!(fabs(a) <= 6.e4)) atomicOr(range, 1u);
       const __half hm = __double2half(a);
       delta = delta + (a - (double)__half2float(hm));
@@ -398,7 +399,7 @@ __global__ void k_half_operator(Dims d, const double* __restrict__ mcoef, __half
     }
     if (!(fabs(delta) <= 6.e4)) atomicOr(range, 1u);
     h[hc] = __double2half(delta);
-    if (dinv) dinv[c] = D != 0. ? (float)(1. / D) : 0.f;
+    if (dinv) dinv[c] = (float)inv;
     if (dval) dval[c] = (float)D;
   }
 }

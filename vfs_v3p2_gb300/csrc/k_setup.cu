@@ -794,8 +794,9 @@ __global__ void k_dense_build(Dims d, const double* __restrict__ mcoef, double s
 // other column is then x'[r] = (r outside the panel's rows ? x[src r] : 0) +
 // sum_t N[r][t] x[src (p0 + t)], a rank-b product over all SMs into the other
 // of two matrices.  Two launches for b columns: at one launch a column the
-// chain of launches bounded it (432 rows: 4.2 ms).
-constexpr int GJ_B = 16;
+// chain of launches bounded it (432 rows, whole set-up: 6.65 ms, by 16 columns
+// 2.92, by 8, whose panel takes half the FP64 operations on its one SM, 2.65).
+constexpr int GJ_B = 8;
 // Columns a step: a power of two whose panel fits a block's shared memory.
 static int gj_width(int n) {
   int b = GJ_B;
