@@ -755,11 +755,11 @@ def main():
     kname = {0: "k_smooth<float, FaceOp>", 1: "k_smooth<float, __half>", 2: "k_smooth<float, float>"}[args.mg_half]
     if args.mg_half == 0 and args.config == "terrain":
         # i-j and j-k cross terms (the hill): the general face form
-        kname = "k_smooth<float, FaceOp, general>"
+        kname = "k_smooth_wg"
     elif args.mg_half == 0:
         # the face form's full-width sweeps run the warp-row kernel (30-column
         # tiles), or with --mg-stage 1 the tensor-copy one
-        kname = "k_smooth_tma" if args.mg_stage else "k_smooth_w<2>"
+        kname = "k_smooth_tma" if args.mg_stage else "k_smooth_w"
     traffic = ncu_traffic(kname + ":" + case.name)
     roof = {"kernel": kname + " (finest-level y-line sweep, x != 0)", "bound": "hbm", "achieved": achieved,
             "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": (achieved / peak) if achieved else None,

@@ -1,11 +1,13 @@
 """Set-up work of vfs_poisson_lhs on the device: the count of connected fluid
 regions (union-find) against a breadth-first search, and the coarsest level's
-dense inverse (Gauss-Jordan, one launch a step)."""
+dense inverse (Gauss-Jordan by column blocks), the coarse masks (sandwich fill
+in one block, or plane by plane on large levels)."""
 from collections import deque
 
 import numpy as np
 import pytest
 
+import oracle as O
 from vfs_v3p2_gb300 import capi, synth
 
 pytestmark = pytest.mark.gpu
@@ -55,11 +57,12 @@ def test_region_count(gpu_ctx, per, share):
         gpu_ctx.grid_destroy(gid)
 
 
-@pytest.mark.parametrize("dims", [(3, 2, 3), (5, 4, 3), (10, 9, 7), (14, 12, 10)])
+@pytest.mark.parametrize("dims", [(3, 2, 3), (5, 4, 3), (10, 9, 7), (14, 12, 10), (16, 14, 15)])
 def test_dense_inverse(gpu_ctx, dims):
     """One level: the preconditioner is the dense solve.  For a right-hand side
     of mean zero against the left null vector it returns A z = v; n eps times a
-    condition number below 1e4 bounds the residual by 1e-8 at n = 1680."""
+    condition number below 1e4 bounds the residual by 1e-8 at n = 3360 (there a
+    block has half the columns)."""
     c = synth.channel_case(*dims, seed=93, levels=1)
     g = c.grid
     gid = gpu_ctx.grid_create(g.coor, g.nvert, 1, 0)
@@ -73,4 +76,26 @@ def test_dense_inverse(gpu_ctx, dims):
         r = gpu_ctx.apply_op(gid, 0, 1, z) - v
         assert np.linalg.norm(r) <= 1e-8 * np.linalg.norm(v)
     finally:
+        gpu_ctx.grid_destroy(gid)
+
+
+@pytest.mark.parametrize("dims,levels", [((16, 24, 16), 3), ((128, 112, 128), 2)])
+def test_coarse_masks(gpu_ctx, dims, levels):
+    """Blocks of solid cells at random, so that many coarse cells lie between
+    solid ones on every axis: the masks are the oracle's."""
+    ni, nj, nk = dims
+    c = synth.channel_case(ni, nj, nk, seed=95, levels=levels)
+    g = c.grid
+    nv = np.zeros(g.nvert.shape)
+    solid = np.random.default_rng(96).random((nk // 2, nj // 2, ni // 2)) < 0.5
+    nv[1:-1, 1:-1, 1:-1] = solid.repeat(2, 0).repeat(2, 1).repeat(2, 2)
+    gid = gpu_ctx.grid_create(g.coor, nv, levels, 1)
+    mg = O.MG(O.dims_of(g), g.coor, nv, levels)
+    try:
+        for l in range(levels - 1):
+            ref = mg.level_array(l, "nvert")
+            assert np.array_equal(gpu_ctx.level_nvert(gid, l).ravel(), ref)
+        assert ref.sum() > solid.sum()  # filled cells
+    finally:
+        mg.close()
         gpu_ctx.grid_destroy(gid)
