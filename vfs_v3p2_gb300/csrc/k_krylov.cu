@@ -209,15 +209,15 @@ __device__ __forceinline__ void dots_finish(KrylovState* st, const double* parts
 
 // NQ consecutive basis columns V0 .. V0 + (NQ-1) n against w: two cells per
 // turn (their loads in flight together), each thread's cells accumulated in
-// increasing order.
-template <int NQ>
-__device__ __forceinline__ void dot_chunk(const double* __restrict__ V0, const double* __restrict__ w, size_t n,
-                                          double* a) {
+// increasing order.  OWN: w's cells were written by this thread (read past the
+// non-coherent path).
+template <int NQ, bool OWN>
+__device__ __forceinline__ void dot_chunk(const double* __restrict__ V0, const double* w, size_t n, double* a) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   for (; t + stride < n; t += 2 * stride) {
     const size_t u = t + stride;
-    const double wv = w[t], wu = w[u];
+    const double wv = OWN ? __ldcg(w + t) : __ldg(w + t), wu = OWN ? __ldcg(w + u) : __ldg(w + u);
     double v[NQ], x[NQ];
 #pragma unroll
     for (int q = 0; q < NQ; q++) {
@@ -228,30 +228,30 @@ __device__ __forceinline__ void dot_chunk(const double* __restrict__ V0, const d
     for (int q = 0; q < NQ; q++) a[q] = fma(x[q], wu, fma(v[q], wv, a[q]));
   }
   if (t < n) {
-    const double wv = w[t];
+    const double wv = OWN ? __ldcg(w + t) : __ldg(w + t);
 #pragma unroll
     for (int q = 0; q < NQ; q++) a[q] = fma(V0[(size_t)q * n + t], wv, a[q]);
   }
 }
 
-__global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* __restrict__ V, int nv,
-                                                 const double* __restrict__ w, size_t n, double* parts, int pass) {
-  if (is_done(st)) return;
-  nv = nv_of(st, nv);
+// The dots of the nv columns and, by the last block, their finish.
+template <bool OWN>
+__device__ __forceinline__ void dots(KrylovState* st, const double* __restrict__ V, int nv, const double* w, size_t n,
+                                     double* parts, int pass) {
   __shared__ double red[KB / 32][MAXCOL + DCH];
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   for (int q0 = 0; q0 < nv; q0 += DCH) {
     double a[DCH] = {0., 0., 0., 0., 0., 0., 0., 0.};
     const double* V0 = V + (size_t)q0 * n;
     switch (min(DCH, nv - q0)) {
-      case 8: dot_chunk<8>(V0, w, n, a); break;
-      case 7: dot_chunk<7>(V0, w, n, a); break;
-      case 6: dot_chunk<6>(V0, w, n, a); break;
-      case 5: dot_chunk<5>(V0, w, n, a); break;
-      case 4: dot_chunk<4>(V0, w, n, a); break;
-      case 3: dot_chunk<3>(V0, w, n, a); break;
-      case 2: dot_chunk<2>(V0, w, n, a); break;
-      default: dot_chunk<1>(V0, w, n, a); break;
+      case 8: dot_chunk<8, OWN>(V0, w, n, a); break;
+      case 7: dot_chunk<7, OWN>(V0, w, n, a); break;
+      case 6: dot_chunk<6, OWN>(V0, w, n, a); break;
+      case 5: dot_chunk<5, OWN>(V0, w, n, a); break;
+      case 4: dot_chunk<4, OWN>(V0, w, n, a); break;
+      case 3: dot_chunk<3, OWN>(V0, w, n, a); break;
+      case 2: dot_chunk<2, OWN>(V0, w, n, a); break;
+      default: dot_chunk<1, OWN>(V0, w, n, a); break;
     }
     const double r = warp_sum8(a, lane);
     if ((lane & 3) == 0) red[wp][q0 + warp_sum8_index(lane)] = r;
@@ -264,13 +264,19 @@ __global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* 
   }
   if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, pass);
 }
+__global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* __restrict__ V, int nv,
+                                                 const double* __restrict__ w, size_t n, double* parts, int pass) {
+  if (is_done(st)) return;
+  dots<false>(st, V, nv_of(st, nv), w, n, parts, pass);
+}
 
 // Blocks of the dots: a warp's reduction of eight columns takes nine FP64 adds
 // whatever its cells, so two blocks per SM until a thread has eight cells
 // (104x40x72, 21 columns: 30.4 us a launch at two cells a thread, 23.6 so).
 static int dots_nblocks(size_t n) {
   const size_t two = (n + KB * 2 - 1) / (KB * 2), eight = (n + KB * 8 - 1) / (KB * 8);
-  const size_t b = eight > 152 * 2 ? eight : (two < 152 * 2 ? two : 152 * 2);
+  const size_t full = eight / 152 * 152;  // no partial wave
+  const size_t b = full > 152 * 2 ? full : (two < 152 * 2 ? two : 152 * 2);
   return (int)(b > 152 * 4 ? 152 * 4 : (b ? b : 1));
 }
 int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
@@ -339,6 +345,43 @@ int launch_arnoldi_finish(KrylovState* st, int nparts, const double* parts, int*
   return (int)cudaGetLastError();
 }
 
+// h of the last dots as factors of the stored columns (in shared memory).
+__device__ __forceinline__ void column_factors(const KrylovState* st, int nv, double* hs) {
+  const double m = column_scale(st).m;
+  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q] / m;
+  __syncthreads();
+}
+// w -= sum_q hs[q] V_q, two cells per turn as in dot_chunk (the same cells a
+// thread); returns the thread's sum of w^2 after the update.
+__device__ __forceinline__ double subtract_columns(const double* __restrict__ V, int nv, double* w, size_t n,
+                                                   const double* hs) {
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  double s = 0.;
+  for (; t + stride < n; t += 2 * stride) {
+    double a0 = w[t], a1 = w[t + stride];
+#pragma unroll 4
+    for (int q = 0; q < nv; q++) {
+      const double h = hs[q];
+      const double v0 = V[(size_t)q * n + t], v1 = V[(size_t)q * n + t + stride];
+      a0 = fma(-h, v0, a0);
+      a1 = fma(-h, v1, a1);
+    }
+    w[t] = a0;
+    w[t + stride] = a1;
+    s = fma(a0, a0, s);
+    s = fma(a1, a1, s);
+  }
+  if (t < n) {
+    double a = w[t];
+#pragma unroll 4
+    for (int q = 0; q < nv; q++) a = fma(-hs[q], V[(size_t)q * n + t], a);
+    w[t] = a;
+    s = fma(a, a, s);
+  }
+  return s;
+}
+
 // w -= sum_q h[q] V_q, with the partials of ||w||^2 after the update; close:
 // the last block closes the Arnoldi column.
 __global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double* __restrict__ V, int nv,
@@ -350,17 +393,8 @@ __global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double*
   nv = nv_of(st, nv);
   __shared__ double sh[32];
   __shared__ double hs[72];
-  const double m = column_scale(st).m;
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) hs[q] = st->h[q] * st->vs[q] / m;
-  __syncthreads();
-  double s = 0.;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    double a = w[t];
-    for (int q = 0; q < nv; q++) a = fma(-hs[q], V[(size_t)q * n + t], a);
-    w[t] = a;
-    s = fma(a, a, s);
-  }
-  s = block_sum(s, sh);
+  column_factors(st, nv, hs);
+  const double s = block_sum(subtract_columns(V, nv, w, n, hs), sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = s;
   if (close && last_block(st->ticket)) arnoldi_close(st, parts, gridDim.x, hst);
 }
@@ -435,65 +469,22 @@ template int launch_cgs_update<float>(KrylovState*, double*, const double*, floa
 template int launch_cgs_update<double>(KrylovState*, double*, const double*, double*, size_t, double*, int, int*,
                                        cudaStream_t, const float*);
 
-// Fused CGS2 middle pass: w <- w - V h (h from the first pass), and the
-// second pass's dots V_q . w computed on the updated element while the basis
-// values are still in registers.  NV = compile-time capacity; the kernel does
-// its work only when NV0 < nv <= NV, so a fixed sequence of launches with
-// increasing capacities serves every column count (graph-replayable) while
-// the FP64 FMAs issued stay within 4 of 2 nv per element.
-template <int NV0, int NV>
-__global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const double* __restrict__ V, int nv,
-                                                       double* __restrict__ w, size_t n, double* parts) {
+// CGS2 middle pass: w <- w - V h (h from the first pass) and the second
+// pass's dots V_q . w.  A thread's dots take the cells that it has updated,
+// in chunks of columns as k_multidot's, the columns from L2 again: one launch
+// for any number of columns (five that held all columns in registers and
+// summed each by a tree of its own took 83 us at 128x64x96, 13 columns).
+__global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const double* __restrict__ V, int nv, double* w,
+                                                       size_t n, double* parts) {
   if (is_done(st)) return;
   nv = nv_of(st, nv);
-  if (nv <= NV0 || nv > NV) return;
-  __shared__ double hs[NV];
-  __shared__ double red[KB / 32][NV];
-  const double m = column_scale(st).m;
-  for (int q = threadIdx.x; q < NV; q += blockDim.x) hs[q] = q < nv ? st->h[q] * st->vs[q] / m : 0.;
-  __syncthreads();
-  double acc[NV];
-#pragma unroll
-  for (int q = 0; q < NV; q++) acc[q] = 0.;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    double v[NV];
-    double a = w[t];
-#pragma unroll
-    for (int q = 0; q < NV; q++) {
-      v[q] = q < nv ? V[(size_t)q * n + t] : 0.;
-      a = fma(-hs[q], v[q], a);
-    }
-    w[t] = a;
-#pragma unroll
-    for (int q = 0; q < NV; q++) acc[q] = fma(v[q], a, acc[q]);
-  }
-  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; q++) {
-    double x = warp_sum(acc[q]);
-    if (lane == 0) red[wp][q] = x;
-  }
-  __syncthreads();
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) {
-    double x = 0.;
-    for (int u = 0; u < KB / 32; u++) x += red[u][q];
-    parts[(size_t)q * gridDim.x + blockIdx.x] = x;
-  }
-  if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, 2);
+  __shared__ double hs[72];
+  column_factors(st, nv, hs);
+  subtract_columns(V, nv, w, n, hs);
+  dots<true>(st, V, nv, w, n, parts, 2);
 }
-
-// nv < 0: device column count, capacity chosen from cap (>= the largest nv).
-int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s,
-                          int cap) {
-  const int nb = krylov_nblocks(n);
-  if (nv > 32 || (nv < 0 && cap > 32)) return -1;
-  // nv >= 0: the one bucket holding nv; nv < 0: every bucket up to cap
-  const int lo = nv < 0 ? 0 : nv, hi = nv < 0 ? cap : nv;
-  if (lo <= 4) { k_gs_update_dots<0, 4><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
-  if (lo <= 8 && hi > 4) { k_gs_update_dots<4, 8><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
-  if (lo <= 16 && hi > 8) { k_gs_update_dots<8, 16><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
-  if (lo <= 24 && hi > 16) { k_gs_update_dots<16, 24><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
-  if (hi > 24) { k_gs_update_dots<24, 32><<<nb, KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches; }
+int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s) {
+  k_gs_update_dots<<<dots_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches;
   return (int)cudaGetLastError();
 }
 

@@ -902,12 +902,7 @@ void issue_krylov(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv) {
   }
   {
     Probed pr(VFS_PROBE_ALL, s, "k_gs_update_dots", g.L - 1, Nd * (nvb + 2.0) * 8.0);
-    if (g.m + 1 <= 32) {
-      dbg("gs_update_dots", 0, launch_gs_update_dots(g.st, g.V, -1, g.w, N, g.parts, s, g.m + 1), s);
-    } else {
-      launch_gs_update(g.st, g.V, -1, g.w, N, g.parts, 0, nullptr, s);
-      launch_multidot(g.st, g.V, -1, g.w, N, g.parts, 2, s);
-    }
+    dbg("gs_update_dots", 0, launch_gs_update_dots(g.st, g.V, -1, g.w, N, g.parts, s), s);
   }
   {
     Probed pr(VFS_PROBE_ALL, s, "k_gs_update", g.L - 1, Nd * (nvb + 2.0) * 8.0);
@@ -920,11 +915,9 @@ void issue_krylov(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv) {
   }
 }
 
-// The CGS2 sequence is graph-replayable up to 32 basis columns (the fused
-// middle pass's largest capacity); the one-pass sequence for any restart.
-bool graphs_allowed(const Grid& g, const vfs_solve_params& p) {
-  return g_probe.kind == 0 && !g_debug && (p.orth == VFS_ORTH_CGS || g.m + 1 <= 32);
-}
+// Every launch of an iteration takes its column count from the device state,
+// so the sequence is graph-replayable for any restart.
+bool graphs_allowed() { return g_probe.kind == 0 && !g_debug; }
 
 // The per-grid iteration graph (captured on first use; re-captured when the
 // solve parameters change).
@@ -1025,7 +1018,7 @@ int fg_after(vfs_ctx* ctx, Fgmres& f, cudaStream_t s) {
 template <typename T>
 int fg_step(vfs_ctx* ctx, Fgmres& f) {
   Grid& g = *f.g;
-  if (graphs_allowed(g, *f.p)) {
+  if (graphs_allowed()) {
     cudaGraphExec_t ex = nullptr;
     int r = iteration_graph<T>(ctx, g, *f.p, &ex);
     if (r) return r;

@@ -132,9 +132,8 @@ int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t
                      cudaStream_t s);
 // In the Krylov kernels nv < 0 (and vn == nullptr) mean "take the column
 // count from the device state", so one iteration is a fixed launch sequence.
-// second CGS pass fused with the first update (capacity <= 32); returns -1 beyond
-int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s,
-                          int cap = 32);
+// second CGS pass fused with the first update
+int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s);
 template <typename T>
 int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, int close, int* hst,
                       cudaStream_t s, const float* dinv = nullptr);
