@@ -207,30 +207,38 @@ __device__ __forceinline__ void dots_finish(KrylovState* st, const double* parts
   }
 }
 
-// NQ consecutive basis columns V0 .. V0 + (NQ-1) n against w: two cells per
-// turn (their loads in flight together), each thread's cells accumulated in
-// increasing order.  OWN: w's cells were written by this thread (read past the
-// non-coherent path).
+// NQ consecutive basis columns V0 .. V0 + (NQ-1) n against w, each thread's
+// cells accumulated in increasing order, the next cell's loads issued before
+// a cell's products: the SM's warps run in step, so without that the loads
+// and the FP64 pipe take turns (256x128x128, 5 columns: 66 -> 59 us; 128x64x96,
+// 7: 37 -> 27; the update, whose chains need two cells a turn, measured slower
+// so, 72 -> 78).  OWN: w's cells were written by this thread
+// (read past the non-coherent path).
 template <int NQ, bool OWN>
 __device__ __forceinline__ void dot_chunk(const double* __restrict__ V0, const double* w, size_t n, double* a) {
   const size_t stride = (size_t)gridDim.x * blockDim.x;
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-  for (; t + stride < n; t += 2 * stride) {
-    const size_t u = t + stride;
-    const double wv = OWN ? __ldcg(w + t) : __ldg(w + t), wu = OWN ? __ldcg(w + u) : __ldg(w + u);
-    double v[NQ], x[NQ];
+  double v[2][NQ], wv[2];
+  auto load = [&](int b, size_t c) {
+    wv[b] = OWN ? __ldcg(w + c) : __ldg(w + c);
 #pragma unroll
-    for (int q = 0; q < NQ; q++) {
-      v[q] = V0[(size_t)q * n + t];
-      x[q] = V0[(size_t)q * n + u];
-    }
+    for (int q = 0; q < NQ; q++) v[b][q] = __ldg(V0 + (size_t)q * n + c);
+  };
+  auto add = [&](int b) {
 #pragma unroll
-    for (int q = 0; q < NQ; q++) a[q] = fma(x[q], wu, fma(v[q], wv, a[q]));
-  }
-  if (t < n) {
-    const double wv = OWN ? __ldcg(w + t) : __ldg(w + t);
-#pragma unroll
-    for (int q = 0; q < NQ; q++) a[q] = fma(V0[(size_t)q * n + t], wv, a[q]);
+    for (int q = 0; q < NQ; q++) a[q] = fma(v[b][q], wv[b], a[q]);
+  };
+  if (t >= n) return;
+  load(0, t);
+  for (;;) {
+    t += stride;
+    if (t >= n) { add(0); return; }
+    load(1, t);
+    add(0);
+    t += stride;
+    if (t >= n) { add(1); return; }
+    load(0, t);
+    add(1);
   }
 }
 
