@@ -803,9 +803,14 @@ static int gj_width(int n) {
   while (b > 1 && (size_t)b * n * sizeof(double) > 192 * 1024) b >>= 1;
   return b;
 }
-// Candidate pivots in order: the larger magnitude, the first of equals.
-__device__ __forceinline__ void gj_better(unsigned long long& v, int& r, unsigned long long ov, int orow) {
-  if (ov > v || (ov == v && orow < r)) { v = ov; r = orow; }
+// The warp's best pivot candidate (magnitude bits v of row r) in every lane:
+// the larger magnitude, the first row of equals.
+__device__ __forceinline__ void gj_best(unsigned long long& v, int& r) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+  const unsigned mh = __reduce_max_sync(FULL, hi), ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+  r = __reduce_min_sync(FULL, hi == mh && lo == ml ? r : 0x7fffffff);
+  v = (unsigned long long)mh << 32 | ml;
 }
 __global__ void __launch_bounds__(1024) k_gj_panel(const double* __restrict__ A, int n, int p0, int b, double* __restrict__ Np,
                                                    int* __restrict__ src, int* __restrict__ perm) {
@@ -822,9 +827,11 @@ __global__ void __launch_bounds__(1024) k_gj_panel(const double* __restrict__ A,
     unsigned long long v = 0ull;
     int row = n;
     for (int r = tid; r < n; r += blockDim.x)
-      if (r >= lo) gj_better(v, row, abs_bits(P[t * n + r]) + 1ull, r);
-    for (int o = 16; o > 0; o >>= 1)
-      gj_better(v, row, __shfl_down_sync(0xffffffffu, v, o), __shfl_down_sync(0xffffffffu, row, o));
+      if (r >= lo) {
+        const unsigned long long a = abs_bits(P[t * n + r]) + 1ull;
+        if (a > v) { v = a; row = r; }
+      }
+    gj_best(v, row);
     if (lane == 0) { cv[warp] = v; cr[warp] = row; }
   };
   candidates(0, p0);
@@ -834,7 +841,7 @@ __global__ void __launch_bounds__(1024) k_gj_panel(const double* __restrict__ A,
     if (warp == 0) {  // pivot row q: swapped with row p, scaled into prow
       unsigned long long v = lane < nw ? cv[lane] : 0ull;
       int q = lane < nw ? cr[lane] : n;
-      for (int o = 16; o > 0; o >>= 1) gj_better(v, q, __shfl_xor_sync(0xffffffffu, v, o), __shfl_xor_sync(0xffffffffu, q, o));
+      gj_best(v, q);
       const double inv = 1. / P[t * n + q];
       __syncwarp();
       if (lane < b) {
