@@ -111,7 +111,7 @@ WORKLOAD = {
     "sphere": "channel 256x128x128 + sphere r=0.3 at (pi,0,pi/2), Poiseuille + N(0,0.1^2)",
     "terrain": "terrain 512x256x256 over a Gaussian hill, log-law + N(0,0.05^2)",
     "batch": "64 independent channel grids, extents log-uniform 32^3..192x96x96, skew U[0,0.1], beta U[1.5,3], "
-             "0-3 spheres r U[0.1,0.3], U ~ N(0,1); one graph launch per FGMRES iteration for all 64",
+             "0-3 spheres r U[0.1,0.3], U ~ N(0,1); one batch call, each grid's iteration graph on its own stream",
     "serve": "Poisson arrivals from 16 streams, extents log-uniform 32^3..256x128x128, U* = previous + N(0,0.01^2), "
              "warm start from the resident phi, HBM admission budget 120 GB",
 }
@@ -411,8 +411,8 @@ def run_batch(args, dist, local, ws):
             "value": value, "unit": "solves/s", "steps": args.steps,
             "ms_per_step": 1e3 * total / args.steps, **base_line(args, ws),
             "config": {"workload": WORKLOAD["batch"], "grids": len(ids), "cells_total": int(cells),
-                       "measures": "batched pressure projection steps/s (64 uneven grids, one graph launch per "
-                                   "FGMRES iteration), mixed FP32-MG/FP64-FGMRES",
+                       "measures": "batched pressure projection steps/s (64 uneven grids, one batch call), "
+                                   "mixed FP32-MG/FP64-FGMRES",
                        "rtol": args.rtol, "div_tol": args.div_tol, "autotuned": not args.no_tune,
                        "autotune_s": tune_s, "mg_grouped": args.mg_grouped,
                        "mg_operator": OPERATOR[base.mg_half],

@@ -141,9 +141,9 @@ typedef struct {
                          launches, operation i of each grid's V-cycle in one
                          launch per kernel with a table of one item per grid,
                          bit for bit the per-grid launches' results.  0 (the
-                         default): each grid's own launches, each grid a branch
-                         of the tick's graph, which measured faster on GB300
-                         (64-grid batch: 877 against 754 solves/s).  Single
+                         default): each grid's own launches and graph, which
+                         measured faster on GB300 (64-grid batch: 877 against
+                         754 solves/s with each grid a branch of one graph).  Single
                          solves and served requests ignore it. */
   int mg_stage;       /* How the finest level's sweeps on the FP32 face form
                          (levels of at least 2^20 interior cells) stage their
@@ -407,11 +407,12 @@ int vfs_inflight(vfs_ctx* ctx);
 /* Device memory the context holds and its budget (0 = none), in bytes. */
 int vfs_memory(vfs_ctx* ctx, unsigned long long* used, unsigned long long* budget);
 
-/* ---- batched solves (many uneven grids, one graph launch per iteration) ---- */
+/* ---- batched solves (many uneven grids at once) ---- */
 /* Runs vfs_projection_step (resident U*, pressure and fluxes stay resident)
- * on n distinct grids.  Every FGMRES iteration of all grids is one CUDA graph
- * launch (one branch per grid, running concurrently; converged grids skip
- * their kernels).  p points to n_params = 1 (shared) or n (per grid) solve
+ * on n distinct grids.  The grids' FGMRES iterations run concurrently, each
+ * grid's a CUDA graph of its own on its stream; with mg_grouped = 1 the
+ * iterations of all grids are one graph launch (converged grids skip their
+ * kernels).  p points to n_params = 1 (shared) or n (per grid) solve
  * parameter sets; infos and divmax (may be NULL) receive n entries. */
 int vfs_projection_step_batch(vfs_ctx* ctx, int n, const int* grids, double dt, double st, double coeff,
                               const vfs_solve_params* p, int n_params, vfs_solve_info* infos, double* divmax);
