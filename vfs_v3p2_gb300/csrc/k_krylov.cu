@@ -8,10 +8,10 @@
 // from the reduction; the matrix-vector product and the solution update
 // apply vs.  With CGS2 (classical with one re-orthogonalisation pass) the
 // columns are stored normalised (vs = 1).  Every pass is a deterministic
-// multi-dot or norm (fixed block partials summed in index order by one
-// block) or one fused update sweep.  The Hessenberg column, Givens rotations and the
-// residual estimate live in a KrylovState in device memory and are updated
-// by a single-block kernel, so the host enqueues iterations without reading
+// multi-dot or norm (fixed block partials summed in index order by the block
+// that arrives last) or one fused update sweep.  The Hessenberg column, Givens rotations and the
+// residual estimate live in a KrylovState in device memory and are updated by
+// the last block of the sweep before them, so the host enqueues iterations without reading
 // anything back; every kernel returns immediately once st->done is set.
 #include "vfs_common.cuh"
 #include "vfs_proj.h"
@@ -21,10 +21,9 @@ namespace vfs {
 constexpr int KB = 256;
 constexpr int MAXCOL = 64;  // largest restart length
 
-// Blocks of the reductions and update sweeps: two cells per thread (one turn of
-// the dots' loop, every load of a thread in flight at once) until the grid
-// fills four blocks per SM.  A 104x40x72 grid (327 k cells) at 20 columns:
-// four cells per thread left half the SMs' blocks unused.
+// Blocks of the norms and update sweeps: two cells per thread (one turn of the
+// update's loop) until the grid fills four blocks per SM (four cells a thread:
+// 32^3 9.2 -> 11.5 us an update).
 int krylov_nblocks(size_t n) {
   size_t b = (n + KB * 2 - 1) / (KB * 2);
   if (b > 152 * 4) b = 152 * 4;
