@@ -418,8 +418,12 @@ int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t
 // (close: by the last block, else k_arnoldi_finish).
 // dinv (nullable): 1 / D of the FP16 normalised multigrid operator, applied
 // to the multigrid copy after its rounding to T.
+// Two columns of two cells a step: the loads of one step overlap the FP64
+// products of another warp's, which longer steps queue behind each other
+// (256x128x128 by 8 columns 92 us, 4 73, 2 60, 1 65; 512x256x256 404 -> 324;
+// with the registers left free: capped for five blocks per SM 61 and 351).
 template <typename T>
-__global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, const double* __restrict__ w,
+__global__ void __launch_bounds__(KB, 1) k_cgs_update(KrylovState* st, double* V, const double* __restrict__ w,
                                                    T* __restrict__ out, size_t n, double* parts,
                                                    const float* __restrict__ dinv, int close, int* hst) {
   if (is_done(st)) {
@@ -439,7 +443,7 @@ __global__ void __launch_bounds__(KB) k_cgs_update(KrylovState* st, double* V, c
   size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   for (; t + stride < n; t += 2 * stride) {
     double a0 = w[t], a1 = w[t + stride];
-#pragma unroll 4
+#pragma unroll 2
     for (int q = 0; q < nv; q++) {
       const double h = hs[q];
       const double v0 = V[(size_t)q * n + t], v1 = V[(size_t)q * n + t + stride];
