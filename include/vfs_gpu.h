@@ -261,25 +261,19 @@ int vfs_divergence_max(vfs_ctx* ctx, int grid, double* out);
  * and no grid buffers to lend.
  *
  * What it does: max over interior cells of |div U| * aj, 0 where the cell or
- * a face neighbour has nvert (the same kernels as vfs_divergence_max), for
+ * a face neighbour has nvert (the same arithmetic as vfs_divergence_max), for
  * the ghosted grid mx x my x mz ([mz][my][mx], i fastest), contravariant
  * fluxes as three component arrays ucont_x/_y/_z, aj and nvert,
  * all device pointers on `device`.  The result is written to the device
  * double *out, ordered on `stream` (a cudaStream_t; NULL = legacy default
- * stream); the call does not synchronise.
+ * stream); the call does not synchronise and may be captured.
  *
- * Scratch: the per-block maxima live in a file-scope static device array of
- * 2432 doubles (19 KB) per device.  Nothing in it has to start at zero (every
- * block writes its entry before the final reduction reads it).  Limits:
- * grids of 2^31 cells or more (ghosts included) are rejected with
- * VFS_ERR_ARG; `device` must be the calling thread's current device.
- * Because the scratch is shared, calls whose kernels may overlap (different
- * streams, or threads, on the same device without ordering between them)
- * race and give undefined results: order them.  The first call on a device
- * looks up the scratch address (cudaGetSymbolAddress, with that device
- * current) and should come before any stream capture; the address is kept
- * for the life of the process, so the device must not be reset
- * (cudaDeviceReset) between calls.  Periodic axes: the flags are accepted
+ * Scratch: none.  *out is cleared on the stream and the blocks' maxima meet in
+ * it, so *out holds the result once the call's work on `stream` has ended, and
+ * nothing else before that.  Calls with an *out each share nothing and may
+ * overlap on any streams and threads.  Limits: grids of 2^31 cells or more
+ * (ghosts included) are rejected with VFS_ERR_ARG; `device` must be the
+ * calling thread's current device.  Periodic axes: the flags are accepted
  * but unused; like the reference's Divergence (main.c:1279-1349) the check
  * reads each cell's west, south and back faces at index - 1, so a periodic
  * axis's ghost faces (index 0 = index m - 2) must be filled before the call.

@@ -7,7 +7,6 @@
 // reference's multiplies and adds in the reference's order, so for equal
 // inputs the outputs are bit-identical (reductions excepted, which sum in a
 // fixed tree order instead of the reference's loop order).
-#include <mutex>
 
 #include "vfs_common.cuh"
 #include "vfs_kernels.h"
@@ -915,11 +914,12 @@ __device__ __forceinline__ bool near_body(const Dims& d, const double* __restric
 
 // What bounds it: the FP64 pipe, six operations a cell (the test for bodies and
 // the maximum run on the integer pipe: 256x128x128 83 -> 72 us; a caller's
-// 151x67x93 arrays with doubles for nvert 44.6 -> 28.7 us a call).
-__global__ void __launch_bounds__(RB) k_divergence(Dims d, Ucont u, const double* __restrict__ aj,
-                                                   const double* __restrict__ nvert, double* parts, double* out,
-                                                   unsigned* ticket, const uint8_t* __restrict__ nb8) {
-  __shared__ double sh[32];
+// 151x67x93 arrays with doubles for nvert 44.6 -> 22.5 us a call).
+// The block's maximum as max_abs bits, in every thread.
+__device__ __forceinline__ unsigned long long divergence_bits(const Dims& d, const Ucont& u,
+                                                              const double* __restrict__ aj,
+                                                              const double* __restrict__ nvert,
+                                                              const uint8_t* __restrict__ nb8, double* sh) {
   unsigned long long mxv = 0ull;
   const size_t sy = d.mx, sz = (size_t)d.mx * d.my;
   ROW_LOOP(d) {
@@ -931,7 +931,13 @@ __global__ void __launch_bounds__(RB) k_divergence(Dims d, Ucont u, const double
       if (!near_body(d, nvert, nb8, c)) max_abs(mxv, v);
     }
   }
-  mxv = block_maxbits(mxv, sh);
+  return block_maxbits(mxv, sh);
+}
+__global__ void __launch_bounds__(RB) k_divergence(Dims d, Ucont u, const double* __restrict__ aj,
+                                                   const double* __restrict__ nvert, double* parts, double* out,
+                                                   unsigned* ticket, const uint8_t* __restrict__ nb8) {
+  __shared__ double sh[32];
+  const unsigned long long mxv = divergence_bits(d, u, aj, nvert, nb8, sh);
   if (threadIdx.x == 0) parts[blockIdx.x] = __longlong_as_double((long long)mxv);
   if (!last_block(ticket)) return;
   const double m = finish_max(parts, sh);
@@ -982,56 +988,36 @@ int launch_norm_absmax(const Dims& d, const double* r, const double* nvert, doub
   return (int)cudaGetLastError();
 }
 
-// ---- allocation-free divergence check (static device scratch) ----
-// The block maxima of k_divergence live in this file-scope array instead of
-// a grid's partials buffer.  row_blocks() caps a launch at 152 * 4 blocks, so
-// the array always holds one partial per block; every block writes its
-// partial before the last one reads it, so none of them has to start at zero.
-// The ticket behind them does: it starts there and every launch leaves it
-// there.
-constexpr int STATIC_PARTS = 152 * 16;
-static __device__ __align__(256) double g_static_parts[STATIC_PARTS + 1];
+// ---- allocation-free divergence check ----
+// The blocks' maxima meet in *out itself, cleared on the stream before the
+// launch: the bits of |v| order like the values, and a maximum does not depend
+// on the order of its blocks.  No scratch and no state outlive a call, so calls
+// on different streams or threads (with an *out each) have nothing to share.
+__global__ void __launch_bounds__(RB) k_divergence_into(Dims d, Ucont u, const double* __restrict__ aj,
+                                                        const double* __restrict__ nvert, unsigned long long* out) {
+  __shared__ double sh[32];
+  const unsigned long long mxv = divergence_bits(d, u, aj, nvert, nullptr, sh);
+  if (threadIdx.x == 0) atomicMax(out, mxv);
+}
 
-int divergence_max_static(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
-                          cudaStream_t s, const char** why) {
+int divergence_max_noalloc(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
+                           cudaStream_t s, const char** why) {
   constexpr int MAXDEV = 64;
-  static std::mutex mu;
-  static double* addr[MAXDEV] = {};
   if (device < 0 || device >= MAXDEV) {
     *why = "device index out of range";
     return 1;
   }
   int cur = -1;
   cudaError_t e = cudaGetDevice(&cur);
-  if (e != cudaSuccess) {
-    *why = cudaGetErrorString(e);
-    return 2;
-  }
-  if (cur != device) {
+  if (e == cudaSuccess && cur != device) {
     *why = "the device argument must be the calling thread's current device";
     return 1;
   }
-  double* parts = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(mu);
-    if (!addr[device]) {
-      // once per device, with that device current
-      e = cudaGetSymbolAddress((void**)&addr[device], g_static_parts);
-      if (e != cudaSuccess) {
-        addr[device] = nullptr;
-        *why = cudaGetErrorString(e);
-        return 2;
-      }
-    }
-    parts = addr[device];
+  if (e == cudaSuccess) e = cudaMemsetAsync(out, 0, sizeof(double), s);
+  if (e == cudaSuccess) {
+    k_divergence_into<<<row_blocks(d), RB, 0, s>>>(d, u, aj, nvert, (unsigned long long*)out); ++g_launches;
+    e = cudaGetLastError();
   }
-  const int nb = row_blocks(d);
-  if (nb > STATIC_PARTS) {  // unreachable while row_blocks caps the grid; kept as the stated limit
-    *why = "more block partials than the static scratch holds";
-    return 1;
-  }
-  k_divergence<<<nb, RB, 0, s>>>(d, u, aj, nvert, parts, out, (unsigned*)(parts + STATIC_PARTS), nullptr); ++g_launches;
-  e = cudaGetLastError();
   if (e != cudaSuccess) {
     *why = cudaGetErrorString(e);
     return 2;

@@ -2501,7 +2501,7 @@ int vfs_divergence_max_noalloc(int device, int mx, int my, int mz, int i_periodi
   Dims d{mx, my, mz, i_periodic ? 1 : 0, j_periodic ? 1 : 0, k_periodic ? 1 : 0};
   Ucont u{const_cast<double*>(ucont_x), const_cast<double*>(ucont_y), const_cast<double*>(ucont_z)};
   const char* why = "";
-  const int rc = divergence_max_static(device, d, u, aj, nvert, out, (cudaStream_t)stream, &why);
+  const int rc = divergence_max_noalloc(device, d, u, aj, nvert, out, (cudaStream_t)stream, &why);
   if (rc) return report(rc == 1 ? VFS_ERR_ARG : VFS_ERR_CUDA, why);
   return report(VFS_OK, "");
 }

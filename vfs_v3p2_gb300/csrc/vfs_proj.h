@@ -58,9 +58,9 @@ int launch_ucont_ghosts(const Dims& d, const Ucont& u, int k0, int k1, cudaStrea
 // row-major), from launch_inverse_metric.
 int launch_contra2cart(const Dims& d, const double* minv, const double* nvert, const Ucont& u, double* ucat, cudaStream_t s);
 int launch_inverse_metric(const Dims& d, const double* M, const double* nvert, double* minv, cudaStream_t s);
-// Divergence check with its block partials in a static device array (no
-// allocation); returns 0, 1 (argument) or 2 (CUDA) and sets *why on error.
-int divergence_max_static(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
+// Divergence check that needs no scratch (no allocation, nothing shared between
+// calls); returns 0, 1 (argument) or 2 (CUDA) and sets *why on error.
+int divergence_max_noalloc(int device, const Dims& d, const Ucont& u, const double* aj, const double* nvert, double* out,
                           cudaStream_t s, const char** why);
 // out[0] = ||r||_2 over the array, out[1] = max |r| over the cells the
 // divergence check keeps
