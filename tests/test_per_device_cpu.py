@@ -1,0 +1,22 @@
+"""Kernel attributes are set once per device, not once per process
+(vfs::PerDevice, compiled for the host from the kernels' own header)."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(HERE)
+
+
+def test_once_per_device(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("nvcc not available")
+    exe = str(tmp_path / "per_device_check")
+    subprocess.run([nvcc, "-O2", "-std=c++17", "-I", os.path.join(ROOT, "vfs_v3p2_gb300", "csrc"),
+                    os.path.join(HERE, "native", "per_device_check.cu"), "-o", exe, "-lpthread"], check=True,
+                   capture_output=True)
+    r = subprocess.run([exe], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr

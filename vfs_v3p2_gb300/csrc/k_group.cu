@@ -5,6 +5,7 @@
 // per-grid launches' bit for bit.
 #include "mg_group.h"
 #include "mg_tiles.cuh"
+#include "per_device.h"
 #include "vfs_kernels.h"
 
 namespace vfs {
@@ -65,26 +66,23 @@ __global__ void __launch_bounds__(256) k_group_gemv(const GroupItem<T>* __restri
   gemv_tile<T>(it.A.d, it.Binv, it.n, it.b, it.y, (const T*)nullptr, r0, min(r0 + 8, it.n), (T*)smraw);
 }
 
-template <typename K>
-static void allow_smem(K k) {
-  cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-}
-
 template <typename T>
 int launch_group(int kind, const GroupItem<T>* items, int nitems, int nblocks, size_t smem, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
+  static PerDevice once;
+  const cudaError_t attr = once([] {
+    constexpr int B = 200 * 1024;
+    cudaError_t e = cudaSuccess;
     if constexpr (sizeof(T) == 4) {
-      allow_smem(k_group_smooth<MASK_CH, T, FaceOp, false>);
-      allow_smem(k_group_smooth<MASK_CH, T, FaceOp, true>);
+      e = allow_smem(k_group_smooth<MASK_CH, T, FaceOp, false>, B);
+      if (e == cudaSuccess) e = allow_smem(k_group_smooth<MASK_CH, T, FaceOp, true>, B);
     }
-    allow_smem(k_group_smooth<MASK_CH, T, T, false>);
-    allow_smem(k_group_smooth<MASK_CH, T, T, true>);
-    allow_smem(k_group_smooth<MASK_ALL, T, T, false>);
-    allow_smem(k_group_smooth<MASK_ALL, T, T, true>);
-    allow_smem(k_group_gemv<T>);
-    attr = true;
-  }
+    if (e == cudaSuccess) e = allow_smem(k_group_smooth<MASK_CH, T, T, false>, B);
+    if (e == cudaSuccess) e = allow_smem(k_group_smooth<MASK_CH, T, T, true>, B);
+    if (e == cudaSuccess) e = allow_smem(k_group_smooth<MASK_ALL, T, T, false>, B);
+    if (e == cudaSuccess) e = allow_smem(k_group_smooth<MASK_ALL, T, T, true>, B);
+    return e != cudaSuccess ? e : allow_smem(k_group_gemv<T>, B);
+  });
+  if (attr != cudaSuccess) return (int)attr;
   if (nitems <= 0 || nblocks <= 0) return (int)cudaSuccess;
   const dim3 g(nblocks), b(256);
   switch (kind) {

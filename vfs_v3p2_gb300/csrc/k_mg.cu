@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "mg_tiles.cuh"
+#include "per_device.h"
 #include "mg_stage.h"
 #include "vfs_common.cuh"
 #include "vfs_kernels.h"
@@ -198,15 +199,20 @@ __global__ void __launch_bounds__(VFS_SMOOTH_NT, 2)
   extern __shared__ float sm[];
   smooth_tile_wg<4, XIK>(A, lf, xi, b, xo, omega, blockIdx.x, plane_block(A.flip, blockIdx.y, gridDim.y), sm);
 }
+// The warp-row sweeps may take the lines' shared memory on this device (else
+// the tiles that need no opt-in run).
+static bool smooth_w_ready() {
+  static PerDevice once;
+  const cudaError_t e = once([] {
+    cudaError_t r = allow_smem(k_smooth_w, 100 * 1024);
+    if (r == cudaSuccess) r = allow_smem(k_smooth_wg<false>, 100 * 1024);
+    return r != cudaSuccess ? r : allow_smem(k_smooth_wg<true>, 100 * 1024);
+  });
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess;
+}
 static int smooth_w_launch(const OpView<float>& A, const float* lf, const float* xi, const float* b, float* xo,
                            float omega, cudaStream_t s) {
-  static const cudaError_t attr = [] {
-    const auto large = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(k_smooth_w, large, 100 * 1024);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_smooth_wg<false>, large, 100 * 1024);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(k_smooth_wg<true>, large, 100 * 1024);
-  }();
-  if (attr != cudaSuccess) return (int)attr;
   const dim3 g((A.d.mx - 2 + SMOOTH_W_TW - 1) / SMOOTH_W_TW, A.d.mz - 2);
   const size_t sm = smooth_smem<float>(32, A.d.my - 2);
   if (A.ffc && fits_tr(A.mask)) k_smooth_wg<false><<<g, VFS_SMOOTH_NT, sm, s>>>(A, lf, xi, b, xo, omega);
@@ -216,17 +222,17 @@ static int smooth_w_launch(const OpView<float>& A, const float* lf, const float*
   return (int)cudaGetLastError();
 }
 template <unsigned MASK, typename T, typename TC, bool PAIR, int UU, bool ZG>
-static void smooth_attrs1() {
-  cudaFuncSetAttribute(k_smooth<MASK, T, TC, PAIR, UU, ZG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  if (VFS_SMOOTH_CARVE >= 0)
-    cudaFuncSetAttribute(k_smooth<MASK, T, TC, PAIR, UU, ZG>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         VFS_SMOOTH_CARVE);
+static cudaError_t smooth_attrs1() {
+  const cudaError_t e = allow_smem(k_smooth<MASK, T, TC, PAIR, UU, ZG>, 200 * 1024);
+  if (e != cudaSuccess || VFS_SMOOTH_CARVE < 0) return e;
+  return cudaFuncSetAttribute(k_smooth<MASK, T, TC, PAIR, UU, ZG>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                              VFS_SMOOTH_CARVE);
 }
 template <unsigned MASK, typename T, typename TC, bool PAIR>
-static void smooth_attrs() {
-  smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U, false>();
-  smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U_SMALL, false>();
-  smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U, true>();
+static cudaError_t smooth_attrs() {
+  cudaError_t e = smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U, false>();
+  if (e == cudaSuccess) e = smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U_SMALL, false>();
+  return e != cudaSuccess ? e : smooth_attrs1<MASK, T, TC, PAIR, VFS_SMOOTH_U, true>();
 }
 
 // One launch of the sweep kernel with the per-level choices: U cells per
@@ -259,19 +265,20 @@ int launch_smooth(const OpView<T>& A, const T* lf, const T* xi, const T* b, T* x
         launch_smooth_tma(A, lf, xi, b, xo, omega, smooth_tma_err(), s) == (int)cudaSuccess)
       return (int)cudaSuccess;
   }
-  static bool attr = false;
-  if (!attr) {
-    smooth_attrs<MASK_CH, T, T, false>();
-    smooth_attrs<MASK_ALL, T, T, false>();
+  static PerDevice once;
+  const cudaError_t attr = once([] {
+    cudaError_t e = smooth_attrs<MASK_CH, T, T, false>();
+    if (e == cudaSuccess) e = smooth_attrs<MASK_ALL, T, T, false>();
     if constexpr (sizeof(T) == 4) {
-      smooth_attrs<MASK_CH, T, __half, false>();
-      smooth_attrs<MASK_CH, T, __half, true>();
-      smooth_attrs<MASK_ALL, T, __half, true>();
-      smooth_attrs<MASK_CH, T, FaceOp, false>();
-      smooth_attrs<MASK_ALL, T, FaceOp, false>();
+      if (e == cudaSuccess) e = smooth_attrs<MASK_CH, T, __half, false>();
+      if (e == cudaSuccess) e = smooth_attrs<MASK_CH, T, __half, true>();
+      if (e == cudaSuccess) e = smooth_attrs<MASK_ALL, T, __half, true>();
+      if (e == cudaSuccess) e = smooth_attrs<MASK_CH, T, FaceOp, false>();
+      if (e == cudaSuccess) e = smooth_attrs<MASK_ALL, T, FaceOp, false>();
     }
-    attr = true;
-  }
+    return e;
+  });
+  if (attr != cudaSuccess) return (int)attr;
   const int nj = A.d.my - 2, ni = A.d.mx - 2, nk = A.d.mz - 2;
   const int tw = smooth_tw<T>(ni, nj, nk, cols, solo || VFS_SMOOTH_NARROW_SHARED);
   const size_t sm = smooth_smem<T>(tw, nj);
@@ -287,7 +294,7 @@ int launch_smooth(const OpView<T>& A, const T* lf, const T* xi, const T* b, T* x
     // tiles (11-slot form) or two blocks per SM (general form, whose lines of
     // more than 128 rows have narrower tiles otherwise)
     const bool wide = ch ? tw == 32 && !small : ni >= SMOOTH_W_TW && (size_t)((ni + 29) / 30) * nk >= 2 * 152;
-    if (A.ffi && (ch || A.ffc) && xi && cols == 0 && wide && smooth_w_fits(A.d, ch)) {
+    if (A.ffi && (ch || A.ffc) && xi && cols == 0 && wide && smooth_w_fits(A.d, ch) && smooth_w_ready()) {
       return smooth_w_launch(A, lf, xi, b, xo, omega, s);
     } else if (A.ffi && ch) {
       smooth_launch<MASK_CH, T, FaceOp, false>(small, g, sm, s, A, lf, xi, b, xo, omega, tw);
@@ -665,11 +672,9 @@ __global__ void __launch_bounds__(1024) k_coarse_gemv(Dims d, const T* __restric
 template <typename T>
 int launch_coarse_gemv(const Dims& d, const T* Binv, int n, const T* b, T* x, const T* dsc, const int* skip,
                        cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_coarse_gemv<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  static PerDevice once;
+  const cudaError_t attr = once([] { return allow_smem(k_coarse_gemv<T>, 200 * 1024); });
+  if (attr != cudaSuccess) return (int)attr;
   const int blocks = (n + 7) / 8 < 152 ? (n + 7) / 8 : 152, rows = (n + blocks - 1) / blocks;
   const int nt = 32 * (rows < 8 ? 8 : (rows > 32 ? 32 : rows));
   k_coarse_gemv<T><<<blocks, nt, (size_t)n * sizeof(T), s>>>(d, Binv, n, b, x, dsc, rows, skip); ++g_launches;

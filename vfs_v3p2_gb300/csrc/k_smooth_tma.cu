@@ -47,6 +47,7 @@
 
 #include "mg_tiles.cuh"
 #include "mg_stage.h"
+#include "per_device.h"
 #include "vfs_kernels.h"
 
 namespace vfs {
@@ -343,15 +344,12 @@ static int g_tma_drop = -1;  // test hook: band whose 1/m copies are left out (-
 
 void smooth_tma_drop(int band) { g_tma_drop = band; }
 
+// the current device's flag
 int* smooth_tma_err() {
-  static int* p = nullptr;
-  if (!p) {
-    if (cudaGetSymbolAddress((void**)&p, g_tma_err) != cudaSuccess) {
-      cudaGetLastError();
-      p = nullptr;
-    }
-  }
-  return p;
+  void* p = nullptr;
+  if (cudaGetSymbolAddress(&p, g_tma_err) == cudaSuccess) return (int*)p;
+  cudaGetLastError();
+  return nullptr;
 }
 
 int smooth_tma_take_error() {
@@ -367,6 +365,7 @@ int smooth_tma_take_error() {
   return v;
 }
 
+constexpr size_t TMA_SMEM_MAX = 220 * 1024;
 static size_t tma_smem(const Dims& d, int stages) {
   return (size_t)stages * TMA_STAGE + (size_t)3 * TMA_TW * (d.my - 2) * 4 + (size_t)2 * stages * 8;
 }
@@ -374,7 +373,7 @@ static size_t tma_smem(const Dims& d, int stages) {
 int smooth_tma_stages(const Dims& d) {
   if (d.mx % 2 || d.my % 2 || d.my - 2 < 2 || !encoder()) return 0;
   for (int s = 4; s >= 2; s--)
-    if (tma_smem(d, s) <= (size_t)220 * 1024) return s;
+    if (tma_smem(d, s) <= TMA_SMEM_MAX) return s;
   return 0;
 }
 
@@ -393,21 +392,15 @@ int launch_smooth_tma(const OpView<float>& A, const float* lf, const float* xi, 
   if (!map4(enc, &m.x, xi, d) || !map4(enc, &m.b, b, d) || !map4(enc, &m.lf, lf, d) || !map4(enc, &m.fj, A.ffj, d) ||
       !map4(enc, &m.aj, A.faj, d) || !map8(enc, &m.fi, A.ffi, d) || !map8(enc, &m.fk, A.ffk, d))
     return (int)cudaErrorInvalidValue;
-  static int nsm = 0;
-  static size_t opted = 0;  // dynamic shared memory the kernel is opted in for
-  if (!nsm) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  int dev = 0, nsm = 0;
+  static PerDevice once;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      once.on(dev, [] { return allow_smem(k_smooth_tma, (int)TMA_SMEM_MAX); }) != cudaSuccess) {
+    cudaGetLastError();
+    return (int)cudaErrorInvalidValue;
   }
   const size_t smem = tma_smem(d, stages);
-  if (smem > opted) {
-    if (cudaFuncSetAttribute(k_smooth_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-      cudaGetLastError();
-      return (int)cudaErrorInvalidValue;
-    }
-    opted = smem;
-  }
   const int ntiles = ((d.mx - 2 + TMA_TW - 1) / TMA_TW) * (d.mz - 2);
   const int grid = std::max(1, std::min(nsm, ntiles));
   k_smooth_tma<<<grid, TMA_NT, smem, s>>>(m, A, lf, xi, b, xo, omega, stages, err, g_tma_drop);
