@@ -8,6 +8,7 @@
 // arithmetic (a*b+c is never contracted to an FMA, as with the gcc build the
 // reference uses on x86-64).
 #include "vfs_common.cuh"
+#include "per_device.h"
 #include "vfs_kernels.h"
 
 namespace vfs {
@@ -797,10 +798,11 @@ __global__ void k_dense_build(Dims d, const double* __restrict__ mcoef, double s
 // chain of launches bounded it (432 rows, whole set-up: 6.65 ms, by 16 columns
 // 2.92, by 8, whose panel takes half the FP64 operations on its one SM, 2.65).
 constexpr int GJ_B = 8;
+constexpr size_t GJ_SMEM = 192 * 1024;
 // Columns a step: a power of two whose panel fits a block's shared memory.
 static int gj_width(int n) {
   int b = GJ_B;
-  while (b > 1 && (size_t)b * n * sizeof(double) > 192 * 1024) b >>= 1;
+  while (b > 1 && (size_t)b * n * sizeof(double) > GJ_SMEM) b >>= 1;
   return b;
 }
 // The warp's best pivot candidate (magnitude bits v of row r) in every lane:
@@ -1029,7 +1031,8 @@ int launch_coarsen(const Dims& f, const Dims& c, int si, int sj, int sk, const d
   const int smax = (c.mx - 2) + (c.my - 2) + (c.mz - 2);
   const size_t plane = (size_t)(c.mx - 2) * (c.my - 2);
   if (ncell(c) <= 200 * 1024) {  // (96x48x48 and its levels: 162 launches)
-    VFS_CUDA_OK(cudaFuncSetAttribute(k_nvert_sandwich_block, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    static PerDevice once;
+    VFS_CUDA_OK(once([] { return allow_smem(k_nvert_sandwich_block, 200 * 1024); }));
     k_nvert_sandwich_block<<<1, 1024, ncell(c), s>>>(c, nv_c); ++g_launches;
   } else {
     for (int sd = 3; sd <= smax; sd++) { k_nvert_sandwich<<<nblk(plane), 256, 0, s>>>(c, sd, nv_c); ++g_launches; }
@@ -1052,7 +1055,10 @@ int launch_dense_inverse(const Dims& d, const double* mcoef, double sigma, doubl
   int *src = (int*)(Np + (size_t)n * GJ_B), *perm = src + n;
   const int b = gj_width(n);
   const size_t sm = (size_t)b * n * sizeof(double);
-  VFS_CUDA_OK(cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sm > 48 * 1024 ? sm : 48 * 1024)));
+  // the most any order takes, not this one's: the attribute is the kernel's, and
+  // a smaller order set in another thread between two panels would refuse them
+  static PerDevice once;
+  VFS_CUDA_OK(once([] { return allow_smem(k_gj_panel, (int)GJ_SMEM); }));
   const int nt = n >= 1024 ? 1024 : (n + 31) / 32 * 32;
   k_dense_build<<<nblk(nn), 256, 0, s>>>(d, mcoef, sigma, A, n, ccomp); ++g_launches;
   for (int p0 = 0; p0 < n; p0 += b) {
