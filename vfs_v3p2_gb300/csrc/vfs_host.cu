@@ -367,9 +367,11 @@ template <> double** xbuf<double>(Level& L) { return L.x64; }
 template <typename T> T*& bbuf(Level& L);
 template <> float*& bbuf<float>(Level& L) { return L.b32; }
 template <> double*& bbuf<double>(Level& L) { return L.b64; }
+// The coarsest level's dense inverse: none while no row of the level is fluid
+// (the buffers may hold a former mask's).
 template <typename T> T* binv(Level& L);
-template <> float* binv<float>(Level& L) { return L.Binv32; }
-template <> double* binv<double>(Level& L) { return L.Binv; }
+template <> float* binv<float>(Level& L) { return L.nco ? L.Binv32 : nullptr; }
+template <> double* binv<double>(Level& L) { return L.nco ? L.Binv : nullptr; }
 
 template <typename T>
 OpView<T> mgview(Level& L, const int* skip) {
@@ -530,7 +532,7 @@ struct SweepRun {
 // bufs[(writes - 1) & 1], so the caller's first buffer is swapped in when
 // needed to make the V-cycle's result always land in xa.
 int level_writes(const Grid& g, int l, const MGCfg& c) {
-  if (l == 0) return g.lev[0].Binv ? 1 : c.ncoarse;
+  if (l == 0) return g.lev[0].nco ? 1 : c.ncoarse;
   return c.pre(l) + (c.pre(l) == 0 ? 1 : 0) + c.post(l);
 }
 
