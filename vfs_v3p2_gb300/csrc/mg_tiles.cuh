@@ -1335,6 +1335,7 @@ template <typename T>
 inline int smooth_tw(int ni, int nj, int nk, int cols, bool narrow = true) {
   int tw = cols > 0 ? cols : VFS_SMOOTH_TWMAX;
   while (tw > 4 && (size_t)3 * tw * nj * sizeof(T) > 48 * 1024) tw >>= 1;
+  while (tw > 2 && (size_t)3 * tw * nj * sizeof(T) > 200 * 1024) tw >>= 1;  // what a block may have (FP64, > 2133 rows)
   while (tw > 4 && tw / 2 >= ni) tw >>= 1;
   if (cols == 0 && narrow)
     while (tw > VFS_SMOOTH_TWMIN && (size_t)((ni + tw - 1) / tw) * nk < VFS_SMOOTH_MINBLK) tw >>= 1;
