@@ -99,7 +99,20 @@ const bool g_debug = [] {
   return e && e[0] == '1';
 }();
 int g_debug_err = 0;
+// The first launch that was refused since launch_errors_clear(), of this
+// thread: a missing kernel must end the solve, whose other kernels would run
+// on what it left unwritten.
+struct LaunchError {
+  int rc = 0;
+  const char* stage = "";
+};
+thread_local LaunchError t_launch_error;
+void launch_errors_clear() {
+  t_launch_error = LaunchError{};
+  cudaGetLastError();  // (also of calls that are not ours, which a launcher would report as its own)
+}
 void dbg(const char* stage, int level, int rc, cudaStream_t s) {
+  if (rc && rc != (int)cudaErrorNotReady && !t_launch_error.rc) t_launch_error = {rc, stage};
   if (!g_debug || g_debug_err) return;
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) return;
@@ -239,6 +252,13 @@ int fail(vfs_ctx* c, int code, const std::string& msg) {
 }
 int cuda_fail(vfs_ctx* c, cudaError_t e, const char* where) {
   return fail(c, VFS_ERR_CUDA, std::string(where) + ": " + cudaGetErrorString(e));
+}
+// VFS_ERR_CUDA if a launch was refused since launch_errors_clear().
+int launch_errors(vfs_ctx* c) {
+  if (!t_launch_error.rc) return VFS_OK;
+  const LaunchError e = t_launch_error;
+  launch_errors_clear();
+  return cuda_fail(c, (cudaError_t)e.rc, (std::string("launch refused: ") + e.stage).c_str());
 }
 #define CK(expr)                                             \
   do {                                                       \
@@ -750,8 +770,10 @@ int precond(vfs_ctx* ctx, Grid& g, const vfs_solve_params& p, const double* v, T
   mc.solo = solo;
   mc.cluster = coarse_top(g, mc);
   const float* dinv = dinv_sel<T>(F, mc.half);
+  launch_errors_clear();
   if (with_input) dbg("scale_in", g.L - 1, launch_scale_in<T>(F.d, nullptr, v, bf, skip, s, dinv), s);
   T* res = vcycle<T>(g, g.L - 1, bf, z, tmp, mc, skip, s);
+  if (int r = launch_errors(ctx)) return r;
   if (res != z) CK(cudaMemcpyAsync(z, res, F.N * sizeof(T), cudaMemcpyDeviceToDevice, s));
   return VFS_OK;
 }
@@ -874,9 +896,8 @@ void issue_krylov(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv) {
               (double)n_interior(F.d) * (8.0 * popcount(F.mask) + 2 * sizeof(T) + 8.0));
     OpView<double> A{F.d, F.mcoef, F.mask, skip};
     A.flip = n_interior(F.d) >= VFS_FLIP_MINCELLS;
-    launch_apply64_krylov<T>(A, zt, zbase<T>(g), g.st, g.w, s);
+    dbg("apply64", g.L - 1, launch_apply64_krylov<T>(A, zt, zbase<T>(g), g.st, g.w, s), s);
   }
-  dbg("apply64", g.L - 1, 0, s);
   {
     // the nv basis columns and w read (the finish reads block partials only)
     Probed pr(VFS_PROBE_ALL, s, "k_multidot", g.L - 1, Nd * (nvb + 1.0) * 8.0);
@@ -945,9 +966,12 @@ int iteration_graph(vfs_ctx* ctx, Grid& g, const vfs_solve_params& p, cudaGraphE
   // captured launches run on replay, not now: count them per replay instead
   g.ig_kernels = g_launches.load() - n0;
   g_launches -= g.ig_kernels;
-  if (e != cudaSuccess) {
+  int r = launch_errors(ctx);
+  if (!r && e != cudaSuccess) r = cuda_fail(ctx, e, "cudaStreamEndCapture");
+  if (r) {
     if (graph) cudaGraphDestroy(graph);
-    return cuda_fail(ctx, e, "cudaStreamEndCapture");
+    cudaGetLastError();
+    return r;
   }
   e = cudaGraphInstantiate(&g.ig_exec, graph, 0);
   cudaGraphDestroy(graph);
@@ -985,9 +1009,9 @@ void fg_cycle_end(Grid& g, const vfs_solve_params& p, bool last, cudaStream_t s,
   {
     Level& F = g.lev[g.L - 1];
     Probed pr(VFS_PROBE_ALL, s, "k_apply64 (residual)", g.L - 1, (double)n_interior(F.d) * (8.0 * popcount(F.mask) + 24.0));
-    apply_outer(g, g.phi, g.bs, g.V, &g.st->done, s);
+    dbg("residual", g.L - 1, apply_outer(g, g.phi, g.bs, g.V, &g.st->done, s), s);
   }
-  launch_beta(g.st, g.V, N, g.parts, s);
+  dbg("beta", 0, launch_beta(g.st, g.V, N, g.parts, s), s);
   fg_open_cycle<T>(g, p, s);
 }
 
@@ -1029,7 +1053,8 @@ int fg_step(vfs_ctx* ctx, Fgmres& f) {
   } else {
     issue_iteration<T>(g, *f.p, g.s, f.j + 1);
   }
-  return fg_after<T>(ctx, f, g.s);
+  const int r = fg_after<T>(ctx, f, g.s);
+  return r ? r : launch_errors(ctx);
 }
 
 double initial_atol(const Grid& g, const vfs_solve_params& p) {
@@ -1134,6 +1159,9 @@ namespace {
 int job_fail(vfs_ctx* ctx, Job& J, int rc) {
   J.rc = rc;
   J.err = ctx->err;
+  // the caller's buffers are the caller's again
+  cudaStreamSynchronize(J.g->cs);
+  cudaStreamSynchronize(J.g->s);
   J.phase = J_DONE;
   return rc;
 }
@@ -1165,7 +1193,7 @@ int job_start(vfs_ctx* ctx, Job& J) {
                            g.cs));
         CK(cudaEventRecord(g.ev_uin, g.cs));
         CK(cudaStreamWaitEvent(g.s, g.ev_uin, 0));
-        launch_aos2soa(c1 - c0, g.aos + 3 * c0, g.u + c0, g.u + N + c0, g.u + 2 * N + c0, g.s);
+        dbg("aos2soa", 0, launch_aos2soa(c1 - c0, g.aos + 3 * c0, g.u + c0, g.u + N + c0, g.u + 2 * N + c0, g.s), g.s);
       }
     } else {
       CK(cudaMemcpyAsync(g.u, g.ustar, 3 * N * sizeof(double), cudaMemcpyDeviceToDevice, g.s));
@@ -1328,29 +1356,29 @@ int job_post_eval(vfs_ctx* ctx, Job& J) {
 template <typename T>
 int job_advance(vfs_ctx* ctx, Job& J) {
   Grid& g = *J.g;
+  // an error on the way ends the job (some steps have ended it themselves)
+  auto step = [&](int r) {
+    if (!r && J.phase != J_DONE) r = launch_errors(ctx);
+    if (r && J.phase != J_DONE) job_fail(ctx, J, r);
+    return 1;
+  };
+  launch_errors_clear();
   switch (J.phase) {
     case J_START:
-      job_start<T>(ctx, J);
-      return 1;
+      return step(job_start<T>(ctx, J));
     case J_ITER: {
       const int r = fg_step<T>(ctx, J.f);
-      if (r) return job_fail(ctx, J, r), 1;
-      if (J.f.finished) job_check_enqueue(ctx, J);
-      return 1;
+      return step(!r && J.f.finished ? job_check_enqueue(ctx, J) : r);
     }
     case J_CHECK: {
       const cudaError_t e = cudaEventQuery(g.ev_chk);
       if (e == cudaErrorNotReady) return 0;
-      if (e != cudaSuccess) return job_fail(ctx, J, cuda_fail(ctx, e, "check")), 1;
-      job_check_eval<T>(ctx, J);
-      return 1;
+      return step(e != cudaSuccess ? cuda_fail(ctx, e, "check") : job_check_eval<T>(ctx, J));
     }
     case J_POST: {
       const cudaError_t e = cudaEventQuery(g.ev_done);
       if (e == cudaErrorNotReady) return 0;
-      if (e != cudaSuccess) return job_fail(ctx, J, cuda_fail(ctx, e, "post")), 1;
-      job_post_eval<T>(ctx, J);
-      return 1;
+      return step(e != cudaSuccess ? cuda_fail(ctx, e, "post") : job_post_eval<T>(ctx, J));
     }
     default:
       return 0;
@@ -1668,6 +1696,7 @@ int batch_capture(vfs_ctx* ctx, cudaStream_t s0, cudaEvent_t fork, std::vector<c
   }
   const unsigned long long n0 = g_launches.load();
   cudaGraph_t graph = nullptr;
+  launch_errors_clear();
   CK(cudaStreamBeginCapture(s0, cudaStreamCaptureModeThreadLocal));
   cudaEventRecord(fork, s0);
   // members not grouped: their whole iteration on their own streams
@@ -1686,8 +1715,10 @@ int batch_capture(vfs_ctx* ctx, cudaStream_t s0, cudaEvent_t fork, std::vector<c
     cudaStream_t gs = members[P.idx[0]]->g->s;
     cudaStreamWaitEvent(gs, fork, 0);
     for (const GroupLaunch& gl : P.launches) {
-      if (P.f32) launch_group<float>(gl.kind, P.d32 + gl.off, gl.nitems, gl.nblocks, gl.smem, gs);
-      else launch_group<double>(gl.kind, P.d64 + gl.off, gl.nitems, gl.nblocks, gl.smem, gs);
+      dbg("group", 0,
+          P.f32 ? launch_group<float>(gl.kind, P.d32 + gl.off, gl.nitems, gl.nblocks, gl.smem, gs)
+                : launch_group<double>(gl.kind, P.d64 + gl.off, gl.nitems, gl.nblocks, gl.smem, gs),
+          gs);
     }
     cudaEventRecord(bg.stage_done[k], gs);
     for (size_t q : P.idx) {
@@ -1702,7 +1733,13 @@ int batch_capture(vfs_ctx* ctx, cudaStream_t s0, cudaEvent_t fork, std::vector<c
   cudaError_t e = cudaStreamEndCapture(s0, &graph);
   bg.kernels = g_launches.load() - n0;
   g_launches -= bg.kernels;
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "batch capture");
+  int r = launch_errors(ctx);
+  if (!r && e != cudaSuccess) r = cuda_fail(ctx, e, "batch capture");
+  if (r) {
+    if (graph) cudaGraphDestroy(graph);
+    cudaGetLastError();
+    return r;
+  }
   e = cudaGraphInstantiate(&bg.exec, graph, 0);
   cudaGraphDestroy(graph);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "batch graph instantiate");
@@ -1746,10 +1783,7 @@ int run_jobs_batch(vfs_ctx* ctx, std::vector<Job*>& jobs, cudaStream_t s0) {
   CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ticks[0], cudaEventDisableTiming));
   CK(cudaEventCreateWithFlags(&ticks[1], cudaEventDisableTiming));
-  for (Job* J : jobs) {
-    if (J->mixed()) job_start<float>(ctx, *J);
-    else job_start<double>(ctx, *J);
-  }
+  for (Job* J : jobs) job_advance_any(ctx, *J);  // (a job that cannot start is done)
   long long t = 0;
   bool ticked_prev = false;
   for (;;) {
@@ -1792,9 +1826,10 @@ int run_jobs_batch(vfs_ctx* ctx, std::vector<Job*>& jobs, cudaStream_t s0) {
     if (have_prev) CK(cudaEventSynchronize(ticks[(t - 1) & 1]));
     for (Job* J : bg.members) {
       if (J->phase != J_ITER) continue;
-      const int r = J->mixed() ? batch_after_tick<float>(ctx, *J, tick, have_prev)
-                               : batch_after_tick<double>(ctx, *J, tick, have_prev);
-      if (r) job_fail(ctx, *J, r);
+      int r = J->mixed() ? batch_after_tick<float>(ctx, *J, tick, have_prev)
+                         : batch_after_tick<double>(ctx, *J, tick, have_prev);
+      if (!r) r = launch_errors(ctx);
+      if (r && J->phase != J_DONE) job_fail(ctx, *J, r);
     }
     // checks and closes of other grids progress between ticks
     for (Job* J : jobs) {
@@ -1874,14 +1909,15 @@ int grid_set_nvert(vfs_ctx* ctx, Grid& g, const double* nvert) {
 // by vfs_poisson_lhs.
 int grid_derive(vfs_ctx* ctx, Grid& g, bool coords) {
   const int L = g.L;
+  launch_errors_clear();
   for (int l = L - 2; l >= 0; l--)
-    launch_coarsen(g.lev[l + 1].d, g.lev[l].d, g.si, g.sj, g.sk, g.lev[l + 1].coor, g.lev[l + 1].nvert, g.lev[l].coor,
-                   g.lev[l].nvert, g.s);
+    CK(launch_coarsen(g.lev[l + 1].d, g.lev[l].d, g.si, g.sj, g.sk, g.lev[l + 1].coor, g.lev[l + 1].nvert, g.lev[l].coor,
+                      g.lev[l].nvert, g.s));
   if (coords)
-    for (int l = 0; l < L; l++) launch_form_metrics(g.lev[l].d, g.lev[l].coor, g.lev[l].M, g.mtmp, g.s);
-  for (int l = 0; l < L; l++) launch_restrict_weights(g.lev[l].N, g.lev[l].nvert, g.lev[l].rw32, g.lev[l].rw64, g.s);
+    for (int l = 0; l < L; l++) CK(launch_form_metrics(g.lev[l].d, g.lev[l].coor, g.lev[l].M, g.mtmp, g.s));
+  for (int l = 0; l < L; l++) CK(launch_restrict_weights(g.lev[l].N, g.lev[l].nvert, g.lev[l].rw32, g.lev[l].rw64, g.s));
   Level& F = g.lev[L - 1];
-  launch_inverse_metric(F.d, F.M, F.nvert, g.minv, g.s);
+  CK(launch_inverse_metric(F.d, F.M, F.nvert, g.minv, g.s));
   cudaError_t e = cudaStreamSynchronize(g.s);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "grid setup");
   // the operator and every captured iteration depend on these
@@ -2231,6 +2267,8 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   Grid& g = *gp;
   CK(cudaSetDevice(ctx->device));
   const size_t N = ncell(g.d);
+  launch_errors_clear();
+  g.lhs = false;  // until the new operator is whole
   // scratch on the grid's own stream: the g tensor in the metric formation's
   // buffer (9 N), the slot mask, range flag, nonzero weights and region count among the scalars
   double* gt = g.mtmp;
@@ -2239,24 +2277,24 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   CK(cudaMemsetAsync(dmask + 1, 0, sizeof(unsigned), g.s));
   for (int l = 0; l < g.L; l++) {
     Level& Lv = g.lev[l];
-    launch_gtensor(Lv.d, Lv.M, gt, g.s);
-    launch_assemble(Lv.d, gt, Lv.nvert, Lv.M + Lv.N * MP_AJ, Lv.coef, Lv.mcoef, Lv.mcoef32, dmask, g.s);
-    launch_face_operator(Lv.d, gt, Lv.nvert, Lv.M + Lv.N * MP_AJ, Lv.ffi, Lv.ffk, Lv.ffj, Lv.faj, Lv.ffc, g.s);
+    CK(launch_gtensor(Lv.d, Lv.M, gt, g.s));
+    CK(launch_assemble(Lv.d, gt, Lv.nvert, Lv.M + Lv.N * MP_AJ, Lv.coef, Lv.mcoef, Lv.mcoef32, dmask, g.s));
+    CK(launch_face_operator(Lv.d, gt, Lv.nvert, Lv.M + Lv.N * MP_AJ, Lv.ffi, Lv.ffk, Lv.ffj, Lv.faj, Lv.ffc, g.s));
     CK(cudaMemcpyAsync(&Lv.mask, dmask, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
-    if (l > 0) launch_prolong_codes(Lv.d, g.lev[l - 1].d, g.si, g.sj, g.sk, Lv.nvert, g.lev[l - 1].nvert, Lv.pcode, g.s);
-    launch_line_factors<float>(Lv.d, Lv.mcoef, Lv.lf32, g.s);
-    launch_line_factors<double>(Lv.d, Lv.mcoef, Lv.lf64, g.s);
-    launch_half_operator(Lv.d, Lv.mcoef, Lv.hcoef, l == g.L - 1 ? Lv.dinvh : nullptr, l == 0 ? Lv.dvalh : nullptr,
-                         dmask + 1, g.s);
-    launch_line_factors_half(Lv.d, Lv.hcoef, Lv.mcoef, Lv.lfh, g.s);
+    if (l > 0) CK(launch_prolong_codes(Lv.d, g.lev[l - 1].d, g.si, g.sj, g.sk, Lv.nvert, g.lev[l - 1].nvert, Lv.pcode, g.s));
+    CK(launch_line_factors<float>(Lv.d, Lv.mcoef, Lv.lf32, g.s));
+    CK(launch_line_factors<double>(Lv.d, Lv.mcoef, Lv.lf64, g.s));
+    CK(launch_half_operator(Lv.d, Lv.mcoef, Lv.hcoef, l == g.L - 1 ? Lv.dinvh : nullptr, l == 0 ? Lv.dvalh : nullptr,
+                         dmask + 1, g.s));
+    CK(launch_line_factors_half(Lv.d, Lv.hcoef, Lv.mcoef, Lv.lfh, g.s));
   }
   CK(cudaMemsetAsync(g.lev[0].rwh, 0, g.lev[0].N * sizeof(float), g.s));
   for (int l = 1; l < g.L; l++)
-    launch_restrict_weights_half(g.lev[l].d, g.lev[l - 1].d, g.si, g.sj, g.sk, g.lev[l].nvert, g.lev[l].mcoef,
-                                 g.lev[l - 1].mcoef, g.lev[l].rwh, g.s);
+    CK(launch_restrict_weights_half(g.lev[l].d, g.lev[l - 1].d, g.si, g.sj, g.sk, g.lev[l].nvert, g.lev[l].mcoef,
+                                 g.lev[l - 1].mcoef, g.lev[l].rwh, g.s));
   Level& F = g.lev[g.L - 1];
-  launch_proj_dots(F.d, F.M, g.pd, g.s);
-  launch_proj_weights(F.d, g.pd, F.M, F.nvert, g.pw, g.pc, dmask + 2, g.s);
+  CK(launch_proj_dots(F.d, F.M, g.pd, g.s));
+  CK(launch_proj_weights(F.d, g.pd, F.M, F.nvert, g.pw, g.pc, dmask + 2, g.s));
   unsigned range = 0;
   CK(cudaMemcpyAsync(&range, dmask + 1, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
   CK(cudaMemcpyAsync(&g.pw_used, dmask + 2, sizeof(unsigned), cudaMemcpyDeviceToHost, g.s));
@@ -2267,7 +2305,7 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
   // grid that bodies cut apart needs the labels.
   g.ncomp = 1;
   if (g.nfluid < (double)n_interior(F.d)) {
-    launch_region_count(F.d, F.nvert, (int*)gt, dregions, g.s);
+    CK(launch_region_count(F.d, F.nvert, (int*)gt, dregions, g.s));
     int regions = 0;
     CK(cudaMemcpyAsync(&regions, dregions, sizeof(int), cudaMemcpyDeviceToHost, g.s));
     CK(cudaStreamSynchronize(g.s));
@@ -2337,8 +2375,9 @@ int vfs_poisson_lhs(vfs_ctx* ctx, int grid) {
         cudaFree(own); cudaFree(ccomp);
         return r;
       }
-      launch_dense_inverse(C.d, C.mcoef, sigma, W, C.Binv, C.Binv32, n, g.s, ccomp);
+      const cudaError_t le = (cudaError_t)launch_dense_inverse(C.d, C.mcoef, sigma, W, C.Binv, C.Binv32, n, g.s, ccomp);
       cudaError_t e = cudaStreamSynchronize(g.s);
+      if (e == cudaSuccess) e = le;
       cudaFree(own); cudaFree(ccomp);
       if (e != cudaSuccess) return cuda_fail(ctx, e, "coarse inverse");
       C.nco = n;
@@ -2600,7 +2639,7 @@ int step_post(Grid& g, double dt, double st, double coeff, bool exact, double* u
     const size_t P = (size_t)F.d.mx * F.d.my;
     auto to_aos = [&](int k0, int k1) {
       const size_t c0 = k0 * P;
-      launch_soa2aos((k1 - k0) * P, g.u + c0, g.u + N + c0, g.u + 2 * N + c0, g.aos + 3 * c0, g.s);
+      dbg("soa2aos", 0, launch_soa2aos((k1 - k0) * P, g.u + c0, g.u + N + c0, g.u + 2 * N + c0, g.aos + 3 * c0, g.s), g.s);
     };
     auto download = [&](int k0, int k1) {
       const size_t c0 = k0 * P;
