@@ -487,6 +487,7 @@ struct MGCfg {
   bool solo;       // the grid's solve runs alone
   int stage;       // how the finest face-form sweeps stage their operands (SweepStage)
   int cluster = 0;  // levels 1 .. cluster (and the coarsest) run as one cluster launch (0: none)
+  int cluster_blocks = 0;  // of this many blocks
   int pre(int l) const { return l == top ? nu1 : nu1c; }
   int post(int l) const { return l == top ? nu2 : nu2c; }
 };
@@ -599,10 +600,10 @@ void coarse_args(Grid& g, int top, const MGCfg& c, CvArgs& a) {
 #ifndef VFS_CV_MAXCELLS
 #define VFS_CV_MAXCELLS 70000
 #endif
-int coarse_top(Grid& g, const MGCfg& c) {
-  if (g_probe.kind != 0 || g_debug || !c.face || c.half || g.si || g.sj || g.sk) return 0;
-  if (!g.lev[0].Binv32 || g.lev[0].nco < 1 || g.lev[0].nco > CV_DENSE_MAX) return 0;
-  if (c.nu1c < 1 || c.nu2c < 1 || c.nu1c > CV_MAXSWEEP || c.nu2c > CV_MAXSWEEP) return 0;
+void choose_cluster(Grid& g, MGCfg& c) {
+  if (g_probe.kind != 0 || g_debug || !c.face || c.half || g.si || g.sj || g.sk) return;
+  if (!g.lev[0].Binv32 || g.lev[0].nco < 1 || g.lev[0].nco > CV_DENSE_MAX) return;
+  if (c.nu1c < 1 || c.nu2c < 1 || c.nu1c > CV_MAXSWEEP || c.nu2c > CV_MAXSWEEP) return;
   int top = 0;
   for (int l = 1; l < g.L && l < CV_MAXLEV; l++) {
     const bool sweeps = l != c.top || (c.nu1 >= 1 && c.nu2 >= 1 && c.nu1 <= CV_MAXSWEEP && c.nu2 <= CV_MAXSWEEP);
@@ -612,9 +613,12 @@ int coarse_top(Grid& g, const MGCfg& c) {
   for (; top > 0; top--) {
     CvArgs a;
     coarse_args(g, top, c, a);
-    if (cv_cluster(a)) return top;
+    if (const int blocks = cv_cluster(a)) {
+      c.cluster = top;
+      c.cluster_blocks = blocks;
+      return;
+    }
   }
-  return 0;
 }
 
 #ifndef VFS_FLIP_MINCELLS
@@ -626,12 +630,13 @@ T* vcycle(Grid& g, int l, T* b, T* xa, T* xb, const MGCfg& c, const int* skip, c
     if (l > 0 && l == c.cluster) {
       CvArgs a;
       coarse_args(g, l, c, a);
-      cv_cluster(a);
-      a.b = b;
-      a.x = xa;
-      a.skip = skip;
-      dbg("coarse_vcycle", l, launch_coarse_vcycle(a, s), s);
-      return xa;
+      if (cv_layout(a, c.cluster_blocks)) {  // (choose_cluster's layout)
+        a.b = b;
+        a.x = xa;
+        a.skip = skip;
+        dbg("coarse_vcycle", l, launch_coarse_vcycle(a, s), s);
+        return xa;
+      }
     }
   }
   Level& L = g.lev[l];
@@ -768,7 +773,7 @@ int precond(vfs_ctx* ctx, Grid& g, const vfs_solve_params& p, const double* v, T
   T* bf = bbuf<T>(F);
   MGCfg mc = mgcfg(p, g.L - 1, g.half_ok);
   mc.solo = solo;
-  mc.cluster = coarse_top(g, mc);
+  choose_cluster(g, mc);
   const float* dinv = dinv_sel<T>(F, mc.half);
   launch_errors_clear();
   if (with_input) dbg("scale_in", g.L - 1, launch_scale_in<T>(F.d, nullptr, v, bf, skip, s, dinv), s);
@@ -875,7 +880,7 @@ void issue_iteration(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv 
   Level& F = g.lev[g.L - 1];
   MGCfg mc = mgcfg(p, g.L - 1, g.half_ok);
   mc.solo = g.solo;
-  mc.cluster = coarse_top(g, mc);
+  choose_cluster(g, mc);
   vcycle<T>(g, g.L - 1, bbuf<T>(F), xbuf<T>(F)[0], xbuf<T>(F)[1], mc, &g.st->done, s);
   issue_krylov<T>(g, p, s, nv);
 }
