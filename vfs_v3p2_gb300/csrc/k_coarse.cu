@@ -26,9 +26,6 @@
 
 namespace vfs {
 
-constexpr int CV_NT = 512;
-constexpr int CV_Q = 4;  // cells a thread may own of a level (their operator in registers)
-
 // Values between two columns of the line arrays: twice an odd number.
 __host__ __device__ inline int cv_line_pitch(int nj) {
   const int p = (nj + 1) & ~1;
@@ -501,7 +498,7 @@ int cv_cluster(CvArgs& a) {
     cudaGetLastError();
     return 0;
   }
-  for (int cl : {16, 8}) {
+  for (int cl : {CV_MAXBLOCKS, 8}) {
     if (!cv_layout(a, cl)) continue;
     cudaLaunchAttribute attr;
     cudaLaunchConfig_t cfg = cv_config(a, nullptr, &attr);

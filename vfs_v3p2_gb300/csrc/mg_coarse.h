@@ -10,6 +10,10 @@
 
 namespace vfs {
 
+constexpr int CV_NT = 512;      // threads of a block
+constexpr int CV_Q = 4;         // cells a thread may own of a level (their operator in registers)
+constexpr int CV_MAXBLOCKS = 16;
+constexpr size_t CV_MAXCELLS = (size_t)CV_MAXBLOCKS * CV_NT * CV_Q;  // largest level
 constexpr int CV_MAXLEV = 6;    // levels a launch may hold (the coarsest included)
 constexpr int CV_MAXSWEEP = 8;  // smoothing sweeps per level and side
 constexpr int CV_DENSE_MAX = 2048;  // largest coarsest level: its right-hand side and solution sit in every block

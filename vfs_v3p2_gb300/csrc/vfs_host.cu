@@ -597,9 +597,6 @@ void coarse_args(Grid& g, int top, const MGCfg& c, CvArgs& a) {
 // their clusters run side by side, nine at a time, where the separate
 // launches of many small levels queue (64 grids of 32^3 21.1 -> 16.8 ms, 24
 // up to 96x64x64 19.6 -> 17.5, six served streams 22.6 -> 22.2).
-#ifndef VFS_CV_MAXCELLS
-#define VFS_CV_MAXCELLS 70000
-#endif
 void choose_cluster(Grid& g, MGCfg& c) {
   if (g_probe.kind != 0 || g_debug || !c.face || c.half || g.si || g.sj || g.sk) return;
   if (!g.lev[0].Binv32 || g.lev[0].nco < 1 || g.lev[0].nco > CV_DENSE_MAX) return;
@@ -607,7 +604,7 @@ void choose_cluster(Grid& g, MGCfg& c) {
   int top = 0;
   for (int l = 1; l < g.L && l < CV_MAXLEV; l++) {
     const bool sweeps = l != c.top || (c.nu1 >= 1 && c.nu2 >= 1 && c.nu1 <= CV_MAXSWEEP && c.nu2 <= CV_MAXSWEEP);
-    if (!face_level(g.lev[l]) || !sweeps || n_interior(g.lev[l].d) > VFS_CV_MAXCELLS) break;
+    if (!face_level(g.lev[l]) || !sweeps || n_interior(g.lev[l].d) > CV_MAXCELLS) break;
     top = l;
   }
   for (; top > 0; top--) {
