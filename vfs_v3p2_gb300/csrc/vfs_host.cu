@@ -2704,7 +2704,6 @@ int vfs_projection_step(vfs_ctx* ctx, int grid, double* ucont_inout, double* p_i
   if (!(dt > 0.)) return fail(ctx, VFS_ERR_ARG, "dt must be > 0");
   if (g.m && p->restart > g.m) return fail(ctx, VFS_ERR_ARG, "restart length cannot grow after the first solve");
   if (g.busy) return fail(ctx, VFS_ERR_BUSY, "the grid has a request in flight");
-  g.solo = false;  // requests share the GPU
   Job J;
   J.g = &g;
   J.p = *p;
@@ -2805,6 +2804,7 @@ int vfs_submit(vfs_ctx* ctx, const vfs_request* req, long long* ticket) {
   J.coeff = req->coeff;
   J.ticket = ctx->next_ticket++;
   g.busy = J.ticket;
+  g.solo = false;  // requests share the GPU
   job_advance_any(ctx, J);  // inputs and right-hand side go to the device now
   *ticket = J.ticket;
   ctx->inflight[J.ticket] = std::move(box);
