@@ -248,8 +248,10 @@ static void smooth_launch(bool small, dim3 g, size_t sm, cudaStream_t s, const O
 }
 
 // The rows' lines must fit: 48 KB a block at four blocks per SM, 96 KB at two
-// (longer lines take narrower tiles of the one-cell-per-thread sweep).
+// (longer lines take narrower tiles of the one-cell-per-thread sweep); and the
+// general form's 32-bit byte offsets its 16-byte entries.
 static bool smooth_w_fits(const Dims& d, bool ch) {
+  if (!ch && !fits_byte_offsets(d)) return false;
   return smooth_smem<float>(32, d.my - 2) <= (size_t)(ch ? 48 : 96) * 1024;
 }
 

@@ -1169,9 +1169,10 @@ __device__ __forceinline__ void smooth_tile_w(const OpView<float>& A, const floa
 //
 // Offsets are unsigned bytes from the arrays' uniform bases (one 32-bit add a
 // row and plane instead of a 64-bit product a load): an array of 16-byte
-// entries stays below 2^32 bytes up to 2^28 cells, whose grid (1.2 KB a cell)
-// no card holds.
+// entries stays below 2^32 bytes up to 2^28 cells (larger levels take the
+// tiles).
 // ---------------------------------------------------------------------------
+__host__ __device__ inline bool fits_byte_offsets(const Dims& d) { return ncell(d) <= ((size_t)1 << 28); }
 template <typename V>
 __device__ __forceinline__ V ldb(const V* __restrict__ p, unsigned o) {
   return __ldg(reinterpret_cast<const V*>(reinterpret_cast<const char*>(p) + o));
