@@ -156,8 +156,8 @@ template int launch_open_v<double>(const KrylovState*, double*, double*, size_t,
 
 // Multi-dot partials: parts[q * nblocks + b] = sum over block b's cells of
 // V_q . w for q < nv, up to DCH columns per sweep (w is re-read from L2).
-// nv < 0: use the device's current column count st->j + 1 (graph-replayable).
-__device__ __forceinline__ int nv_of(const KrylovState* st, int nv) { return nv < 0 ? st->j + 1 : nv; }
+// The column count nv = st->j + 1 is the device's, so that a launch can be
+// replayed from a graph.
 constexpr int DCH = 8;
 
 // Sums of DCH values over a warp by halving exchanges: 4 + 2 + 1 adds leave
@@ -271,10 +271,10 @@ __device__ __forceinline__ void dots(KrylovState* st, const double* __restrict__
   }
   if (last_block(st->ticket)) dots_finish(st, parts, gridDim.x, nv, pass);
 }
-__global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* __restrict__ V, int nv,
-                                                 const double* __restrict__ w, size_t n, double* parts, int pass) {
+__global__ void __launch_bounds__(KB) k_multidot(KrylovState* st, const double* __restrict__ V,
+                                                 const double* __restrict__ w, size_t n, double* parts) {
   if (is_done(st)) return;
-  dots<false>(st, V, nv_of(st, nv), w, n, parts, pass);
+  dots<false>(st, V, st->j + 1, w, n, parts, 1);
 }
 
 // Blocks of the dots: a warp's reduction of eight columns takes nine FP64 adds
@@ -286,9 +286,8 @@ static int dots_nblocks(size_t n) {
   const size_t b = full > 152 * 2 ? full : (two < 152 * 2 ? two : 152 * 2);
   return (int)(b > 152 * 4 ? 152 * 4 : (b ? b : 1));
 }
-int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
-                    cudaStream_t s) {
-  k_multidot<<<dots_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, pass); ++g_launches;
+int launch_multidot(KrylovState* st, const double* V, const double* w, size_t n, double* parts, cudaStream_t s) {
+  k_multidot<<<dots_nblocks(n), KB, 0, s>>>(st, V, w, n, parts); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -391,13 +390,13 @@ __device__ __forceinline__ double subtract_columns(const double* __restrict__ V,
 
 // w -= sum_q h[q] V_q, with the partials of ||w||^2 after the update; close:
 // the last block closes the Arnoldi column.
-__global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double* __restrict__ V, int nv,
+__global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double* __restrict__ V,
                                                   double* __restrict__ w, size_t n, double* parts, int close, int* hst) {
   if (is_done(st)) {
     if (close && blockIdx.x == 0 && threadIdx.x == 0) post_status(st, hst);
     return;
   }
-  nv = nv_of(st, nv);
+  const int nv = st->j + 1;
   __shared__ double sh[32];
   __shared__ double hs[72];
   column_factors(st, nv, hs);
@@ -405,9 +404,9 @@ __global__ void __launch_bounds__(KB) k_gs_update(KrylovState* st, const double*
   if (threadIdx.x == 0) parts[blockIdx.x] = s;
   if (close && last_block(st->ticket)) arnoldi_close(st, parts, gridDim.x, hst);
 }
-int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int close, int* hst,
+int launch_gs_update(KrylovState* st, const double* V, double* w, size_t n, double* parts, int close, int* hst,
                      cudaStream_t s) {
-  k_gs_update<<<krylov_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts, close, hst); ++g_launches;
+  k_gs_update<<<krylov_nblocks(n), KB, 0, s>>>(st, V, w, n, parts, close, hst); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -485,17 +484,17 @@ template int launch_cgs_update<double>(KrylovState*, double*, const double*, dou
 // in chunks of columns as k_multidot's, the columns from L2 again: one launch
 // for any number of columns (five that held all columns in registers and
 // summed each by a tree of its own took 83 us at 128x64x96, 13 columns).
-__global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const double* __restrict__ V, int nv, double* w,
-                                                       size_t n, double* parts) {
+__global__ void __launch_bounds__(KB) k_gs_update_dots(KrylovState* st, const double* __restrict__ V, double* w, size_t n,
+                                                       double* parts) {
   if (is_done(st)) return;
-  nv = nv_of(st, nv);
+  const int nv = st->j + 1;
   __shared__ double hs[72];
   column_factors(st, nv, hs);
   subtract_columns(V, nv, w, n, hs);
   dots<true>(st, V, nv, w, n, parts, 2);
 }
-int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s) {
-  k_gs_update_dots<<<dots_nblocks(n), KB, 0, s>>>(st, V, nv, w, n, parts); ++g_launches;
+int launch_gs_update_dots(KrylovState* st, const double* V, double* w, size_t n, double* parts, cudaStream_t s) {
+  k_gs_update_dots<<<dots_nblocks(n), KB, 0, s>>>(st, V, w, n, parts); ++g_launches;
   return (int)cudaGetLastError();
 }
 
@@ -550,14 +549,13 @@ template int launch_x_update<double>(KrylovState*, const double*, size_t, double
 
 // Next basis vector and multigrid input in one sweep: V_{j+1} = w / h_{j+1,j}
 // and out = T(V_{j+1}) over the interior; ghost entries of w are zero.
-// vn == nullptr: the target is V + st->j * n (the column just opened).
+// V_{j+1} is V + st->j * n (the column just opened).
 template <typename T>
-__global__ void __launch_bounds__(KB) k_vnext_in(const KrylovState* st, const double* __restrict__ w, double* vn,
-                                                  T* __restrict__ out, size_t n, double* V,
-                                                  const float* __restrict__ dinv) {
+__global__ void __launch_bounds__(KB) k_vnext_in(const KrylovState* st, const double* __restrict__ w, double* V,
+                                                  T* __restrict__ out, size_t n, const float* __restrict__ dinv) {
   if (is_done(st)) return;
   const double f = st->inv_hn;
-  if (!vn) vn = V + (size_t)st->j * n;
+  double* vn = V + (size_t)st->j * n;
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
     const double v = w[t] * f;
     vn[t] = v;
@@ -565,14 +563,11 @@ __global__ void __launch_bounds__(KB) k_vnext_in(const KrylovState* st, const do
   }
 }
 template <typename T>
-int launch_vnext_in(KrylovState* st, const double* w, double* vn, T* out, size_t n, cudaStream_t s, double* V,
-                    const float* dinv) {
-  k_vnext_in<T><<<krylov_nblocks(n) * 4, KB, 0, s>>>(st, w, vn, out, n, V, dinv); ++g_launches;
+int launch_vnext_in(KrylovState* st, const double* w, double* V, T* out, size_t n, const float* dinv, cudaStream_t s) {
+  k_vnext_in<T><<<krylov_nblocks(n) * 4, KB, 0, s>>>(st, w, V, out, n, dinv); ++g_launches;
   return (int)cudaGetLastError();
 }
-template int launch_vnext_in<float>(KrylovState*, const double*, double*, float*, size_t, cudaStream_t, double*,
-                                    const float*);
-template int launch_vnext_in<double>(KrylovState*, const double*, double*, double*, size_t, cudaStream_t, double*,
-                                     const float*);
+template int launch_vnext_in<float>(KrylovState*, const double*, double*, float*, size_t, const float*, cudaStream_t);
+template int launch_vnext_in<double>(KrylovState*, const double*, double*, double*, size_t, const float*, cudaStream_t);
 
 }  // namespace vfs

@@ -903,7 +903,7 @@ void issue_krylov(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv) {
   {
     // the nv basis columns and w read (the finish reads block partials only)
     Probed pr(VFS_PROBE_ALL, s, "k_multidot", g.L - 1, Nd * (nvb + 1.0) * 8.0);
-    dbg("multidot1", 0, launch_multidot(g.st, g.V, -1, g.w, N, g.parts, 1, s), s);
+    dbg("multidot1", 0, launch_multidot(g.st, g.V, g.w, N, g.parts, s), s);
   }
   // The update's last block closes the Arnoldi column and writes the status to
   // the pinned hstat; a probed iteration closes it in a launch of its own, so
@@ -927,16 +927,16 @@ void issue_krylov(Grid& g, const vfs_solve_params& p, cudaStream_t s, int nv) {
   }
   {
     Probed pr(VFS_PROBE_ALL, s, "k_gs_update_dots", g.L - 1, Nd * (nvb + 2.0) * 8.0);
-    dbg("gs_update_dots", 0, launch_gs_update_dots(g.st, g.V, -1, g.w, N, g.parts, s), s);
+    dbg("gs_update_dots", 0, launch_gs_update_dots(g.st, g.V, g.w, N, g.parts, s), s);
   }
   {
     Probed pr(VFS_PROBE_ALL, s, "k_gs_update", g.L - 1, Nd * (nvb + 2.0) * 8.0);
-    dbg("gs_update2", 0, launch_gs_update(g.st, g.V, -1, g.w, N, g.parts, close, g.hstat, s), s);
+    dbg("gs_update2", 0, launch_gs_update(g.st, g.V, g.w, N, g.parts, close, g.hstat, s), s);
   }
   close_probed();
   {
     Probed pr(VFS_PROBE_ALL, s, "k_vnext_in", g.L - 1, Nd * (16.0 + sizeof(T)));
-    dbg("vnext_in", 0, launch_vnext_in<T>(g.st, g.w, nullptr, bbuf<T>(F), N, s, g.V, dinv), s);
+    dbg("vnext_in", 0, launch_vnext_in<T>(g.st, g.w, g.V, bbuf<T>(F), N, dinv, s), s);
   }
 }
 

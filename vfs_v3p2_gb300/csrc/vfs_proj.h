@@ -123,23 +123,22 @@ int launch_beta(KrylovState* st, const double* r, size_t n, double* parts, cudaS
 // v = r / beta in place and out = T(v)
 template <typename T>
 int launch_open_v(const KrylovState* st, double* v, T* out, size_t n, const float* dinv, cudaStream_t s);
-int launch_multidot(KrylovState* st, const double* V, int nv, const double* w, size_t n, double* parts, int pass,
-                    cudaStream_t s);
+// The Krylov kernels take the column count from the device state, so one
+// iteration is a fixed launch sequence.
+// first pass: the dots of the columns with w
+int launch_multidot(KrylovState* st, const double* V, const double* w, size_t n, double* parts, cudaStream_t s);
 // close: the launch's last block closes the Arnoldi column (what
 // launch_arnoldi_finish does as its own launch) and writes done and epoch to
 // the pinned host ints hst.
-int launch_gs_update(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, int close, int* hst,
+int launch_gs_update(KrylovState* st, const double* V, double* w, size_t n, double* parts, int close, int* hst,
                      cudaStream_t s);
-// In the Krylov kernels nv < 0 (and vn == nullptr) mean "take the column
-// count from the device state", so one iteration is a fixed launch sequence.
 // second CGS pass fused with the first update
-int launch_gs_update_dots(KrylovState* st, const double* V, int nv, double* w, size_t n, double* parts, cudaStream_t s);
+int launch_gs_update_dots(KrylovState* st, const double* V, double* w, size_t n, double* parts, cudaStream_t s);
 template <typename T>
 int launch_cgs_update(KrylovState* st, double* V, const double* w, T* out, size_t n, double* parts, int close, int* hst,
                       cudaStream_t s, const float* dinv = nullptr);
 template <typename T>
-int launch_vnext_in(KrylovState* st, const double* w, double* vn, T* out, size_t n, cudaStream_t s, double* V = nullptr,
-                    const float* dinv = nullptr);
+int launch_vnext_in(KrylovState* st, const double* w, double* V, T* out, size_t n, const float* dinv, cudaStream_t s);
 // w = A z (aj-scaled FP64 operator, z in T) and Z[st->j] = z on the interior
 template <typename T>
 int launch_apply64_krylov(const OpView<double>& A, const T* z, T* Z, const KrylovState* st, double* w, cudaStream_t s);
