@@ -142,8 +142,8 @@ typedef struct {
                          launch per kernel with a table of one item per grid,
                          bit for bit the per-grid launches' results.  0 (the
                          default): each grid's own launches and graph, which
-                         measured faster on GB300 (64-grid batch: 877 against
-                         754 solves/s with each grid a branch of one graph).  Single
+                         measured faster on GB300 (64-grid batch: 1084 against
+                         888 solves/s).  Single
                          solves and served requests ignore it. */
   int mg_stage;       /* How the finest level's sweeps on the FP32 face form
                          (levels of at least 2^20 interior cells) stage their

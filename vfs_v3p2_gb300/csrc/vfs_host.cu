@@ -593,10 +593,13 @@ void coarse_args(Grid& g, int top, const MGCfg& c, CvArgs& a) {
 // levels under full coarsening, with a dense coarsest solve that fits every
 // block, at least one sweep on each side, and room in shared memory.  A
 // probed or debugged solve runs the levels' own launches, which it times or
-// checks one by one (the same bits).  Grids that share the GPU take it too:
-// their clusters run side by side, nine at a time, where the separate
-// launches of many small levels queue (64 grids of 32^3 21.1 -> 16.8 ms, 24
-// up to 96x64x64 19.6 -> 17.5, six served streams 22.6 -> 22.2).
+// checks one by one (the same bits).  Grids that share the GPU take it too,
+// nine clusters side by side: it pays for few grids and costs for many, whose
+// separate launches fill the GPU (batches with against without: 4 grids of
+// 32^3 1.25 / 1.66 ms, 16 2.7 / 2.9, 64 10.7 / 9.2; 5 grids up to 192x96x96
+// 7.8 / 8.3, 16 17.0 / 17.1; 24 up to 96x64x64 10.8 / 10.0; 64 up to
+// 192x96x96 1085 / 1141 solves/s; served streams differ by less than one
+// setting's runs do).
 void choose_cluster(Grid& g, MGCfg& c) {
   if (g_probe.kind != 0 || g_debug || !c.face || c.half || g.si || g.sj || g.sk) return;
   if (!g.lev[0].Binv32 || g.lev[0].nco < 1 || g.lev[0].nco > CV_DENSE_MAX) return;
@@ -2757,7 +2760,7 @@ int vfs_projection_step_batch(vfs_ctx* ctx, int n, const int* grids, double dt, 
   // graph for all is captured on every call and again as grids finish, and
   // each of its launches ends with the slowest grid (64 grids of 32^3 16.7 ms
   // against 14.9, 24 up to 96x64x64 17.3 against 14.3, 5 up to 192x96x96 7.5
-  // against 7.1).
+  // against 7.1, all with cluster launches).
   bool grouped = false;
   for (const Job* J : jobs) grouped |= J->p.mg_grouped != 0;
   if (grouped && !ctx->s0) CK(cudaStreamCreateWithFlags(&ctx->s0, cudaStreamNonBlocking));
